@@ -1,0 +1,63 @@
+// The hierarchy closure of a row as one independent minimum per string
+// vertex, and the vertex records of the bit-row kernels (bit_rows.cuh).
+//
+// The sweeps of align.hpp:279-345 lower the first score of every string
+// vertex over the hierarchy, level by level, and read the *last* score of
+// each edge's source. They never refresh a last score from a lowered first
+// score, so the source of an edge is a value the row update left -- a
+// constant of the sweep -- unless the source is a one-char vertex, whose
+// first and last score are one. Only one-char sources chain, and replacing
+// such a source by its own sources (weights added) removes the chain: after
+// expansion every swept first score is
+//     F(v) = min(first(v), min over A(v) of raw_last(x) + w)
+// over raw scores only, with no order between vertices. On the variation
+// graphs measured (labels of 1..32 chars) the expansion adds 5-21 % to the
+// hierarchy's edges, and the sweeps' 30-45 dependent levels become one pass.
+//
+// The row update takes a first char's in-edges from the final last scores,
+//     M(v) = min over in-edges u of min(raw_last(u), F(u) + len(u) - 1),
+// expanded the same way into a list B(v) of raw last scores (raw_last(u) is
+// never above raw_first(u) + len(u) - 1, so F(u)'s own raw first drops out).
+// T(first) = min(F + 1, M + delta), so an entry of B whose weight is above
+// that of the same source in A can never win and is dropped; a source with
+// w_B = w_A - 1 (the usual case: x reaches v through u) is read once for both.
+//
+// Graphs of one-char vertices chain without bound; there the lists would
+// grow far beyond the edges, build_closure gives up (ok = false) and the
+// engine sweeps the levels instead.
+#pragma once
+
+#include <cstdint>
+#include <vector>
+
+#include "device_graph.hpp"
+
+namespace chsga {
+
+// Longest list a vertex may have, and entries per hierarchy edge above which
+// the level sweeps are kept.
+constexpr uint32_t kClosureMaxList = 192;
+constexpr uint32_t kClosureMaxGrowth = 6;
+
+struct HostClosure {
+  bool ok = false;
+  // 4 words per string vertex: first bit word of its chain chars; length |
+  // label key of the first char << 29; first entry; entries of each class
+  // (both | M only << 8 | F only << 16)
+  std::vector<uint32_t> rec;
+  // {source vertex, weight}, classes in that order; the weight counts for M
+  // (a "both" entry has weight w + 1 for F), for F-only entries for F
+  std::vector<EdgeW> ent;
+  // per bit word the label planes of its 32 chain chars (bit k of word j of
+  // vertex s = char first(s) + 1 + 32 j + k): {code bit 0, code bit 1, special, 0}
+  std::vector<uint32_t> lab;
+  uint64_t words = 0;
+  // order of the vertices inside every window of 256 by list length, and
+  // inside every window of 64, 128 and 256 by label length (local indexes)
+  std::vector<uint8_t> by_list;
+  std::vector<uint8_t> by_len[3];
+};
+
+HostClosure build_closure(const HostLayout& L);
+
+}  // namespace chsga

@@ -14,6 +14,8 @@
 #include <set>
 #include <type_traits>
 
+#include "bit_rows.cuh"
+#include "closure.hpp"
 #include "device_graph.hpp"
 #include "engine_api.hpp"
 #include "host_graph.hpp"
@@ -98,6 +100,10 @@ struct GraphDev {
   DevArr<uint4> t1_desc, t1_vrec;  // tiles of the one-read row kernel (k_row_t1)
   DevArr<uint8_t> t1_heads;
   DevArr<uint32_t> delta_order;    // k_row_delta: runs of 32 string vertices by decreasing char count
+  // bit-row kernels (closure.hpp)
+  DevArr<uint4> cl_rec, cl_lab;
+  DevArr<uint2> cl_ent;
+  DevArr<uint8_t> cl_by_list, cl_by_len[3];
 };
 
 struct TopDev {
@@ -119,6 +125,17 @@ struct SlotBufs {
   DevArr<unsigned long long> best;
   DevArr<dev::StepCtl> ctl;
   DevArr<dev::GridBar> bar;  // grid barrier of the persistent row-step kernel
+};
+
+// Buffers of the bit-row engine for R slots.
+struct BitBufs {
+  DevArr<unsigned char> rf[2], rl[2];  // raw first / last scores, alternating by row-step
+  DevArr<unsigned char> bits;
+  DevArr<dev::SlotState> slots;
+  DevArr<uint32_t> word;
+  DevArr<dev::StepTab> tab;
+  DevArr<unsigned long long> best;
+  DevArr<dev::StepCtl> ctl;
 };
 
 // Row kernel choice: the DPX kernel for 16-bit rows (default), the direct
@@ -147,6 +164,8 @@ struct LoadedGraph {
   dev::GraphPtrs gp{};
   std::unique_ptr<TopDev> top;
   dev::T1Ptrs t1{};  // ntiles = 0: some vertex is too long for k_row_t1
+  bool bits = false;       // the closure lists exist: rows can run on the bit-row kernels
+  dev::BitGraph bg{};      // by_len is set per kernel
   size_t pitch = 0;  // traceback matrix row stride (elements), 16-byte aligned rows
   bool nul_label = false;
   bool n_label = false;  // some label byte is 'N'
@@ -162,6 +181,7 @@ struct chsga_ctx {
   bool loaded = false;
   std::shared_ptr<chsga::LoadedGraph> g;
   std::map<int, std::unique_ptr<chsga::SlotBufs>> bufs;
+  std::map<int, std::unique_ptr<chsga::BitBufs>> bit_bufs;  // by R * 8 + sizeof(score)
   std::map<int, std::unique_ptr<chsga::RowTileDev>> row_tiles;  // by R * 8 + sizeof(score)
   // top regions other than the graph's default, by their vertex limit
   std::map<uint32_t, std::unique_ptr<chsga::TopDev>> tops;
@@ -710,6 +730,106 @@ void launch_persist(chsga_ctx& c, SlotBufs& b, uint32_t grid, uint32_t steps, cu
   CK(cudaLaunchKernelEx(&cfg, dev::k_persist<R>, a));
 }
 
+// ---- bit-row engine (bit_rows.cuh) --------------------------------------------
+
+// Whether score-only row-steps run on the bit-row kernels: the graph's
+// closure lists exist and the caller chose neither a row kernel nor a level
+// grouping (those select the level-sweep kernels).
+bool bits_apply(const chsga_ctx& c) {
+  return c.g->bits && c.row_kernel == RowKernel::Auto && c.top_sel == nullptr;
+}
+
+// 32 to 128 slots of 16-bit scores slice the bits over the slots; fewer slots,
+// 32-bit scores and vertices too long for one thread's serial chain keep a
+// read's bits in words.
+template <int R, typename ST>
+bool bits_sliced(const chsga_ctx& c) {
+  return R >= 32 && std::is_same_v<ST, uint16_t> && c.g->L.max_len <= 512;
+}
+
+template <int R, typename ST>
+BitBufs& get_bit_bufs(chsga_ctx& c) {
+  auto& b = c.bit_bufs[R * 8 + (int)sizeof(ST)];
+  if (!b) b = std::make_unique<BitBufs>();
+  const size_t S = c.g->L.S;
+  for (int i = 0; i < 2; ++i) {
+    b->rf[i].alloc(S * R * sizeof(ST));
+    b->rl[i].alloc(S * R * sizeof(ST));
+  }
+  b->bits.alloc(bits_sliced<R, ST>(c) ? (size_t)c.g->L.N * (R / 32) * 8 : (size_t)c.g->bg.words * R * 8);
+  b->slots.alloc(R);
+  b->word.alloc(R);
+  b->tab.alloc(1);
+  b->best.alloc(2 * R);
+  b->ctl.alloc(1);
+  return *b;
+}
+
+dev::AdvanceArgs advance_args(const chsga_ctx& c, dev::SlotState* slots) {
+  dev::AdvanceArgs a{};
+  a.slots = slots;
+  a.queue = c.queue.p;
+  a.reads = c.reads.p;
+  a.res_score = c.res_score.p;
+  a.res_vertex = c.res_vertex.p;
+  a.res_t0 = c.res_t0.p;
+  a.res_t1 = c.res_t1.p;
+  a.done_ring = c.done_ring.p;
+  a.qmask = c.qmask;
+  a.special = c.g->L.special;
+  a.match_n = match_n(c);
+  return a;
+}
+
+// Arguments of the row-step that reads the scores of parity `par`.
+dev::BitArgs bit_args(const chsga_ctx& c, BitBufs& b, int par) {
+  dev::BitArgs a{};
+  a.g = c.g->bg;
+  a.RFin = b.rf[par].p;
+  a.RLin = b.rl[par].p;
+  a.RFout = b.rf[par ^ 1].p;
+  a.RLout = b.rl[par ^ 1].p;
+  a.bits = b.bits.p;
+  a.word = b.word.p;
+  a.tab = b.tab.p;
+  a.best = b.best.p;
+  a.ctl = b.ctl.p;
+  a.adv = advance_args(c, b.slots.p);
+  return a;
+}
+
+template <int R, typename ST>
+void bit_step(chsga_ctx& c, BitBufs& b, int par, cudaStream_t s) {
+  dev::BitArgs a = bit_args(c, b, par);
+  if constexpr (R >= 32 && std::is_same_v<ST, uint16_t>) {
+    if (bits_sliced<R, ST>(c)) {
+      constexpr uint32_t VB = 8192 / R;
+      a.g.by_len = c.g->gd.cl_by_len[R == 128 ? 0 : R == 64 ? 1 : 2].p;
+      chain_launch(c, dev::k_row_sliced<R>, (c.g->L.S + VB - 1) / VB, 256, 0, s, a);
+      return;
+    }
+  }
+  constexpr uint32_t VB = 256 / R;
+  chain_launch(c, dev::k_row_words<R, ST, false>, (c.g->L.S + VB - 1) / VB, 256, 0, s, a);
+}
+
+template <int R>
+void bit_admit(chsga_ctx& c, BitBufs& b, cudaStream_t s) {
+  chain_launch(c, dev::k_bits_advance<R>, 1, 128, 0, s, bit_args(c, b, 0), 1);
+}
+
+// Every slot idle, q_count reads queued.
+template <int R>
+void reset_bit_slots(chsga_ctx& c, BitBufs& b, uint32_t q_count) {
+  std::vector<dev::SlotState> s(R);
+  for (auto& x : s) x = dev::SlotState{0, 0, 0, -1, 0};
+  CK(cudaMemcpyAsync(b.slots.p, s.data(), sizeof(dev::SlotState) * R, cudaMemcpyHostToDevice, c.st));
+  dev::StepCtl ctl{};
+  ctl.q_count = q_count;
+  CK(cudaMemcpyAsync(b.ctl.p, &ctl, sizeof(ctl), cudaMemcpyHostToDevice, c.st));
+  CK(cudaStreamSynchronize(c.st));  // host copies above are from stack memory
+}
+
 // Runs every queued read to completion through R slots, in blocks of
 // `per_graph` row-steps (even, so the two row buffers alternate identically
 // in every block). mode: kLaunchStream = every kernel launched from the
@@ -718,9 +838,18 @@ void launch_persist(chsga_ctx& c, SlotBufs& b, uint32_t grid, uint32_t steps, cu
 // kernel (the CUDA-graph chain where that kernel does not apply).
 template <int R, typename ST>
 void run_queue(chsga_ctx& c, uint32_t n, uint64_t total_rows, uint32_t mode, uint32_t per_graph) {
-  SlotBufs& b = get_bufs<R, ST>(c, true);
-  if (c.row_kernel == RowKernel::Tiled) row_tiles<R, ST>(c);  // allocates: never inside a capture
-  reset_slots<R>(c, b, n);
+  const bool use_bits = bits_apply(c) && mode != kLaunchPersistent;
+  SlotBufs* sb = nullptr;
+  BitBufs* bb = nullptr;
+  if (use_bits) {
+    bb = &get_bit_bufs<R, ST>(c);
+    reset_bit_slots<R>(c, *bb, n);
+  } else {
+    sb = &get_bufs<R, ST>(c, true);
+    if (c.row_kernel == RowKernel::Tiled) row_tiles<R, ST>(c);  // allocates: never inside a capture
+    reset_slots<R>(c, *sb, n);
+  }
+  dev::StepCtl* const ctl = use_bits ? bb->ctl.p : sb->ctl.p;
   const bool profile = (c.flags & CHSGA_FLAG_PROFILE) != 0;
   if (profile) mode = kLaunchStream;
   uint32_t pgrid = 0;
@@ -740,10 +869,19 @@ void run_queue(chsga_ctx& c, uint32_t n, uint64_t total_rows, uint32_t mode, uin
   CK(cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming));
   cudaGraphExec_t exec = nullptr;
   cudaGraph_t graph = nullptr;
-  ST* rows[2] = {reinterpret_cast<ST*>(b.rows[0].p), reinterpret_cast<ST*>(b.rows[1].p)};
+  auto enqueue_step = [&](uint32_t i, cudaStream_t s, StepEvents* e) {
+    if (use_bits) {
+      if (e) CK(cudaEventRecord(e->e[0], s));
+      bit_step<R, ST>(c, *bb, i & 1, s);
+      if (e)
+        for (int k = 1; k < 6; ++k) CK(cudaEventRecord(e->e[k], s));
+    } else {
+      ST* rows[2] = {reinterpret_cast<ST*>(sb->rows[0].p), reinterpret_cast<ST*>(sb->rows[1].p)};
+      row_step<R, true, ST>(c, *sb, rows[i & 1], rows[(i + 1) & 1], s, e);
+    }
+  };
   auto enqueue_block = [&](cudaStream_t s) {
-    for (uint32_t i = 0; i < per_graph; ++i)
-      row_step<R, true, ST>(c, b, rows[i & 1], rows[(i + 1) & 1], s);
+    for (uint32_t i = 0; i < per_graph; ++i) enqueue_step(i, s, nullptr);
   };
   if (use_graphs) {
     cudaStream_t cap;
@@ -760,15 +898,19 @@ void run_queue(chsga_ctx& c, uint32_t n, uint64_t total_rows, uint32_t mode, uin
   CK(cudaEventCreate(&t_start));
   CK(cudaEventCreate(&t_stop));
   CK(cudaEventRecord(t_start, c.st));
-  launch_advance<R>(c, b, 0, c.st);  // admit the first reads
+  // admit the first reads
+  if (use_bits)
+    bit_admit<R>(c, *bb, c.st);
+  else
+    launch_advance<R>(c, *sb, 0, c.st);
   auto launch_block = [&]() {
     if (mode == kLaunchPersistent) {
-      if constexpr (std::is_same_v<ST, uint16_t>) launch_persist<R>(c, b, pgrid, per_graph, c.st);
+      if constexpr (std::is_same_v<ST, uint16_t>) launch_persist<R>(c, *sb, pgrid, per_graph, c.st);
     } else if (use_graphs) {
       CK(cudaGraphLaunch(exec, c.st));
     } else if (profile) {
       for (uint32_t i = 0; i < per_graph; ++i) {
-        row_step<R, true, ST>(c, b, rows[i & 1], rows[(i + 1) & 1], c.st, sev.get());
+        enqueue_step(i, c.st, sev.get());
         sev->add(c.prof);
       }
     } else {
@@ -779,7 +921,8 @@ void run_queue(chsga_ctx& c, uint32_t n, uint64_t total_rows, uint32_t mode, uin
   // batched engine polls its done counter, one block behind the device.
   uint64_t launched = 0;
   if (R == 1) {
-    const uint64_t blocks = (total_rows + per_graph - 1) / per_graph;
+    // the bit rows take a read's closure minimum one step after its last row
+    const uint64_t blocks = (total_rows + (use_bits ? 1 : 0) + per_graph - 1) / per_graph;
     for (uint64_t i = 0; i < blocks; ++i) launch_block();
     launched = blocks;
     CK(cudaStreamSynchronize(c.st));
@@ -787,7 +930,7 @@ void run_queue(chsga_ctx& c, uint32_t n, uint64_t total_rows, uint32_t mode, uin
     const uint64_t max_blocks = total_rows / per_graph + 4;
     while (true) {
       launch_block();
-      CK(cudaMemcpyAsync(c.h_ctl.p, b.ctl.p, sizeof(dev::StepCtl), cudaMemcpyDeviceToHost, c.st));
+      CK(cudaMemcpyAsync(c.h_ctl.p, ctl, sizeof(dev::StepCtl), cudaMemcpyDeviceToHost, c.st));
       CK(cudaEventRecord(ev[launched & 1], c.st));
       ++launched;
       if (launched >= 2) {
@@ -811,14 +954,14 @@ void run_queue(chsga_ctx& c, uint32_t n, uint64_t total_rows, uint32_t mode, uin
   cudaEventDestroy(ev[0]);
   cudaEventDestroy(ev[1]);
   dev::StepCtl fin{};
-  CK(cudaMemcpy(&fin, b.ctl.p, sizeof(fin), cudaMemcpyDeviceToHost));
+  CK(cudaMemcpy(&fin, ctl, sizeof(fin), cudaMemcpyDeviceToHost));
   require_step_ok(fin.error);
   c.prof.total_ms = dev_ms;
   c.prof.rows = total_rows;
   c.prof.steps = fin.steps;
   // every kernel launched, the early-exit ones of steps after the last read included
   c.prof.launches = mode == kLaunchPersistent ? 1 + launched
-                                              : 1 + (uint64_t)kernels_per_step(c) * launched * per_graph;
+                                              : 1 + (uint64_t)(use_bits ? 1 : kernels_per_step(c)) * launched * per_graph;
   c.prof.row_launches = profile ? fin.steps : launched * per_graph;
 }
 
@@ -886,6 +1029,22 @@ void upload_graph(chsga_ctx& c, const chsga_graph_host& g) {
                           d.up_in.p,    d.dn_off.p,   d.dn_in.p,    d.istr_off.p, d.istr_src.p,
                           d.dn_head.p,  d.up_head.p,  d.fin.p,
                           (uint32_t)L.vin_srcv.size(), (uint32_t)L.up_in.size(), (uint32_t)L.dn_in.size()};
+  {
+    const HostClosure cl = build_closure(L);
+    if (cl.ok) {
+      d.cl_rec.upload(to4(cl.rec), s);
+      d.cl_lab.upload(to4(cl.lab), s);
+      std::vector<uint2> ent(cl.ent.size());
+      if (!ent.empty()) std::memcpy(ent.data(), cl.ent.data(), ent.size() * sizeof(uint2));
+      d.cl_ent.upload(ent, s);
+      d.cl_by_list.upload(cl.by_list, s);
+      for (int i = 0; i < 3; ++i) d.cl_by_len[i].upload(cl.by_len[i], s);
+      CK(cudaStreamSynchronize(s));  // the host vectors die with this scope
+      lg->bits = true;
+      lg->bg = dev::BitGraph{L.S, (uint32_t)cl.ent.size(), cl.words, d.cl_rec.p, d.cl_ent.p, d.cl_lab.p,
+                             d.cl_by_list.p, nullptr, d.sv_off.p, d.lab4.p, L.N};
+    }
+  }
   lg->nul_label = false;
   for (uint32_t i = 0; i < g.num_chars; ++i) {
     lg->nul_label |= g.labels[i] == '\0';
@@ -896,6 +1055,7 @@ void upload_graph(chsga_ctx& c, const chsga_graph_host& g) {
   lg->top = std::move(top);
   c.g = std::move(lg);
   c.bufs.clear();
+  c.bit_bufs.clear();
   c.row_tiles.clear();
   c.tops.clear();
   c.top_sel = nullptr;
@@ -1873,10 +2033,19 @@ class ScoreLaneImpl final : public ScoreLane {
     c.res_t0.alloc(cap);
     c.res_t1.alloc(cap);
     c.done_ring.alloc(cap);
-    b_ = &get_bufs<R, ST>(c, true);
-    if (c.row_kernel == RowKernel::Tiled) row_tiles<R, ST>(c);  // allocates: before the capture
-    reset_slots<R>(c, *b_, 0);
-    launch_advance<R>(c, *b_, 0, c.st);  // every slot idle
+    use_bits_ = bits_apply(c);
+    if (use_bits_) {
+      bb_ = &get_bit_bufs<R, ST>(c);
+      ctl_ = bb_->ctl.p;
+      reset_bit_slots<R>(c, *bb_, 0);
+      bit_admit<R>(c, *bb_, c.st);  // every slot idle
+    } else {
+      b_ = &get_bufs<R, ST>(c, true);
+      ctl_ = b_->ctl.p;
+      if (c.row_kernel == RowKernel::Tiled) row_tiles<R, ST>(c);  // allocates: before the capture
+      reset_slots<R>(c, *b_, 0);
+      launch_advance<R>(c, *b_, 0, c.st);  // every slot idle
+    }
     harena_.alloc(arena + 64);
     hq_.alloc(cap);
     hctl_.alloc(2);
@@ -1885,8 +2054,12 @@ class ScoreLaneImpl final : public ScoreLane {
     cudaStream_t cap_st;
     CK(cudaStreamCreateWithFlags(&cap_st, cudaStreamNonBlocking));
     CK(cudaStreamBeginCapture(cap_st, cudaStreamCaptureModeThreadLocal));
-    ST* rows[2] = {reinterpret_cast<ST*>(b_->rows[0].p), reinterpret_cast<ST*>(b_->rows[1].p)};
-    for (uint32_t i = 0; i < per_; ++i) row_step<R, true, ST>(c, *b_, rows[i & 1], rows[(i + 1) & 1], cap_st);
+    if (use_bits_) {
+      for (uint32_t i = 0; i < per_; ++i) bit_step<R, ST>(c, *bb_, i & 1, cap_st);
+    } else {
+      ST* rows[2] = {reinterpret_cast<ST*>(b_->rows[0].p), reinterpret_cast<ST*>(b_->rows[1].p)};
+      for (uint32_t i = 0; i < per_; ++i) row_step<R, true, ST>(c, *b_, rows[i & 1], rows[(i + 1) & 1], cap_st);
+    }
     CK(cudaStreamEndCapture(cap_st, &graph_));
     CK(cudaGraphInstantiate(&exec_, graph_, 0));
     CK(cudaStreamDestroy(cap_st));
@@ -1905,10 +2078,10 @@ class ScoreLaneImpl final : public ScoreLane {
   uint64_t arena_bytes() const override { return arena_; }
   unsigned char* staging() override { return harena_.p; }
   uint64_t blocks() const override { return launched_; }
-  uint32_t kernels_per_block() const override { return kernels_per_step(*c_) * per_; }
+  uint32_t kernels_per_block() const override { return (use_bits_ ? 1 : kernels_per_step(*c_)) * per_; }
 
   void inject_wait_timeout() override {
-    dev::k_wait_selftest<<<1, 32, 0, c_->st>>>(b_->ctl.p, 4096);
+    dev::k_wait_selftest<<<1, 32, 0, c_->st>>>(ctl_, 4096);
     check_launch();
   }
 
@@ -1932,7 +2105,7 @@ class ScoreLaneImpl final : public ScoreLane {
       CK(cudaMemcpyAsync(c.queue.p, hq_.p, (n - n1) * sizeof(dev::ReadDesc), cudaMemcpyHostToDevice,
                          c.st));
     qpub_ += n;
-    k_publish<<<1, 1, 0, c.st>>>(b_->ctl.p, qpub_);
+    k_publish<<<1, 1, 0, c.st>>>(ctl_, qpub_);
     check_launch();
   }
 
@@ -1940,7 +2113,7 @@ class ScoreLaneImpl final : public ScoreLane {
     chsga_ctx& c = *c_;
     const int k = (int)(launched_ & 1);
     CK(cudaGraphLaunch(exec_, c.st));
-    CK(cudaMemcpyAsync(hctl_.p + k, b_->ctl.p, sizeof(dev::StepCtl), cudaMemcpyDeviceToHost, c.st));
+    CK(cudaMemcpyAsync(hctl_.p + k, ctl_, sizeof(dev::StepCtl), cudaMemcpyDeviceToHost, c.st));
     CK(cudaMemcpyAsync(hring_.p + (size_t)k * cap_, c.done_ring.p, (size_t)cap_ * sizeof(dev::CompletionRec),
                        cudaMemcpyDeviceToHost, c.st));
     CK(cudaEventRecord(ev_[k], c.st));
@@ -1991,6 +2164,9 @@ class ScoreLaneImpl final : public ScoreLane {
 
   chsga_ctx* c_;
   SlotBufs* b_ = nullptr;
+  BitBufs* bb_ = nullptr;
+  dev::StepCtl* ctl_ = nullptr;
+  bool use_bits_ = false;
   uint32_t cap_;
   uint64_t arena_;
   uint32_t per_ = 8;
