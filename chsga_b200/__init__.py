@@ -421,6 +421,20 @@ def _read_ptrs(reads: Sequence[bytes]):
     return arr, lens
 
 
+_OP_DTYPE = np.dtype([("row", "<i8"), ("vertex", "<u4"), ("op", "u1"), ("pad", "u1", 3)])
+
+
+def _ops_array(r: TbResult) -> np.ndarray:
+    """The result's ops as an int64 array of (row, vertex, op)."""
+    n = int(r.num_ops)
+    ops = np.zeros((n, 3), dtype=np.int64)
+    if n:
+        raw = np.frombuffer(C.string_at(r.ops, n * _OP_DTYPE.itemsize), dtype=_OP_DTYPE)
+        for j, f in enumerate(("row", "vertex", "op")):
+            ops[:, j] = raw[f]
+    return ops
+
+
 class Context:
     """A device context with a loaded graph (chsga_open + chsga_load_graph)."""
 
@@ -495,12 +509,7 @@ class Context:
         r = TbResult()
         self._ck(_lib.chsga_align_traceback(self._h, read, len(read), C.byref(o), C.byref(r)))
         try:
-            n = int(r.num_ops)
-            ops = np.zeros((n, 3), dtype=np.int64)
-            for i in range(n):
-                x = r.ops[i]
-                ops[i] = (x.row, x.vertex, x.op)
-            return ops, int(r.score), bool(r.checkpointed)
+            return _ops_array(r), int(r.score), bool(r.checkpointed)
         finally:
             _lib.chsga_tb_result_free(C.byref(r))
 
@@ -515,12 +524,7 @@ class Context:
         out = []
         for i in range(len(reads)):
             r = res[i]
-            n = int(r.num_ops)
-            ops = np.zeros((n, 3), dtype=np.int64)
-            for j in range(n):
-                x = r.ops[j]
-                ops[j] = (x.row, x.vertex, x.op)
-            out.append((ops, int(r.score), bool(r.checkpointed)))
+            out.append((_ops_array(r), int(r.score), bool(r.checkpointed)))
             _lib.chsga_tb_result_free(C.byref(r))
         return out
 
@@ -621,12 +625,7 @@ class Server:
             r = buf[i]
             d = {k: getattr(r, k) for k, _ in ServerResult._fields_ if k not in ("tb", "pad", "pad2")}
             if r.mode == REQ_TRACEBACK:
-                m = int(r.tb.num_ops)
-                ops = np.zeros((m, 3), dtype=np.int64)
-                for j in range(m):
-                    x = r.tb.ops[j]
-                    ops[j] = (x.row, x.vertex, x.op)
-                d["ops"] = ops
+                d["ops"] = _ops_array(r.tb)
                 d["checkpointed"] = bool(r.tb.checkpointed)
                 _lib.chsga_tb_result_free(C.byref(r.tb))
             out.append(d)

@@ -12,8 +12,8 @@
 // RF and RL alternate between two buffers (other vertices gather the old
 // ones); the bits are the vertex's own and are updated in place, or written
 // into the read's matrix (traceback). Nothing orders one vertex after
-// another, so the row-step has no phases between blocks, and the block that
-// finishes last moves the slots on (bits_advance).
+// another, so the row-step has no phases between blocks; every block moves
+// the slots on for itself at its start (bits_head).
 //
 // A row's minimum after its closure needs the closure's first scores, which
 // the next row-step computes: a read on its last row leaves its slot with its
@@ -31,27 +31,16 @@
 namespace chsga {
 namespace dev {
 
-constexpr uint32_t SW_DRAIN = 1u << 13;  // the slot's previous read takes its closure minimum
-constexpr uint32_t SW_PAR = 1u << 14;    // which of the slot's two minima its current read uses
-
-// Words of the current row-step for the bit-sliced kernel, written by
-// bits_advance: per label key the mismatch bits of 32 slots, and the same per
-// slot as 16-bit increments; row-0 (or idle), last-row and draining slots.
-struct StepTab {
-  uint32_t mis[8][4];
-  uint32_t keep[4];   // 0 where the slot is on row 0 or idle
-  uint32_t end[4];
-  uint32_t drain[4];
-  uint32_t any_end, any_drain, pad[2];
-  uint16_t mis16[8][128];
-  uint16_t init16[128];  // 0xFFFF on row 0 or idle
-};
+constexpr uint32_t SW_DRAIN = 1u << 13;     // the slot's previous read takes its closure minimum
+constexpr uint32_t SW_PAR_SHIFT = 14;       // bits 14..15: which of the slot's four minima its read uses
+constexpr uint32_t kBitsNarrowMax = 32767;  // longest read whose sums need no saturation
 
 struct BitGraph {
   uint32_t S, n_ent;
   uint64_t words;
   const uint4* rec;       // closure.hpp
-  const uint2* ent;
+  const uint2* ent;       // {source, weight}
+  const uint2* ent16;     // {source, weight for M | weight for F << 16}, 0xFFFF = none
   const uint4* lab;
   const uint8_t* by_list;
   const uint8_t* by_len;  // of the kernel's window
@@ -67,8 +56,23 @@ struct SlotRows {
   unsigned char* cur;
 };
 
-struct AdvanceArgs {
-  SlotState* slots;
+// The slots before a row-step; every launch reads one and writes the other.
+// SlotState::pad: (id of the draining read + 1) << 2 | minimum of the slot.
+struct BitState {
+  SlotState s[128];
+  SlotRows rows[128];  // traceback
+  uint32_t q_head, pad[3];
+};
+
+struct BitArgs {
+  BitGraph g;
+  const void *RFin, *RLin;
+  void *RFout, *RLout;
+  void* bits;  // uint2 words (one read a word) or bit-sliced char words
+  const BitState* st_in;
+  BitState* st_out;
+  unsigned long long* best;  // [4][R]
+  StepCtl* ctl;
   const ReadDesc* queue;
   const unsigned char* reads;
   int32_t* res_score;
@@ -77,179 +81,130 @@ struct AdvanceArgs {
   CompletionRec* done_ring;
   uint32_t qmask;
   int special, match_n;
-  // traceback: matrix of every read id and the slots' row pointers
-  unsigned char* const* mats;
-  SlotRows* rows;
+  unsigned char* const* mats;  // traceback: matrix of every read id
   size_t pitch;
 };
 
-struct BitArgs {
-  BitGraph g;
-  const void *RFin, *RLin;
-  void *RFout, *RLout;
-  void* bits;  // uint2 words (one read a word) or bit-sliced char words
-  uint32_t* word;
-  StepTab* tab;
-  unsigned long long* best;  // [2][R]
-  StepCtl* ctl;
-  AdvanceArgs adv;
+// What a row-step has to do, the same in every block.
+struct HeadFlags {
+  bool work, end, drain, init, wide;
 };
 
-// Moves every slot to its next row (one block, at least R threads): finishes
-// the reads that drained, lets reads past their last row drain, admits queued
-// reads and writes the slot words and tables of the next row-step. prime:
-// only the first admission (nothing was computed yet).
+// Moves the slots to the row-step about to run. Every block does it for
+// itself from the state the launch before left (a few hundred bytes), so no
+// block waits for one that advances the slots after all others are done;
+// block 0 also finishes the reads that drained, writes the new state and
+// counts the step. Admission is by slot order from the queue's head, so the
+// blocks agree. word: the slots' words (shared memory, R entries); rows: the
+// slots' row pointers (traceback, else null).
+//
+// A read's minimum is reset when it is read out, by block 0 of the step
+// after its drain, while other blocks may already take minima of the slot's
+// next but one read: with four minima a slot that is another one.
 template <int R>
-__device__ void bits_advance(const AdvanceArgs& a, uint32_t* slot_word, StepTab* tab, unsigned long long* best,
-                             StepCtl* ctl, bool prime) {
+__device__ __forceinline__ HeadFlags bits_head(const BitArgs& a, uint32_t* word, SlotRows* rows) {
   static_assert(R <= 128, "one thread per slot");
-  __shared__ uint32_t s_need[128];
-  __shared__ uint32_t s_base, s_take, s_active, s_ending, s_drain;
-  const int r = threadIdx.x;
+  __shared__ uint32_t s_cnt[4], s_flag[4];
+  const int r = threadIdx.x, lane = r & 31, wp = r >> 5;
+  constexpr int NW = R < 32 ? 1 : R / 32;
+  const bool first = blockIdx.x == 0 && blockIdx.y == 0;
   SlotState st{};
-  bool need = false;
-  uint32_t drain = 0, par = 0;
-  if (r == 0) s_active = s_ending = s_drain = 0;
   SlotRows sr{nullptr, nullptr};
-  if (r < R) {
-    st = a.slots[r];
-    par = st.pad & 1u;
-    if (a.mats) sr = a.rows[r];
-    sr.prev = sr.cur;
-    if (!prime) {
-      const int32_t did = (int32_t)(st.pad >> 1) - 1;
-      if (did >= 0) {
-        const unsigned long long b = __ldcg(best + (par ^ 1u) * R + r);
-        const unsigned long long t1 = global_ns();
+  bool need = false, wide = false;
+  uint32_t drain = 0, par = 0, q_head = 0, avail = 0;
+  unsigned before = 0;
+  if (wp < NW) {
+    if (r < R) {
+      st = a.st_in->s[r];
+      q_head = a.st_in->q_head;
+      avail = a.ctl->q_count - q_head;
+      par = st.pad & 3u;
+      if (a.mats) {
+        sr = a.st_in->rows[r];
+        sr.prev = sr.cur;
+      }
+      const int32_t did = (int32_t)(st.pad >> 2) - 1;
+      if (did >= 0 && first) {
+        unsigned long long* bp = a.best + ((par + 3u) & 3u) * R + r;
+        const unsigned long long b = __ldcg(bp), t1 = global_ns();
+        *bp = ~0ull;
         a.res_score[did] = (int32_t)(b >> 32);
         a.res_vertex[did] = (uint32_t)(b & 0xffffffffu);
         a.res_t1[did] = t1;
-        const uint32_t k = atomicAdd(&ctl->done, 1u);
+        const uint32_t k = atomicAdd(&a.ctl->done, 1u);
         if (a.done_ring)
           a.done_ring[k & a.qmask] = CompletionRec{did, (int32_t)(b >> 32), (uint32_t)(b & 0xffffffffu), 0u,
                                                    a.res_t0[did], t1};
       }
+      wide = st.id >= 0 && st.len > kBitsNarrowMax;  // also while it drains
       if (st.id >= 0) {
         if (st.row + 1 >= st.len) {
           drain = (uint32_t)st.id + 1;
           st.id = -1;
-          par ^= 1u;
+          par = (par + 1u) & 3u;
         } else {
           st.row += 1;
         }
       }
+      need = st.id < 0;
     }
-    need = st.id < 0;
+    const unsigned nb = __ballot_sync(0xFFFFFFFFu, need);
+    before = __popc(nb & ((1u << lane) - 1u));
+    if (lane == 0) s_cnt[wp] = __popc(nb);
   }
-  if (r < 128) s_need[r] = need ? 1u : 0u;
-  __syncthreads();
-  if (r == 0) {
+  if constexpr (NW > 1)
+    __syncthreads();
+  else
+    __syncwarp();
+  if (wp < NW) {
     uint32_t total = 0;
-    for (int i = 0; i < R; ++i) {
-      const uint32_t n = s_need[i];
-      s_need[i] = total;
-      total += n;
-    }
-    const uint32_t avail = ctl->q_count - ctl->q_head;
-    s_take = total < avail ? total : avail;
-    s_base = ctl->q_head;
-    ctl->q_head += s_take;
-  }
-  __syncthreads();
-  uint32_t w = 0;
-  if (r < R) {
-    if (need && s_need[r] < s_take) {
-      const ReadDesc q = a.queue[(s_base + s_need[r]) & a.qmask];
-      st.off = q.off;
-      st.len = q.len;
-      st.row = 0;
-      st.id = q.id;
-      best[par * R + r] = ~0ull;
-      a.res_t0[q.id] = global_ns();
-    }
-    if (st.id >= 0) {
-      const int byte = a.reads[st.off + st.row];
-      w = base_code(byte, a.special) | (mismatch_mask(byte, a.special, a.match_n) << SW_MASK_SHIFT) | SW_ACTIVE;
-      w |= st.row == 0 ? SW_INIT : SW_CLOSURE;
-      if (st.row + 1 == st.len) w |= SW_ENDING;
-      if (a.mats) sr.cur = a.mats[st.id] + (size_t)st.row * a.pitch;
-    }
-    if (drain) w |= SW_DRAIN;
-    if (par) w |= SW_PAR;
-    st.pad = drain << 1 | par;
-    if (w & (SW_ACTIVE | SW_DRAIN)) atomicOr(&s_active, 1u);
-    if (w & SW_ENDING) atomicOr(&s_ending, 1u);
-    if (w & SW_DRAIN) atomicOr(&s_drain, 1u);
-    a.slots[r] = st;
-    slot_word[r] = w;
-    if (a.mats) a.rows[r] = sr;
-  }
-  if constexpr (R >= 32) {
-    if (r < R) {
-      const bool init = (w & SW_INIT) || !(w & SW_ACTIVE);
-      const uint32_t m = (w >> SW_MASK_SHIFT) & SW_MASK;
-      const int g = r >> 5;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const uint32_t bit = (m >> k) & 1u;
-        const uint32_t word = __ballot_sync(0xFFFFFFFFu, bit);
-        if ((r & 31) == 0) tab->mis[k][g] = word;
-        tab->mis16[k][r] = (uint16_t)bit;
+    for (int i = 0; i < NW; ++i) {
+      if (i < wp) before += s_cnt[i];
+      total += s_cnt[i];
+    }
+    uint32_t w = 0;
+    if (r < R) {
+      if (need && before < avail) {
+        const ReadDesc q = a.queue[(q_head + before) & a.qmask];
+        st.off = q.off;
+        st.len = q.len;
+        st.row = 0;
+        st.id = q.id;
+        if (first) a.res_t0[q.id] = global_ns();
       }
-      tab->init16[r] = init ? 0xFFFFu : 0u;
-      const uint32_t ki = __ballot_sync(0xFFFFFFFFu, !init), ke = __ballot_sync(0xFFFFFFFFu, (w & SW_ENDING) != 0),
-                     kd = __ballot_sync(0xFFFFFFFFu, (w & SW_DRAIN) != 0);
-      if ((r & 31) == 0) {
-        tab->keep[g] = ki;
-        tab->end[g] = ke;
-        tab->drain[g] = kd;
+      if (st.id >= 0) {
+        const int byte = a.reads[st.off + st.row];
+        w = base_code(byte, a.special) | (mismatch_mask(byte, a.special, a.match_n) << SW_MASK_SHIFT) | SW_ACTIVE;
+        w |= st.row == 0 ? SW_INIT : SW_CLOSURE;
+        if (st.row + 1 == st.len) w |= SW_ENDING;
+        if (a.mats) sr.cur = a.mats[st.id] + (size_t)st.row * a.pitch;
+      }
+      if (drain) w |= SW_DRAIN;
+      w |= par << SW_PAR_SHIFT;
+      word[r] = w;
+      if (rows) rows[r] = sr;
+      if (first) {
+        st.pad = drain << 2 | par;
+        a.st_out->s[r] = st;
+        if (a.mats) a.st_out->rows[r] = sr;
+        if (r == 0) a.st_out->q_head = q_head + (total < avail ? total : avail);
       }
     }
+    const bool act = (w & SW_ACTIVE) != 0;
+    const uint32_t f = (__any_sync(0xFFFFFFFFu, (w & (SW_ACTIVE | SW_DRAIN)) != 0) ? 1u : 0u) |
+                       (__any_sync(0xFFFFFFFFu, (w & SW_ENDING) != 0) ? 2u : 0u) |
+                       (__any_sync(0xFFFFFFFFu, (w & SW_DRAIN) != 0) ? 4u : 0u) |
+                       (__any_sync(0xFFFFFFFFu, r < R && (!act || (w & SW_INIT))) ? 8u : 0u) |
+                       (__any_sync(0xFFFFFFFFu, wide) ? 16u : 0u);
+    if (lane == 0) s_flag[wp] = f;
   }
   __syncthreads();
-  if (r == 0) {
-    if constexpr (R >= 32) {
-      tab->any_end = s_ending;
-      tab->any_drain = s_drain;
-    }
-    ctl->any_active = s_active;
-    ctl->any_ending = s_ending | s_drain;
-    ctl->arrive = 0;
-    if (s_active) ctl->steps += 1;
-  }
-}
-
-template <int R>
-__global__ void __launch_bounds__(128) k_bits_advance(BitArgs a, int prime) {
-  pdl_wait();
-  bits_advance<R>(a.adv, a.word, a.tab, a.best, a.ctl, prime != 0);
-}
-
-// The last block of the launch moves the slots on. Every thread's writes of
-// this block are ordered before the arrival (block barrier, then a fence by
-// the arriving thread); the last arrival's block sees them all.
-template <int R>
-__device__ __forceinline__ void bits_finish(const BitArgs& a, uint32_t nblocks) {
-  __shared__ uint32_t s_last;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    s_last = atomicAdd(&a.ctl->arrive, 1u) == nblocks - 1;
-    __threadfence();
-  }
-  __syncthreads();
-  if (s_last) bits_advance<R>(a.adv, a.word, a.tab, a.best, a.ctl, false);
-}
-
-// Nothing to compute in this launch: true, and when reads wait in the queue
-// (published to an idle engine) the launch still ends in their admission.
-// Every block takes the same way: only the last arrival changes the words
-// this reads.
-template <int R>
-__device__ __forceinline__ bool bits_idle(const BitArgs& a, uint32_t nblocks) {
-  if (a.ctl->any_active) return false;
-  if (a.ctl->q_count != a.ctl->q_head) bits_finish<R>(a, nblocks);
-  return true;
+  uint32_t f = 0;
+#pragma unroll
+  for (int i = 0; i < NW; ++i) f |= s_flag[i];
+  if (first && threadIdx.x == 0 && (f & 1u)) a.ctl->steps += 1;
+  return HeadFlags{(f & 1u) != 0, (f & 2u) != 0, (f & 4u) != 0, (f & 8u) != 0, (f & 16u) != 0};
 }
 
 // Row layout of a traceback matrix: bit words, raw first scores, first
@@ -270,50 +225,53 @@ __host__ __device__ constexpr size_t bits_row_bytes(uint64_t words, uint32_t S) 
 // matrix. Vertices of a 256-vertex window are taken by list length, so a
 // warp's lists end together.
 // ---------------------------------------------------------------------------
-template <int R, typename ST, bool MAT>
-__global__ void __launch_bounds__(256) k_row_words(BitArgs a) {
+#ifndef CHSGA_WORDS_THREADS
+#define CHSGA_WORDS_THREADS 1280  // threads per SM the register budget is sized for (build-time tuning)
+#endif
+template <int R, typename ST, int H, int NT>
+__global__ void __launch_bounds__(NT, CHSGA_WORDS_THREADS / NT) k_row_words(BitArgs a) {
+  constexpr bool MAT = H > 0;
+  constexpr int SLOTS = MAT ? H : R;
   static_assert(!MAT || (R == 1 && sizeof(ST) == 2), "matrix rows hold one slot each, 16 bits");
+  static_assert(NT >= (SLOTS < 32 ? 32 : SLOTS), "the head needs a thread per slot");
   using bits::PN;
-  constexpr int VB = 256 / R;  // vertices per block
+  constexpr int VB = NT / R;  // vertices per block and turn
   const BitGraph& g = a.g;
-  const int r = MAT ? (int)blockIdx.y : (int)(threadIdx.x % R);
-  const uint32_t i = blockIdx.x * VB + threadIdx.x / R;  // position in the windows' order
+  __shared__ uint32_t s_word[SLOTS];
+  __shared__ SlotRows s_rows[MAT ? SLOTS : 1];
+  __shared__ unsigned long long s_min[4 * R];
+  const int r = (int)(threadIdx.x % R);  // of this block's slots
+  uint32_t i = blockIdx.x * VB + threadIdx.x / R;  // position in the windows' order
   uint32_t s = 0;
   uint4 rec = make_uint4(0, 1, 0, 0);
-  if (i < g.S) {
-    s = (i & ~255u) + __ldg(g.by_list + i);
-    s = CHSGA_CHK(s, g.S, 20);
-    rec = __ldg(g.rec + s);
-  }
+  auto fetch = [&] {
+    if (i < g.S) {
+      s = CHSGA_CHK((i & ~255u) + __ldg(g.by_list + i), g.S, 20);
+      rec = __ldg(g.rec + s);
+    }
+  };
+  fetch();
   pdl_wait();
-  if constexpr (MAT) {
-    if (!a.ctl->any_active) return;
-  } else {
-    if (bits_idle<R>(a, gridDim.x)) return;
-  }
-  const uint32_t w = a.word[r];
+  for (int k = threadIdx.x; k < 4 * R; k += NT) s_min[k] = ~0ull;
+  const HeadFlags hf = bits_head<SLOTS>(a, s_word, MAT ? s_rows : nullptr);
+  if (!hf.work) return;
+  const uint32_t w = s_word[MAT ? blockIdx.y : r];
   const bool init = (w & SW_INIT) != 0;
-  constexpr int NB = R;  // minima per block
-  __shared__ unsigned long long s_min[2 * NB];
-  const bool ends = a.ctl->any_ending != 0;
-  if (ends) {
-    if (threadIdx.x < 2 * NB) s_min[threadIdx.x] = ~0ull;
-    __syncthreads();
-  }
+  const uint32_t par = (w >> SW_PAR_SHIFT) & 3u;
   const ST *RFin, *RLin;
   ST *RFout, *RLout, *Fout = nullptr;
   const uint2* win;
   uint2* wout;
   if constexpr (MAT) {
-    const SlotRows sr = a.adv.rows[r];
+    const SlotRows sr = s_rows[blockIdx.y];
     const size_t rf = bits_row_rf(g.words);
     RFin = reinterpret_cast<const ST*>(sr.prev + rf);
     RFout = reinterpret_cast<ST*>(sr.cur + rf);
     Fout = reinterpret_cast<ST*>(sr.prev + bits_row_f(g.words, g.S));
     win = reinterpret_cast<const uint2*>(sr.prev);
     wout = reinterpret_cast<uint2*>(sr.cur);
-    RLin = static_cast<const ST*>(a.RLin) + (size_t)r * g.S;
-    RLout = static_cast<ST*>(a.RLout) + (size_t)r * g.S;
+    RLin = static_cast<const ST*>(a.RLin) + (size_t)blockIdx.y * g.S;
+    RLout = static_cast<ST*>(a.RLout) + (size_t)blockIdx.y * g.S;
   } else {
     RFin = static_cast<const ST*>(a.RFin) + r;
     RLin = static_cast<const ST*>(a.RLin) + r;
@@ -322,12 +280,13 @@ __global__ void __launch_bounds__(256) k_row_words(BitArgs a) {
     win = static_cast<const uint2*>(a.bits) + r;
     wout = static_cast<uint2*>(a.bits) + r;
   }
-  if (i < g.S && (w & (SW_ACTIVE | SW_DRAIN))) {
-    const uint32_t len = rec.y & 0x1FFFFFFFu, key = rec.y >> 29, mask = (w >> SW_MASK_SHIFT) & SW_MASK;
+  const uint32_t mask = (w >> SW_MASK_SHIFT) & SW_MASK;
+  for (; i - threadIdx.x / R < g.S && (w & (SW_ACTIVE | SW_DRAIN)); i += gridDim.x * VB, fetch()) {
+    if (i >= g.S) break;
+    const uint32_t len = rec.y & 0x1FFFFFFFu, key = rec.y >> 29;
     const uint32_t nb = rec.w & 0xFFu, nm = (rec.w >> 8) & 0xFFu, nf = (rec.w >> 16) & 0xFFu;
     const uint32_t nw = (len + 30) / 32;
     const int delta = (int)((mask >> key) & 1u);
-    unsigned long long mn = ~0ull;
     // closure of the previous row (a no-op on row 0: its scores are 0 and 1
     // and every weight is at least 1)
     int rf = 0, F = 0, M = 0x3fffffff, dl = 0;
@@ -355,10 +314,9 @@ __global__ void __launch_bounds__(256) k_row_words(BitArgs a) {
             if (k + u < kb || k + u >= km) F = min(F, x[u] + (k + u < kb ? 1 : 0));
           }
       }
-      if (MAT && (w & SW_DRAIN || !init)) Fout[s] = (ST)F;
-      if (w & SW_DRAIN) mn = pack_min(F, __ldg(g.sv_off + s));
+      if constexpr (MAT) Fout[s] = (ST)F;
+      if (w & SW_DRAIN) atomicMin(&s_min[((par + 3u) & 3u) * R + r], pack_min(F, __ldg(g.sv_off + s)));
     }
-    if (w & SW_DRAIN) atomicMin(&s_min[(((w & SW_PAR) ? 0 : 1)) * NB + (MAT ? 0 : r)], mn);
     if (w & SW_ACTIVE) {
       int T, last;
       if (init) {
@@ -406,20 +364,211 @@ __global__ void __launch_bounds__(256) k_row_words(BitArgs a) {
             }
           }
         }
-        atomicMin(&s_min[((w & SW_PAR) ? 1 : 0) * NB + (MAT ? 0 : r)], pack_min(bm, bc));
+        atomicMin(&s_min[par * R + r], pack_min(bm, bc));
       }
     }
   }
-  if (ends) {
+  if (hf.end || hf.drain) {
     __syncthreads();
-    // the minima's array is [parity][slot]
-    const int slots = MAT ? (int)gridDim.y : R;
-    if (threadIdx.x < 2 * NB && s_min[threadIdx.x] != ~0ull) {
-      const int p = threadIdx.x / NB, q = MAT ? r : (int)(threadIdx.x % NB);
-      atomicMin(a.best + (MAT ? p * slots : p * NB) + q, s_min[threadIdx.x]);
+    for (int k = threadIdx.x; k < 4 * R; k += NT)
+      if (s_min[k] != ~0ull) atomicMin(a.best + (MAT ? k * SLOTS + (int)blockIdx.y : k), s_min[k]);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// k_close_row: the final row (after its closure) of a row-step state, as the
+// 32-bit scores of every char: one thread per string vertex (checkpoint
+// files).
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) k_close_row(BitGraph g, const uint2* __restrict__ bits,
+                                                   const uint16_t* __restrict__ RF,
+                                                   const uint16_t* __restrict__ RL, int* __restrict__ out) {
+  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= g.S) return;
+  const uint4 rec = __ldg(g.rec + s);
+  const uint32_t nb = rec.w & 0xFFu, nm = (rec.w >> 8) & 0xFFu, nf = (rec.w >> 16) & 0xFFu;
+  int F = RF[s], cur = F;
+  for (uint32_t k = rec.z; k < rec.z + nb + nm + nf; ++k) {
+    if (k >= rec.z + nb && k < rec.z + nb + nm) continue;
+    const uint2 e = __ldg(g.ent + k);
+    F = min(F, (int)RL[e.x] + (int)e.y + (k < rec.z + nb ? 1 : 0));
+  }
+  const uint32_t f = __ldg(g.sv_off + s), len = rec.y & 0x1FFFFFFFu;
+  out[f] = F;
+  for (uint32_t k = 0; k + 1 < len; ++k) {
+    const uint2 x = bits[rec.x + (k >> 5)];
+    cur += (int)((x.x >> (k & 31u)) & 1u) - (int)((x.y >> (k & 31u)) & 1u);
+    out[f + 1 + k] = min(cur, F + (int)(k + 1));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// k_walk_bits: k_walk over a matrix of bit rows (row i at M + (i - row_lo) *
+// pitch), one warp. The path stays in a vertex for about as many rows as the
+// vertex has chars, so on entering one every lane loads that vertex's words
+// of one row (31 rows ahead) and the steps inside it only shuffle; at a first
+// char every lane takes one in-edge. One thread reading the rows one after
+// another pays a memory round trip a row. Same tie order as k_walk.
+// ---------------------------------------------------------------------------
+struct BitRowView {
+  const unsigned char* M;
+  size_t pitch, rf, f;
+  __device__ __forceinline__ int first_raw(long long i, uint32_t s) const {
+    return reinterpret_cast<const uint16_t*>(M + (size_t)i * pitch + rf)[s];
+  }
+  __device__ __forceinline__ int first_final(long long i, uint32_t s) const {
+    return reinterpret_cast<const uint16_t*>(M + (size_t)i * pitch + f)[s];
+  }
+  __device__ __forceinline__ uint2 word(long long i, uint32_t w) const {
+    return reinterpret_cast<const uint2*>(M + (size_t)i * pitch)[w];
+  }
+  // final score of char k of the vertex with record words at wo
+  __device__ __forceinline__ int score(long long i, uint32_t s, uint32_t wo, uint32_t k) const {
+    int cur = first_raw(i, s);
+    const int F = first_final(i, s);
+    for (uint32_t j = 0; 32 * j < k; ++j) {
+      const uint2 x = word(i, wo + j);
+      const uint32_t m = k - 32 * j >= 32 ? 0xFFFFFFFFu : (1u << (k - 32 * j)) - 1u;
+      cur += __popc(x.x & m) - __popc(x.y & m);
+    }
+    return min(cur, F + (int)k);
+  }
+};
+
+__global__ void __launch_bounds__(32) k_walk_bits(GraphPtrs g, BitGraph bg, const unsigned char* __restrict__ M,
+                                                  size_t pitch, long long row_lo, long long row_hi, uint32_t start,
+                                                  const unsigned char* __restrict__ read, WalkOp* __restrict__ ops,
+                                                  uint32_t max_ops, WalkOut* __restrict__ out, int match_n) {
+  constexpr unsigned FULL = 0xFFFFFFFFu;
+  const int lane = threadIdx.x;
+  const BitRowView v{M, pitch, bits_row_rf(bg.words), bits_row_f(bg.words, bg.S)};
+  uint32_t lo = 0, hi = g.S;
+  while (hi - lo > 1) {
+    const uint32_t m = (lo + hi) / 2;
+    if (g.sv_off[m] <= start) lo = m; else hi = m;
+  }
+  uint32_t sv = lo, n = 0;
+  long long row = row_hi;
+  int status = 0, fail_row = 0;
+  uint32_t first = g.sv_off[sv], k = start - first;  // char k of vertex sv
+  uint32_t wo = bg.rec[sv].x;
+  // lane j: vertex sv in row held - j (its first word, enough up to char 32)
+  long long held = -1;
+  int h_rf = 0, h_f = 0;
+  uint2 h_w = make_uint2(0, 0);
+  uint32_t h_key = 0, h_byte = 0;
+  auto hold = [&] {
+    held = row;
+    const long long i = row - lane;
+    if (i >= row_lo) {
+      h_rf = v.first_raw(i - row_lo, sv);
+      h_f = v.first_final(i - row_lo, sv);
+      if (k > 0) h_w = v.word(i - row_lo, wo);
+      h_byte = read[i];
+    }
+    // label keys of the chars k, k - 1, ... of the vertex
+    h_key = (uint32_t)lane <= k ? label_key(g, first + k - (uint32_t)lane) : 0u;
+  };
+  uint32_t held_k = 0;
+  auto at = [&](long long i, uint32_t kk) -> int {  // final score of char kk in row i (held or held - 1 .. - 31)
+    if (kk > 32) return v.score(i - row_lo, sv, wo, kk);
+    const int j = (int)(held - i);
+    const int rf = __shfl_sync(FULL, h_rf, j), f = __shfl_sync(FULL, h_f, j);
+    const uint32_t p = __shfl_sync(FULL, h_w.x, j), m = __shfl_sync(FULL, h_w.y, j);
+    const uint32_t mask = kk >= 32 ? 0xFFFFFFFFu : (1u << kk) - 1u;
+    return min(rf + __popc(p & mask) - __popc(m & mask), f + (int)kk);
+  };
+  hold();
+  held_k = k;
+  int s = at(row, k);
+  while (row > row_lo) {
+    if (n >= max_ops) {
+      status = 8;
+      fail_row = (int)row;
+      break;
+    }
+    if (held - row >= 31 || held_k - k >= 31) {
+      hold();
+      held_k = k;
+    }
+    uint32_t op = 255, src_sv = sv, src_k = k;
+    int src_s = 0;
+    // scores of up to 32 in-neighbours' last chars in row i: the first (in
+    // list order) with value + add == s
+    auto from_edges = [&](const uint32_t* list, uint32_t e0, uint32_t e1, long long i, int add, bool& found) {
+      for (uint32_t b = e0; b < e1 && !found; b += 32) {
+        uint32_t u = 0, kl = 0;
+        int x = 0x3fffffff;
+        if (b + lane < e1) {
+          u = list[b + lane];
+          const uint4 rec = bg.rec[u];
+          kl = (rec.y & 0x1FFFFFFFu) - 1;
+          x = v.score(i - row_lo, u, rec.x, kl);
+        }
+        const unsigned hit = __ballot_sync(FULL, x + add == s);
+        if (hit) {
+          const int l = __ffs(hit) - 1;
+          src_sv = __shfl_sync(FULL, u, l);
+          src_k = __shfl_sync(FULL, kl, l);
+          src_s = __shfl_sync(FULL, x, l);
+          found = true;
+        }
+      }
+    };
+    bool found = false;
+    if (k > 0) {
+      const int x = at(row, k - 1);
+      if (x + 1 == s) {
+        op = 2;
+        src_k = k - 1;
+        src_s = x;
+      }
+    } else {
+      from_edges(g.istr_src, g.istr_off[sv], g.istr_off[sv + 1], row, 1, found);
+      if (found) op = 2;
+    }
+    if (op == 255) {
+      const int x = at(row - 1, k);
+      if (x + 1 == s) {
+        op = 0;
+        src_s = x;
+      }
+    }
+    if (op == 255) {
+      const uint32_t key = __shfl_sync(FULL, h_key, (int)(held_k - k));
+      const int byte = (int)__shfl_sync(FULL, h_byte, (int)(held - row));
+      const int delta = (int)((mismatch_mask(byte, g.special, match_n) >> key) & 1u);
+      if (k > 0) {
+        const int x = at(row - 1, k - 1);
+        if (x + delta == s) {
+          op = 1;
+          src_k = k - 1;
+          src_s = x;
+        }
+      } else {
+        from_edges(g.vin_srcv, g.vin_off[sv], g.vin_off[sv + 1], row - 1, delta, found);
+        if (found) op = 1;
+      }
+    }
+    if (op == 255) {
+      status = 7;
+      fail_row = (int)row;
+      break;
+    }
+    if (lane == 0) ops[n] = WalkOp{row, first + k, op};
+    ++n;
+    if (op != 2) --row;
+    s = src_s;
+    k = src_k;
+    if (src_sv != sv || found) {  // an in-edge may lead back to the same vertex (cycles)
+      sv = src_sv;
+      first = g.sv_off[sv];
+      wo = bg.rec[sv].x;
+      if (row > row_lo) hold();
+      held_k = k;
     }
   }
-  if constexpr (!MAT) bits_finish<R>(a, gridDim.x);
+  if (lane == 0) *out = WalkOut{first + k, n, status, fail_row};
 }
 
 // ---------------------------------------------------------------------------
@@ -498,133 +647,146 @@ __device__ __noinline__ void line_slot(uint2* p, int W, uint32_t n, uint32_t bit
 #ifndef CHSGA_SLICED_BLOCKS
 #define CHSGA_SLICED_BLOCKS 4  // blocks per SM the register budget is sized for (build-time tuning)
 #endif
-template <int R>
-__global__ void __launch_bounds__(256, CHSGA_SLICED_BLOCKS) k_row_sliced(BitArgs a) {
-  constexpr int C = R / 8, W = R / 32, VB = 8192 / R, NT = 256;
+__device__ __forceinline__ uint4 viaddmin4(const uint4& a, uint32_t w, const uint4& c) {  // min(a + w, c), no half wraps
+  return make_uint4(__viaddmin_u16x2(a.x, w, c.x), __viaddmin_u16x2(a.y, w, c.y), __viaddmin_u16x2(a.z, w, c.z),
+                    __viaddmin_u16x2(a.w, w, c.w));
+}
+
+enum { G0, G1, VP, VN, GBIG, LOW, NPL };
+
+// Shared memory of a k_row_sliced block: K times 256 (vertex, 8 slots) items.
+template <int R, int K>
+struct SlicedShared {
+  static constexpr int C = R / 8, W = R / 32, NT = 256, VB = K * NT / C;
+  uint16_t F[VB * R];
+  uint16_t mis16[8][R];
+  uint16_t init[R];
+  uint8_t P[NPL][VB * C];
+  uint32_t mis[8 * W], keep[W], end[W], word[R];
+  unsigned long long best[4 * R];
+};
+
+// The windows of one block. WIDE: some read is so long that a sum of a score
+// and a weight may leave 16 bits (saturating sums).
+template <int R, int K, bool WIDE>
+__device__ __forceinline__ void sliced_windows(const BitArgs& a, const HeadFlags& hf, SlicedShared<R, K>& sh) {
+  constexpr int C = R / 8, W = R / 32, NT = 256, VB = K * NT / C;
   constexpr uint32_t ONES = 0x00010001u;
   const BitGraph& g = a.g;
-  __shared__ __align__(16) uint16_t sF[VB * R];
-  enum { G0, G1, VP, VN, GBIG, LOW, NPL };
-  __shared__ __align__(4) uint8_t sP[NPL][VB * C];
-  __shared__ __align__(16) uint4 sMis16[8 * C], sInit[C];
-  __shared__ uint32_t sMis[8 * W], sKeep[W], sEnd[W];
-  __shared__ unsigned long long sMin[2 * R];
-  const uint32_t v0 = blockIdx.x * VB;
-  const uint32_t nv = min((uint32_t)VB, g.S - v0);
-  pdl_wait();
-  if (bits_idle<R>(a, gridDim.x)) return;
-  const StepTab* tab = a.tab;
-  const bool ends = a.ctl->any_ending != 0;
-  for (int i = threadIdx.x; i < 8 * C; i += NT)
-    sMis16[i] = *(reinterpret_cast<const uint4*>(tab->mis16[i / C]) + i % C);
-  if (threadIdx.x < C) sInit[threadIdx.x] = *(reinterpret_cast<const uint4*>(tab->init16) + threadIdx.x);
-  if (threadIdx.x < 8 * W) sMis[threadIdx.x] = tab->mis[threadIdx.x / W][threadIdx.x % W];
-  if (threadIdx.x < W) {
-    sKeep[threadIdx.x] = tab->keep[threadIdx.x];
-    sEnd[threadIdx.x] = tab->end[threadIdx.x];
-  }
-  if (ends)
-    for (int i = threadIdx.x; i < 2 * R; i += NT) sMin[i] = ~0ull;
-  __syncthreads();
   const uint16_t* RFin = static_cast<const uint16_t*>(a.RFin);
   const uint16_t* RLin = static_cast<const uint16_t*>(a.RLin);
   uint16_t* RFout = static_cast<uint16_t*>(a.RFout);
   uint16_t* RLout = static_cast<uint16_t*>(a.RLout);
-  const bool drains = ends && tab->any_drain != 0;
-  // ---- pass 1
-  for (uint32_t it = threadIdx.x; it < nv * C; it += NT) {
-    const uint32_t vl = it / C, q = it % C, s = v0 + vl;
-    const uint4 rec = __ldg(g.rec + s);
-    const uint32_t key = rec.y >> 29;
-    const size_t so = (size_t)s * R + 8 * q;
-    const uint4 rf = __ldg(reinterpret_cast<const uint4*>(RFin + so));
-    const uint32_t nb = rec.w & 0xFFu, nm = (rec.w >> 8) & 0xFFu, nf = (rec.w >> 16) & 0xFFu;
-    uint32_t k0 = rec.z, k1 = k0 + nb + nm + nf;
-    CHSGA_CHK_RANGE(k0, k1, g.n_ent, 21);
-    const uint32_t kb = k0 + nb, km = kb + nm;
-    uint4 F = rf, M = make_uint4(~0u, ~0u, ~0u, ~0u);
-    constexpr int U = 4;
-    for (uint32_t k = k0; k < k1; k += U) {
-      uint2 e[U];
-      uint4 x[U];
+  const uint4 zero = make_uint4(0, 0, 0, 0), one = make_uint4(ONES, ONES, ONES, ONES);
+  for (uint32_t v0 = blockIdx.x * VB; v0 < g.S; v0 += gridDim.x * VB) {
+    const uint32_t nv = min((uint32_t)VB, g.S - v0);
+    // ---- pass 1
+    for (uint32_t it = threadIdx.x; it < nv * C; it += NT) {
+      const uint32_t vl = it / C, q = it % C, s = v0 + vl;
+      const uint4 rec = __ldg(g.rec + s);
+      const uint32_t key = rec.y >> 29;
+      const size_t so = (size_t)s * R + 8 * q;
+      const uint4 rf = __ldg(reinterpret_cast<const uint4*>(RFin + so));
+      uint32_t k0 = rec.z, k1 = k0 + (rec.w & 0xFFu) + ((rec.w >> 8) & 0xFFu) + ((rec.w >> 16) & 0xFFu);
+      CHSGA_CHK_RANGE(k0, k1, g.n_ent, 21);
+      const uint4 d = *reinterpret_cast<const uint4*>(&sh.mis16[key][8 * q]);
+      uint4 F = rf, M, T;
+      constexpr int U = 4;
+      {
+        // no source: above every score, and one more does not wrap
+        const uint32_t none = WIDE ? 0xFFFFFFFFu : 0x80008000u;
+        M = make_uint4(none, none, none, none);
+        for (uint32_t k = k0; k < k1; k += U) {
+          uint2 e[U];
+          uint4 x[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (k + u < k1) e[u] = __ldg(g.ent + k + u);
+          for (int u = 0; u < U; ++u)
+            if (k + u < k1) e[u] = __ldg(g.ent16 + k + u);
 #pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (k + u < k1)
-          x[u] = __ldg(reinterpret_cast<const uint4*>(RLin + (size_t)CHSGA_CHK(e[u].x, g.S, 22) * R + 8 * q));
+          for (int u = 0; u < U; ++u)
+            if (k + u < k1)
+              x[u] = __ldg(reinterpret_cast<const uint4*>(RLin + (size_t)CHSGA_CHK(e[u].x, g.S, 22) * R + 8 * q));
 #pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (k + u < k1) {
-          const uint4 y = addw4(x[u], min(e[u].y, 0xFFFFu) * ONES);
-          if (k + u < km) M = min4(M, y);
-          if (k + u < kb)
-            F = min4(F, addw4(y, ONES));
-          else if (k + u >= km)
-            F = min4(F, y);
+          for (int u = 0; u < U; ++u)
+            if (k + u < k1) {
+              const uint32_t ww = WIDE ? e[u].y : __vminu2(e[u].y, 0x80008000u);
+              const uint32_t wm = __byte_perm(ww, 0, 0x1010), wf = __byte_perm(ww, 0, 0x3232);
+              if (WIDE) {
+                M = min4(M, addw4(x[u], wm));
+                F = min4(F, addw4(x[u], wf));
+              } else {
+                M = viaddmin4(x[u], wm, M);
+                F = viaddmin4(x[u], wf, F);
+              }
+            }
         }
-    }
-    const uint4 d = sMis16[key * C + q], in = sInit[q];
-    const uint4 one = make_uint4(ONES, ONES, ONES, ONES);
-    uint4 T = min4(addw4(F, ONES), add4(M, d));
-    T = sel4(d, T, in);
-    *reinterpret_cast<uint4*>(RFout + so) = T;
-    *reinterpret_cast<uint4*>(sF + vl * R + 8 * q) = F;
-    if (drains) {
-      const uint32_t f = __ldg(g.sv_off + s), fw[4] = {F.x, F.y, F.z, F.w};
-#pragma unroll
-      for (int v = 0; v < 8; ++v) {
-        const uint32_t w = a.word[8 * q + v];
-        if (w & SW_DRAIN)
-          atomicMin(&sMin[((w & SW_PAR) ? 0 : R) + 8 * q + v],
-                    pack_min((int)((fw[v >> 1] >> (16 * (v & 1))) & 0xFFFFu), f));
+        const uint4 F1 = make_uint4(F.x + ONES, F.y + ONES, F.z + ONES, F.w + ONES);
+        if (WIDE)
+          T = min4(F1, add4(M, d));
+        else
+          T = make_uint4(__viaddmin_u16x2(M.x, d.x, F1.x), __viaddmin_u16x2(M.y, d.y, F1.y),
+                         __viaddmin_u16x2(M.z, d.z, F1.z), __viaddmin_u16x2(M.w, d.w, F1.w));
       }
+      uint4 in = zero;
+      if (hf.init) {
+        in = *reinterpret_cast<const uint4*>(sh.init + 8 * q);
+        T = sel4(d, T, in);
+      }
+      *reinterpret_cast<uint4*>(RFout + so) = T;
+      *reinterpret_cast<uint4*>(sh.F + vl * R + 8 * q) = F;
+      if (hf.drain) {
+        const uint32_t f = __ldg(g.sv_off + s), fw[4] = {F.x, F.y, F.z, F.w};
+#pragma unroll
+        for (int v = 0; v < 8; ++v) {
+          const uint32_t w = sh.word[8 * q + v];
+          if (w & SW_DRAIN)
+            atomicMin(&sh.best[((w >> SW_PAR_SHIFT) + 3u & 3u) * R + 8 * q + v],
+                      pack_min((int)((fw[v >> 1] >> (16 * (v & 1))) & 0xFFFFu), f));
+        }
+      }
+      // chain start: not below F - 1 (max(T + 1, F) - 1; no half wraps)
+      const uint4 T1 = max4(make_uint4(T.x + ONES, T.y + ONES, T.z + ONES, T.w + ONES), F);  // + 1
+      uint4 low = sub4(sub4(T1, one), T), gap = sub4(rf, F);
+      uint4 ch = sub4(T1, F);  // change of the first score + 1: 0..2
+      if (hf.init) {  // row 0: its mismatch + 1
+        low = sel4(zero, low, in);
+        gap = sel4(zero, gap, in);
+        ch = sel4(make_uint4(d.x + ONES, d.y + ONES, d.z + ONES, d.w + ONES), ch, in);
+      }
+      uint32_t g0, g1, c0, c1, big = 0;
+      if ((gap.x | gap.y | gap.z | gap.w) & 0xFFFCFFFCu) {
+        big = nonzero8(make_uint4(gap.x & 0xFFFCFFFCu, gap.y & 0xFFFCFFFCu, gap.z & 0xFFFCFFFCu, gap.w & 0xFFFCFFFCu));
+        const uint4 b16 = unplane(big);
+        gap = sel4(zero, gap, make_uint4(b16.x * 0xFFFFu, b16.y * 0xFFFFu, b16.z * 0xFFFFu, b16.w * 0xFFFFu));
+      }
+      planes2(gap, g0, g1);
+      planes2(ch, c0, c1);
+      const uint32_t at = vl * C + q;
+      sh.P[G0][at] = (uint8_t)g0;
+      sh.P[G1][at] = (uint8_t)g1;
+      sh.P[VP][at] = (uint8_t)c1;
+      sh.P[VN][at] = (uint8_t)(~(c0 | c1));
+      sh.P[GBIG][at] = (uint8_t)big;
+      sh.P[LOW][at] = (low.x | low.y | low.z | low.w) ? (uint8_t)nonzero8(low) : (uint8_t)0;
     }
-    // F - 1 never drops below 0 where it matters: T >= 0
-    const uint4 Fm = make_uint4(__vsubus2(F.x, ONES), __vsubus2(F.y, ONES), __vsubus2(F.z, ONES), __vsubus2(F.w, ONES));
-    const uint4 Tc = max4(T, Fm);
-    const uint4 zero = make_uint4(0, 0, 0, 0);
-    const uint4 gap = sel4(zero, sub4(rf, F), in), low = sel4(zero, sub4(Tc, T), in);
-    // change of the first score + 1: 0..2 (row 0: its mismatch + 1)
-    const uint4 ch = sel4(add4(d, one), sub4(add4(Tc, one), F), in);
-    uint32_t g0, g1, c0, c1, big = 0;
-    uint4 gl = gap;
-    if ((gap.x | gap.y | gap.z | gap.w) & 0xFFFCFFFCu) {
-      big = nonzero8(make_uint4(gap.x & 0xFFFCFFFCu, gap.y & 0xFFFCFFFCu, gap.z & 0xFFFCFFFCu, gap.w & 0xFFFCFFFCu));
-      const uint4 b16 = unplane(big);
-      const uint4 keepm = make_uint4(b16.x * 0xFFFFu, b16.y * 0xFFFFu, b16.z * 0xFFFFu, b16.w * 0xFFFFu);
-      gl = sel4(zero, gap, keepm);
-    }
-    planes2(gl, g0, g1);
-    planes2(ch, c0, c1);
-    const uint32_t at = vl * C + q;
-    sP[G0][at] = (uint8_t)g0;
-    sP[G1][at] = (uint8_t)g1;
-    sP[VP][at] = (uint8_t)c1;
-    sP[VN][at] = (uint8_t)(~(c0 | c1));
-    sP[GBIG][at] = (uint8_t)big;
-    sP[LOW][at] = (low.x | low.y | low.z | low.w) ? (uint8_t)nonzero8(low) : (uint8_t)0;
-  }
-  __syncthreads();
-  // ---- pass 2
-  {
-    const uint32_t vi = threadIdx.x / W, w = threadIdx.x % W;
-    if (vi < nv) {
-      const uint32_t vl = CHSGA_CHK((uint32_t)__ldg(g.by_len + v0 + vi), nv, 24);
+    __syncthreads();
+    // ---- pass 2
+    for (uint32_t t = threadIdx.x; t < nv * W; t += NT) {
+      const uint32_t vi = t / W, w = t % W;
+      const uint32_t vl = K == 4 ? CHSGA_CHK((uint32_t)__ldg(g.by_len + v0 + vi), nv, 24) : vi;
       const uint32_t s = v0 + vl;
       uint32_t f = __ldg(g.sv_off + s), e = __ldg(g.sv_off + s + 1);
       CHSGA_CHK_CHARS(f, e, g.N, 1);
       const uint32_t n = e - f - 1;  // chain chars
       uint2* z = static_cast<uint2*>(a.bits) + (size_t)(f + 1) * W + w;
-      auto plane = [&](int p) { return reinterpret_cast<const uint32_t*>(sP[p])[vl * W + w]; };
-      uint32_t vp = plane(VP), vn = plane(VN);
-      const uint32_t keep = sKeep[w], low = plane(LOW);
+      auto plane = [&](int p) { return reinterpret_cast<const uint32_t*>(sh.P[p])[vl * W + w]; };
       if (n) {
+        uint32_t vp = plane(VP), vn = plane(VN);
+        const uint32_t keep = sh.keep[w];
         uint32_t g0 = plane(G0), g1 = plane(G1);
         for (uint32_t big = plane(GBIG); big; big &= big - 1) {
           const uint32_t b = __ffs(big) - 1, r = 32 * w + b;
-          line_slot(z, W, n, 1u << b, (uint32_t)RFin[(size_t)s * R + r] - sF[vl * R + r]);
+          line_slot(z, W, n, 1u << b, (uint32_t)RFin[(size_t)s * R + r] - sh.F[vl * R + r]);
         }
         // label keys, 8 chars a word
         const uint32_t* kp = g.lab4 + ((f + 1) >> 3);
@@ -642,7 +804,7 @@ __global__ void __launch_bounds__(256, CHSGA_SLICED_BLOCKS) k_row_sliced(BitArgs
 #pragma unroll
           for (int u = 0; u < U; ++u)
             if (c + u < n) {
-              const uint32_t d = sMis[((keys >> (4 * u)) & 7u) * W + w];
+              const uint32_t d = sh.mis[((keys >> (4 * u)) & 7u) * W + w];
               const uint32_t p = x[u].x, m = x[u].y;
               // the previous row under its line (row 0 slots have none)
               const uint32_t t0 = g0 & ~m;
@@ -651,26 +813,25 @@ __global__ void __launch_bounds__(256, CHSGA_SLICED_BLOCKS) k_row_sliced(BitArgs
               const uint32_t b = g1 & ~(g0 ^ m);
               g1 &= p | t0;
               g0 = (p & g0) | (~p & b);
-              // new score is 1 above the char's left neighbour of the
-              // previous row, else level with it
-              const uint32_t t = d & ~(vn | hn);
-              const uint32_t op = vn | (t & ~vp), om = vp & ~t;
-              vp = hn | (t & ~hp);
-              vn = hp & ~t;
+              // the new score is 1 above the previous row's left neighbour, else level with it
+              const uint32_t t1 = d & ~(vn | hn);
+              const uint32_t op = vn | (t1 & ~vp), om = vp & ~t1;
+              vp = hn | (t1 & ~hp);
+              vn = hp & ~t1;
               z[u * W] = make_uint2(op, om);
             }
           z += U * W;
         }
         z = static_cast<uint2*>(a.bits) + (size_t)(f + 1) * W + w;
-        for (uint32_t lb = low; lb; lb &= lb - 1) {
+        for (uint32_t lb = plane(LOW); lb; lb &= lb - 1) {
           const uint32_t b = __ffs(lb) - 1, r = 32 * w + b;
-          line_slot(z, W, n, 1u << b, (uint32_t)sF[vl * R + r] - 1u - RFout[(size_t)s * R + r]);
+          line_slot(z, W, n, 1u << b, (uint32_t)sh.F[vl * R + r] - 1u - RFout[(size_t)s * R + r]);
         }
-        reinterpret_cast<uint32_t*>(sP[VP])[vl * W + w] = vp;
-        reinterpret_cast<uint32_t*>(sP[VN])[vl * W + w] = vn;
+        reinterpret_cast<uint32_t*>(sh.P[VP])[vl * W + w] = vp;
+        reinterpret_cast<uint32_t*>(sh.P[VN])[vl * W + w] = vn;
       }
-      if (ends) {
-        for (uint32_t eb = sEnd[w]; eb; eb &= eb - 1) {
+      if (hf.end) {
+        for (uint32_t eb = sh.end[w]; eb; eb &= eb - 1) {
           const uint32_t b = __ffs(eb) - 1, r = 32 * w + b;
           int cur = RFout[(size_t)s * R + r], bm = cur;
           uint32_t bc = f;
@@ -682,37 +843,71 @@ __global__ void __launch_bounds__(256, CHSGA_SLICED_BLOCKS) k_row_sliced(BitArgs
               bc = f + 1 + c;
             }
           }
-          atomicMin(&sMin[((a.word[r] & SW_PAR) ? R : 0) + r], pack_min(bm, bc));
+          atomicMin(&sh.best[((sh.word[r] >> SW_PAR_SHIFT) & 3u) * R + r], pack_min(bm, bc));
         }
       }
     }
-  }
-  __syncthreads();
-  // ---- pass 3
-  for (uint32_t it = threadIdx.x; it < nv * C; it += NT) {
-    const uint32_t vl = it / C, q = it % C, s = v0 + vl;
-    const uint32_t len = __ldg(&g.rec[s].y) & 0x1FFFFFFFu;
-    const size_t so = (size_t)s * R + 8 * q;
-    uint4 o;
-    if (len == 1) {
-      o = *reinterpret_cast<const uint4*>(RFout + so);
-    } else {
-      const uint32_t lw = min(len - 1, 0xFFFFu) * ONES, at = vl * C + q;
-      const uint4 F = *reinterpret_cast<const uint4*>(sF + vl * R + 8 * q);
-      o = min4(__ldg(reinterpret_cast<const uint4*>(RLin + so)), addw4(F, lw));
-      o = sel4(make_uint4(0, 0, 0, 0), o, sInit[q]);
-      const uint4 p = unplane(sP[VP][at]), m = unplane(sP[VN][at]);
-      o = make_uint4(o.x + p.x - m.x, o.y + p.y - m.y, o.z + p.z - m.z, o.w + p.w - m.w);
-      if (sP[LOW][at]) o = min4(o, addw4(*reinterpret_cast<const uint4*>(RFout + so), lw));
-    }
-    *reinterpret_cast<uint4*>(RLout + so) = o;
-  }
-  if (ends) {
     __syncthreads();
-    for (int i = threadIdx.x; i < 2 * R; i += NT)
-      if (sMin[i] != ~0ull) atomicMin(a.best + i, sMin[i]);
+    // ---- pass 3 (first + len - 1 stays below 2^16: the kernel runs up to 512 chars)
+    for (uint32_t it = threadIdx.x; it < nv * C; it += NT) {
+      const uint32_t vl = it / C, q = it % C, s = v0 + vl;
+      const uint32_t len = __ldg(&g.rec[s].y) & 0x1FFFFFFFu;
+      const size_t so = (size_t)s * R + 8 * q;
+      uint4 o;
+      if (len == 1) {
+        o = *reinterpret_cast<const uint4*>(RFout + so);
+      } else {
+        const uint32_t lw = (len - 1) * ONES, at = vl * C + q;
+        o = viaddmin4(*reinterpret_cast<const uint4*>(sh.F + vl * R + 8 * q), lw,
+                      __ldg(reinterpret_cast<const uint4*>(RLin + so)));
+        if (hf.init) o = sel4(zero, o, *reinterpret_cast<const uint4*>(sh.init + 8 * q));
+        const uint4 p = unplane(sh.P[VP][at]), m = unplane(sh.P[VN][at]);
+        o = make_uint4(o.x + p.x - m.x, o.y + p.y - m.y, o.z + p.z - m.z, o.w + p.w - m.w);
+        if (sh.P[LOW][at]) o = viaddmin4(*reinterpret_cast<const uint4*>(RFout + so), lw, o);
+      }
+      *reinterpret_cast<uint4*>(RLout + so) = o;
+    }
+    __syncthreads();  // the next window reuses the shared arrays
   }
-  bits_finish<R>(a, gridDim.x);
+}
+
+template <int R, int K>
+__global__ void __launch_bounds__(256, CHSGA_SLICED_BLOCKS) k_row_sliced(BitArgs a) {
+  using Shared = SlicedShared<R, K>;
+  constexpr int NT = Shared::NT, W = Shared::W;
+  __shared__ __align__(16) Shared sh;
+  pdl_wait();
+  const HeadFlags hf = bits_head<R>(a, sh.word, nullptr);
+  if (!hf.work) return;
+  // the step's words: per label key the mismatches of 32 slots, and as 16-bit increments
+  for (int i = threadIdx.x; i < R; i += NT) {
+    const uint32_t w = sh.word[i], m = (w >> SW_MASK_SHIFT) & SW_MASK;
+    const bool init = (w & SW_INIT) || !(w & SW_ACTIVE);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      sh.mis16[k][i] = (uint16_t)((m >> k) & 1u);
+      const uint32_t b = __ballot_sync(0xFFFFFFFFu, (m >> k) & 1u);
+      if ((i & 31) == 0) sh.mis[k * W + (i >> 5)] = b;
+    }
+    sh.init[i] = init ? 0xFFFFu : 0u;
+    const uint32_t bk = __ballot_sync(0xFFFFFFFFu, !init), be = __ballot_sync(0xFFFFFFFFu, (w & SW_ENDING) != 0);
+    if ((i & 31) == 0) {
+      sh.keep[i >> 5] = bk;
+      sh.end[i >> 5] = be;
+    }
+  }
+  const bool ends = hf.end || hf.drain;
+  if (ends)
+    for (int i = threadIdx.x; i < 4 * R; i += NT) sh.best[i] = ~0ull;
+  __syncthreads();
+  if (hf.wide)
+    sliced_windows<R, K, true>(a, hf, sh);
+  else
+    sliced_windows<R, K, false>(a, hf, sh);
+  if (ends) {
+    for (int i = threadIdx.x; i < 4 * R; i += NT)
+      if (sh.best[i] != ~0ull) atomicMin(a.best + i, sh.best[i]);
+  }
 }
 
 }  // namespace dev

@@ -208,6 +208,17 @@ HostClosure build_closure(const HostLayout& L) {
       if (x & 4) w[2] |= bit;
     }
   }
+  c.ent16.resize(2 * c.ent.size());
+#pragma omp parallel for schedule(static)
+  for (int64_t s = 0; s < (int64_t)S; ++s) {
+    const uint32_t n = c.rec[4 * s + 3], kb = e_cnt[s] + (n & 255), km = kb + ((n >> 8) & 255);
+    for (uint32_t k = e_cnt[s]; k < e_cnt[s + 1]; ++k) {
+      const uint32_t w = std::min<uint32_t>((uint32_t)c.ent[k].w, 0xFFFE), none = 0xFFFF;
+      const uint32_t wm = k < km ? w : none, wf = k < kb ? w + 1 : k >= km ? w : none;
+      c.ent16[2 * (size_t)k] = (uint32_t)c.ent[k].src;
+      c.ent16[2 * (size_t)k + 1] = wm | wf << 16;
+    }
+  }
   auto windows = [&](std::vector<uint8_t>& out, uint32_t W, auto&& weight) {
     out.resize(S);
 #pragma omp parallel for schedule(static)

@@ -52,6 +52,9 @@ struct HostClosure {
   // vertex s = char first(s) + 1 + 32 j + k): {code bit 0, code bit 1, special, 0}
   std::vector<uint32_t> lab;
   uint64_t words = 0;
+  // the entries for 16-bit rows: {source, weight for M | weight for F << 16},
+  // 0xFFFF = no such entry (or a weight no 16-bit score can win with)
+  std::vector<uint32_t> ent16;
   // order of the vertices inside every window of 256 by list length, and
   // inside every window of 64, 128 and 256 by label length (local indexes)
   std::vector<uint8_t> by_list;

@@ -102,7 +102,7 @@ struct GraphDev {
   DevArr<uint32_t> delta_order;    // k_row_delta: runs of 32 string vertices by decreasing char count
   // bit-row kernels (closure.hpp)
   DevArr<uint4> cl_rec, cl_lab;
-  DevArr<uint2> cl_ent;
+  DevArr<uint2> cl_ent, cl_ent16;
   DevArr<uint8_t> cl_by_list, cl_by_len[3];
 };
 
@@ -131,9 +131,7 @@ struct SlotBufs {
 struct BitBufs {
   DevArr<unsigned char> rf[2], rl[2];  // raw first / last scores, alternating by row-step
   DevArr<unsigned char> bits;
-  DevArr<dev::SlotState> slots;
-  DevArr<uint32_t> word;
-  DevArr<dev::StepTab> tab;
+  DevArr<dev::BitState> state;  // [2], alternating by row-step
   DevArr<unsigned long long> best;
   DevArr<dev::StepCtl> ctl;
 };
@@ -212,6 +210,11 @@ struct chsga_ctx {
   chsga::PinnedArr<chsga::dev::StepCtl> h_ctl;
   chsga::PinnedArr<int32_t> h_ckpt;     // checkpoint rows of the checkpointed traceback (int32 rows)
   chsga::PinnedArr<uint16_t> h_ckpt16;  // the same for 16-bit rows
+  // traceback on bit rows: checkpoint states, a matrix of up to kKeepMatrix
+  // bytes kept between calls, the matrix pointer and the walk's output
+  chsga::PinnedArr<unsigned char> h_ckbits, h_walk;
+  chsga::DevArr<unsigned char> tb_mat, tb_walk;
+  chsga::DevArr<unsigned char*> tb_ptr;
   chsga_profile prof{};
 };
 
@@ -757,17 +760,25 @@ BitBufs& get_bit_bufs(chsga_ctx& c) {
     b->rl[i].alloc(S * R * sizeof(ST));
   }
   b->bits.alloc(bits_sliced<R, ST>(c) ? (size_t)c.g->L.N * (R / 32) * 8 : (size_t)c.g->bg.words * R * 8);
-  b->slots.alloc(R);
-  b->word.alloc(R);
-  b->tab.alloc(1);
-  b->best.alloc(2 * R);
+  b->state.alloc(2);
+  b->best.alloc(4 * R);
   b->ctl.alloc(1);
   return *b;
 }
 
-dev::AdvanceArgs advance_args(const chsga_ctx& c, dev::SlotState* slots) {
-  dev::AdvanceArgs a{};
-  a.slots = slots;
+// Arguments of the row-step that reads the scores of parity `par`.
+dev::BitArgs bit_args(const chsga_ctx& c, BitBufs& b, int par) {
+  dev::BitArgs a{};
+  a.g = c.g->bg;
+  a.RFin = b.rf[par].p;
+  a.RLin = b.rl[par].p;
+  a.RFout = b.rf[par ^ 1].p;
+  a.RLout = b.rl[par ^ 1].p;
+  a.bits = b.bits.p;
+  a.st_in = b.state.p + par;
+  a.st_out = b.state.p + (par ^ 1);
+  a.best = b.best.p;
+  a.ctl = b.ctl.p;
   a.queue = c.queue.p;
   a.reads = c.reads.p;
   a.res_score = c.res_score.p;
@@ -781,52 +792,88 @@ dev::AdvanceArgs advance_args(const chsga_ctx& c, dev::SlotState* slots) {
   return a;
 }
 
-// Arguments of the row-step that reads the scores of parity `par`.
-dev::BitArgs bit_args(const chsga_ctx& c, BitBufs& b, int par) {
-  dev::BitArgs a{};
-  a.g = c.g->bg;
-  a.RFin = b.rf[par].p;
-  a.RLin = b.rl[par].p;
-  a.RFout = b.rf[par ^ 1].p;
-  a.RLout = b.rl[par ^ 1].p;
-  a.bits = b.bits.p;
-  a.word = b.word.p;
-  a.tab = b.tab.p;
-  a.best = b.best.p;
-  a.ctl = b.ctl.p;
-  a.adv = advance_args(c, b.slots.p);
-  return a;
+// Blocks of `threads` threads of kernel k that fit the device at once.
+uint32_t resident_blocks(const chsga_ctx& c, const void* k, int threads) {
+  int per_sm = 0;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, 0));
+  return (uint32_t)std::max(per_sm, 1) * (uint32_t)c.num_sms;
 }
 
 template <int R, typename ST>
 void bit_step(chsga_ctx& c, BitBufs& b, int par, cudaStream_t s) {
   dev::BitArgs a = bit_args(c, b, par);
+  const uint32_t S = c.g->L.S;
   if constexpr (R >= 32 && std::is_same_v<ST, uint16_t>) {
     if (bits_sliced<R, ST>(c)) {
-      constexpr uint32_t VB = 8192 / R;
       a.g.by_len = c.g->gd.cl_by_len[R == 128 ? 0 : R == 64 ? 1 : 2].p;
-      chain_launch(c, dev::k_row_sliced<R>, (c.g->L.S + VB - 1) / VB, 256, 0, s, a);
+      // windows of 8192 / R vertices where they fill the device, else a
+      // quarter of that: a small graph's row-step is as long as one block's
+      auto launch = [&](auto kern, uint32_t VB) {
+        const uint32_t wins = (S + VB - 1) / VB;
+        chain_launch(c, kern, std::min(wins, resident_blocks(c, (const void*)kern, 256)), 256, 0, s, a);
+      };
+      if (S >= 8192 / R * 2u * (uint32_t)c.num_sms)
+        launch(dev::k_row_sliced<R, 4>, 8192 / R);
+      else
+        launch(dev::k_row_sliced<R, 1>, 2048 / R);
       return;
     }
   }
-  constexpr uint32_t VB = 256 / R;
-  chain_launch(c, dev::k_row_words<R, ST, false>, (c.g->L.S + VB - 1) / VB, 256, 0, s, a);
+  auto launch = [&](auto kern, uint32_t threads) {
+    const uint32_t VB = threads / R;
+    chain_launch(c, kern, std::min((S + VB - 1) / VB, resident_blocks(c, (const void*)kern, (int)threads)), threads, 0, s, a);
+  };
+  if constexpr (R <= 64) {
+    // fewer threads a block where blocks of 256 would leave SMs idle
+    if ((uint64_t)S * R < 256ull * 2 * c.num_sms) return launch(dev::k_row_words<R, ST, 0, 64>, 64);
+  }
+  launch(dev::k_row_words<R, ST, 0, 256>, 256);
 }
 
-template <int R>
-void bit_admit(chsga_ctx& c, BitBufs& b, cudaStream_t s) {
-  chain_launch(c, dev::k_bits_advance<R>, 1, 128, 0, s, bit_args(c, b, 0), 1);
+// Buffers of H slots whose rows go to their reads' matrices (traceback): the
+// raw last scores alternate here, one slot after another.
+template <int H>
+BitBufs& get_mat_bufs(chsga_ctx& c) {
+  auto& b = c.bit_bufs[-H];
+  if (!b) b = std::make_unique<BitBufs>();
+  for (auto& r : b->rl) r.alloc((size_t)c.g->L.S * H * 2);
+  b->state.alloc(2);
+  b->best.alloc(4 * H);
+  b->ctl.alloc(1);
+  return *b;
+}
+
+size_t bit_row_bytes(const chsga_ctx& c) { return dev::bits_row_bytes(c.g->bg.words, c.g->L.S); }
+
+// Row-step of H slots with rows of bit_row_bytes in mats[read id].
+template <int H>
+void mat_step(chsga_ctx& c, BitBufs& b, unsigned char* const* mats, int par, cudaStream_t s) {
+  dev::BitArgs a = bit_args(c, b, par);
+  a.mats = mats;
+  a.pitch = bit_row_bytes(c);
+  const uint32_t S = c.g->L.S;
+  auto launch = [&](auto kern, uint32_t threads) {
+    const uint32_t res = std::max(1u, resident_blocks(c, (const void*)kern, (int)threads) / H);
+    chain_launch(c, kern, dim3(std::min((S + threads - 1) / threads, res), H), threads, 0, s, a);
+  };
+  if ((uint64_t)S * H < 256ull * 2 * c.num_sms)
+    launch(dev::k_row_words<1, uint16_t, H, 64>, 64);
+  else
+    launch(dev::k_row_words<1, uint16_t, H, 256>, 256);
 }
 
 // Every slot idle, q_count reads queued.
 template <int R>
 void reset_bit_slots(chsga_ctx& c, BitBufs& b, uint32_t q_count) {
-  std::vector<dev::SlotState> s(R);
-  for (auto& x : s) x = dev::SlotState{0, 0, 0, -1, 0};
-  CK(cudaMemcpyAsync(b.slots.p, s.data(), sizeof(dev::SlotState) * R, cudaMemcpyHostToDevice, c.st));
+  std::vector<dev::BitState> st(1);
+  for (auto& x : st[0].s) x = dev::SlotState{0, 0, 0, -1, 0};
+  for (auto& x : st[0].rows) x = dev::SlotRows{nullptr, nullptr};
+  st[0].q_head = 0;
+  CK(cudaMemcpyAsync(b.state.p, st.data(), sizeof(dev::BitState), cudaMemcpyHostToDevice, c.st));
   dev::StepCtl ctl{};
   ctl.q_count = q_count;
   CK(cudaMemcpyAsync(b.ctl.p, &ctl, sizeof(ctl), cudaMemcpyHostToDevice, c.st));
+  CK(cudaMemsetAsync(b.best.p, 0xFF, 4 * R * sizeof(unsigned long long), c.st));
   CK(cudaStreamSynchronize(c.st));  // host copies above are from stack memory
 }
 
@@ -898,11 +945,8 @@ void run_queue(chsga_ctx& c, uint32_t n, uint64_t total_rows, uint32_t mode, uin
   CK(cudaEventCreate(&t_start));
   CK(cudaEventCreate(&t_stop));
   CK(cudaEventRecord(t_start, c.st));
-  // admit the first reads
-  if (use_bits)
-    bit_admit<R>(c, *bb, c.st);
-  else
-    launch_advance<R>(c, *sb, 0, c.st);
+  // admit the first reads (a bit-row step admits by itself)
+  if (!use_bits) launch_advance<R>(c, *sb, 0, c.st);
   auto launch_block = [&]() {
     if (mode == kLaunchPersistent) {
       if constexpr (std::is_same_v<ST, uint16_t>) launch_persist<R>(c, *sb, pgrid, per_graph, c.st);
@@ -922,7 +966,8 @@ void run_queue(chsga_ctx& c, uint32_t n, uint64_t total_rows, uint32_t mode, uin
   uint64_t launched = 0;
   if (R == 1) {
     // the bit rows take a read's closure minimum one step after its last row
-    const uint64_t blocks = (total_rows + (use_bits ? 1 : 0) + per_graph - 1) / per_graph;
+    // and hand it in at the start of the step after that
+    const uint64_t blocks = (total_rows + (use_bits ? 2 : 0) + per_graph - 1) / per_graph;
     for (uint64_t i = 0; i < blocks; ++i) launch_block();
     launched = blocks;
     CK(cudaStreamSynchronize(c.st));
@@ -1034,14 +1079,18 @@ void upload_graph(chsga_ctx& c, const chsga_graph_host& g) {
     if (cl.ok) {
       d.cl_rec.upload(to4(cl.rec), s);
       d.cl_lab.upload(to4(cl.lab), s);
-      std::vector<uint2> ent(cl.ent.size());
-      if (!ent.empty()) std::memcpy(ent.data(), cl.ent.data(), ent.size() * sizeof(uint2));
+      std::vector<uint2> ent(cl.ent.size()), ent16(cl.ent.size());
+      if (!ent.empty()) {
+        std::memcpy(ent.data(), cl.ent.data(), ent.size() * sizeof(uint2));
+        std::memcpy(ent16.data(), cl.ent16.data(), ent.size() * sizeof(uint2));
+      }
       d.cl_ent.upload(ent, s);
+      d.cl_ent16.upload(ent16, s);
       d.cl_by_list.upload(cl.by_list, s);
       for (int i = 0; i < 3; ++i) d.cl_by_len[i].upload(cl.by_len[i], s);
       CK(cudaStreamSynchronize(s));  // the host vectors die with this scope
       lg->bits = true;
-      lg->bg = dev::BitGraph{L.S, (uint32_t)cl.ent.size(), cl.words, d.cl_rec.p, d.cl_ent.p, d.cl_lab.p,
+      lg->bg = dev::BitGraph{L.S, (uint32_t)cl.ent.size(), cl.words, d.cl_rec.p, d.cl_ent.p, d.cl_ent16.p, d.cl_lab.p,
                              d.cl_by_list.p, nullptr, d.sv_off.p, d.lab4.p, L.N};
     }
   }
@@ -1380,9 +1429,286 @@ void traceback_rows(chsga_ctx& c, const char* read, uint32_t len, const chsga_tb
   fill_result(res, path, best_s);
 }
 
+// Largest matrix a context keeps between tracebacks (a 150 bp read's on the
+// 5 Mbp graph is 0.8 GB; mapping and unmapping it costs as much as the
+// read's row-steps). Larger ones live for one call.
+constexpr uint64_t kKeepMatrix = 1ull << 30;
+
+// A device buffer of one traceback: the context's kept one where it fits,
+// counted by the request meter as if it were allocated for the call.
+struct TbMatrix {
+  DevArr<unsigned char> own;
+  unsigned char* p = nullptr;
+  int64_t counted = 0;
+  TbMatrix(chsga_ctx& c, uint64_t bytes) {
+    if (bytes <= kKeepMatrix) {
+      const bool fresh = !c.tb_mat.p || c.tb_mat.n < bytes;
+      c.tb_mat.alloc(bytes);
+      p = c.tb_mat.p;
+      if (!fresh) {
+        counted = (int64_t)bytes;
+        t_live_bytes += counted;
+        t_peak_bytes = std::max(t_peak_bytes, t_live_bytes);
+      }
+    } else {
+      own.alloc(bytes);
+      p = own.p;
+    }
+  }
+  ~TbMatrix() { t_live_bytes -= counted; }
+  TbMatrix(const TbMatrix&) = delete;
+  TbMatrix& operator=(const TbMatrix&) = delete;
+};
+
+// Whether a traceback of `len` bases runs on bit rows: their row must be no
+// larger than the 32-bit row the byte cap counts (labels of two or three
+// chars take a word each, so it can be up to 6 bytes a char), and where it
+// is larger than a 16-bit row the segments of a checkpointed read must still
+// fit the budget.
+bool traceback_on_bits(const chsga_ctx& c, uint32_t len, int64_t k = 500, uint64_t cap = 0) {
+  if (len > kRow16Max || !bits_apply(c)) return false;
+  const uint64_t row = bit_row_bytes(c), NC = c.g->L.N;
+  if (row > NC * 4) return false;
+  if (!cap) cap = c.cap;
+  if (row <= c.g->pitch * 2 || (uint64_t)len * NC * 4 <= cap) return true;
+  const uint64_t budget = std::max<uint64_t>(c.cap, cap), seg = std::min<uint64_t>((uint64_t)k, len - 1) + 1;
+  return seg * row <= budget || seg <= 2 || sub_segment_rows(seg - 1, budget / row) > 0;
+}
+
+// Walks rows [lo, hi] of a bit-row matrix from char `start`; the ops are
+// appended to `path`, end first.
+void walk_bits(chsga_ctx& c, const unsigned char* M, int64_t lo, int64_t hi, uint32_t start, uint32_t len,
+               std::vector<dev::WalkOp>& path, uint32_t* landing) {
+  const uint32_t max_ops = (uint32_t)(2 * (hi - lo) + 2 * (uint64_t)len + 16);
+  const size_t head = 32, bytes = head + max_ops * sizeof(dev::WalkOp);
+  c.tb_walk.alloc(bytes);
+  c.h_walk.alloc(bytes);
+  auto* out = reinterpret_cast<dev::WalkOut*>(c.tb_walk.p);
+  auto* ops = reinterpret_cast<dev::WalkOp*>(c.tb_walk.p + head);
+  dev::k_walk_bits<<<1, 32, 0, c.st>>>(c.g->gp, c.g->bg, M, bit_row_bytes(c), lo, hi, start, c.reads.p, ops, max_ops,
+                                       out, match_n(c));
+  check_launch();
+  // a path has about one op a row: copy that many with the result
+  const uint32_t guess = (uint32_t)std::min<uint64_t>(max_ops, (uint64_t)(hi - lo) + (uint64_t)(hi - lo) / 8 + 16);
+  CK(cudaMemcpyAsync(c.h_walk.p, c.tb_walk.p, head + guess * sizeof(dev::WalkOp), cudaMemcpyDeviceToHost, c.st));
+  CK(cudaStreamSynchronize(c.st));
+  const dev::WalkOut h = *reinterpret_cast<const dev::WalkOut*>(c.h_walk.p);
+  if (h.status == 7)
+    fail(CHSGA_ERR_NO_PATH, "score-matrix traceback: no valid predecessor at row " + std::to_string(h.fail_row));
+  require(h.status == 0, CHSGA_ERR_INTERNAL, "traceback walk exceeded its op budget");
+  auto* hops = reinterpret_cast<dev::WalkOp*>(c.h_walk.p + head);
+  if (h.nops > guess)
+    CK(cudaMemcpy(hops + guess, ops + guess, (h.nops - guess) * sizeof(dev::WalkOp), cudaMemcpyDeviceToHost));
+  path.insert(path.end(), hops, hops + h.nops);
+  *landing = h.vertex;
+}
+
+// traceback_rows on bit rows: a row of the matrix is the raw first scores,
+// the difference bits and the closure's first scores (5.6 MB on the 5 Mbp
+// graph, where the 16-bit row is 12.7), and a checkpoint is the state a
+// row-step starts from.
+void traceback_bits(chsga_ctx& c, const char* read, uint32_t len, const chsga_tb_opts* o, chsga_tb_result* res) {
+  require(len > 0, CHSGA_ERR_INVALID_ARG, "traceback of an empty read");
+  const size_t NC = c.g->L.N, S = c.g->L.S, W8 = (size_t)c.g->bg.words * 8;
+  const size_t row = bit_row_bytes(c), rf = dev::bits_row_rf(c.g->bg.words);
+  const int64_t k = (o && o->k > 0) ? o->k : 500;
+  const uint64_t cap = (o && o->cap_bytes) ? o->cap_bytes : c.cap;
+  const std::string dir = (o && o->dir) ? o->dir : "";
+  const bool keep = o && o->keep_files;
+  const char* rp[1] = {read};
+  upload_reads(c, rp, &len, 1);
+  BitBufs& mb = get_mat_bufs<1>(c);
+  c.tb_ptr.alloc(1);
+  c.h_ctl.alloc(1);
+  std::vector<dev::WalkOp> path;
+  uint32_t best_v = 0;
+  int32_t best_s = 0;
+  auto harvest = [&](BitBufs& b) {
+    CK(cudaMemcpyAsync(c.h_ctl.p, b.ctl.p, sizeof(dev::StepCtl), cudaMemcpyDeviceToHost, c.st));
+    CK(cudaMemcpyAsync(&best_s, c.res_score.p, 4, cudaMemcpyDeviceToHost, c.st));
+    CK(cudaMemcpyAsync(&best_v, c.res_vertex.p, 4, cudaMemcpyDeviceToHost, c.st));
+    CK(cudaStreamSynchronize(c.st));
+    require_step_ok(c.h_ctl.p->error);
+    require(c.h_ctl.p->done == 1, CHSGA_ERR_INTERNAL, "traceback lost its read");
+  };
+  // mats[0] + row * pitch is matrix row `row`; row `first` of it lies at p
+  auto set_matrix = [&](unsigned char* p, int64_t first) {
+    unsigned char* base = reinterpret_cast<unsigned char*>(reinterpret_cast<uintptr_t>(p) - (uintptr_t)first * row);
+    CK(cudaMemcpyAsync(c.tb_ptr.p, &base, sizeof(base), cudaMemcpyHostToDevice, c.st));
+    CK(cudaStreamSynchronize(c.st));  // `base` is on the stack
+  };
+  res->checkpointed = 0;
+  res->num_checkpoints = 0;
+  // the full-matrix / checkpointed decision counts int32 rows, as the
+  // reference does (src/traceback.hpp:614-645), whatever a row takes here
+  if ((uint64_t)len * NC * 4 <= cap) {
+    TbMatrix M(c, (uint64_t)len * row);
+    reset_bit_slots<1>(c, mb, 1);
+    set_matrix(M.p, 0);
+    // the read's rows, the closure of its last row, the hand-in
+    for (uint32_t i = 0; i < len + 2; ++i) mat_step<1>(c, mb, c.tb_ptr.p, i & 1, c.st);
+    harvest(mb);
+    uint32_t v = best_v;
+    if (len > 1) walk_bits(c, M.p, 0, len - 1, best_v, len, path, &v);
+    path.push_back(dev::WalkOp{0, v, CHSGA_OP_MATCHSUB});
+    fill_result(res, path, best_s);
+    return;
+  }
+  // forward with checkpoints every k rows (src/traceback.hpp:855-892): a
+  // state is {bits, raw first scores, raw last scores}
+  res->checkpointed = 1;
+  const uint64_t nck = (len - 1) / (uint64_t)k + 1;
+  res->num_checkpoints = nck;
+  const size_t ckb = W8 + 4 * S;
+  c.h_ckbits.alloc(nck * ckb);
+  BitBufs& b = get_bit_bufs<1, uint16_t>(c);
+  {
+    DevArr<unsigned char> stage[2];
+    cudaEvent_t freed[2], ready;
+    for (auto& e : freed) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+    for (auto& x : stage) x.alloc(ckb);
+    reset_bit_slots<1>(c, b, 1);
+    for (uint32_t i = 0; i < len + 2; ++i) {
+      const int par = (int)(i & 1);
+      bit_step<1, uint16_t>(c, b, par, c.st);
+      if (i >= len || i % k) continue;
+      // the next row-step overwrites the bits: a copy on the device first,
+      // then to pinned memory beside the following row-steps
+      const uint64_t j = i / k;
+      unsigned char* d = stage[j & 1].p;
+      if (j >= 2) CK(cudaStreamWaitEvent(c.st, freed[j & 1], 0));
+      CK(cudaMemcpyAsync(d, b.bits.p, W8, cudaMemcpyDeviceToDevice, c.st));
+      CK(cudaMemcpyAsync(d + W8, b.rf[par ^ 1].p, 2 * S, cudaMemcpyDeviceToDevice, c.st));
+      CK(cudaMemcpyAsync(d + W8 + 2 * S, b.rl[par ^ 1].p, 2 * S, cudaMemcpyDeviceToDevice, c.st));
+      CK(cudaEventRecord(ready, c.st));
+      CK(cudaStreamWaitEvent(c.side, ready, 0));
+      CK(cudaMemcpyAsync(c.h_ckbits.p + j * ckb, d, ckb, cudaMemcpyDeviceToHost, c.side));
+      CK(cudaEventRecord(freed[j & 1], c.side));
+    }
+    harvest(b);
+    CK(cudaStreamSynchronize(c.side));
+    for (auto& e : freed) cudaEventDestroy(e);
+    cudaEventDestroy(ready);
+  }
+  if (!dir.empty()) {
+    // checkpoint files hold raw int32 rows (the reference's format,
+    // src/traceback.hpp:215-227)
+    DevArr<int> out;
+    out.alloc(NC);
+    std::vector<int32_t> host(NC);
+    for (uint64_t j = 0; j < nck; ++j) {
+      const unsigned char* ck = c.h_ckbits.p + j * ckb;
+      CK(cudaMemcpyAsync(b.bits.p, ck, W8, cudaMemcpyHostToDevice, c.st));
+      CK(cudaMemcpyAsync(b.rf[0].p, ck + W8, 2 * S, cudaMemcpyHostToDevice, c.st));
+      CK(cudaMemcpyAsync(b.rl[0].p, ck + W8 + 2 * S, 2 * S, cudaMemcpyHostToDevice, c.st));
+      dev::k_close_row<<<nblocks(S), 256, 0, c.st>>>(c.g->bg, reinterpret_cast<const uint2*>(b.bits.p),
+                                                      reinterpret_cast<const uint16_t*>(b.rf[0].p),
+                                                      reinterpret_cast<const uint16_t*>(b.rl[0].p), out.p);
+      check_launch();
+      CK(cudaMemcpyAsync(host.data(), out.p, NC * 4, cudaMemcpyDeviceToHost, c.st));
+      CK(cudaStreamSynchronize(c.st));
+      write_ckpt(dir, (int64_t)(j * k), host.data(), NC);
+    }
+  }
+  // rows a+1 .. z into matrix rows 1 .. z - a of `mat`, from row a: its bits
+  // and first scores in matrix row 0, its last scores in mb.rl[0]. The last
+  // scores of row z end up in the returned buffer.
+  auto run_rows = [&](int64_t a, int64_t z, unsigned char* mat) -> int {
+    std::vector<dev::BitState> st(1);
+    for (auto& x : st[0].s) x = dev::SlotState{0, 0, 0, -1, 0};
+    for (auto& x : st[0].rows) x = dev::SlotRows{nullptr, nullptr};
+    st[0].s[0] = dev::SlotState{0, (uint32_t)(z + 1), (uint32_t)a, 0, 0};
+    st[0].rows[0].cur = mat;
+    st[0].q_head = 0;
+    const dev::StepCtl ctl{};
+    CK(cudaMemcpyAsync(mb.state.p, st.data(), sizeof(dev::BitState), cudaMemcpyHostToDevice, c.st));
+    CK(cudaMemcpyAsync(mb.ctl.p, &ctl, sizeof(ctl), cudaMemcpyHostToDevice, c.st));
+    CK(cudaMemsetAsync(mb.best.p, 0xFF, 4 * sizeof(unsigned long long), c.st));
+    set_matrix(mat, a);
+    // the rows and the closure of the last one
+    for (int64_t j = 0; j <= z - a; ++j) mat_step<1>(c, mb, c.tb_ptr.p, (int)(j & 1), c.st);
+    return (int)((z - a) & 1);
+  };
+  // backward, one segment at a time (src/traceback.hpp:945-1011)
+  int64_t cur_row = len - 1;
+  uint32_t cur_v = best_v;
+  // like the reference, the cap only decides between the two paths
+  // (traceback.hpp:614-645); segment recompute is sized by device memory
+  const uint64_t budget = std::max<uint64_t>(c.cap, cap);
+  while (cur_row > 0) {
+    int64_t seg_start = (cur_row % k == 0) ? (cur_row - k) : (cur_row / k * k);
+    if (seg_start < 0) seg_start = 0;
+    const int64_t seg_end = cur_row;
+    const unsigned char* ck = c.h_ckbits.p + (size_t)(seg_start / k) * ckb;
+    const uint64_t rows = (uint64_t)(seg_end - seg_start + 1);
+    uint32_t landing = cur_v;
+    // row 0 of `mat` and mb.rl[0] from a state
+    auto load_state = [&](unsigned char* mat, const unsigned char* src, cudaMemcpyKind kind) {
+      CK(cudaMemcpyAsync(mat, src, W8, kind, c.st));
+      CK(cudaMemcpyAsync(mat + rf, src + W8, 2 * S, kind, c.st));
+      CK(cudaMemcpyAsync(mb.rl[0].p, src + W8 + 2 * S, 2 * S, kind, c.st));
+    };
+    if (rows * row <= budget || rows <= 2) {
+      TbMatrix seg(c, rows * row);
+      load_state(seg.p, ck, cudaMemcpyHostToDevice);
+      run_rows(seg_start, seg_end, seg.p);
+      walk_bits(c, seg.p, seg_start, seg_end, cur_v, len, path, &landing);
+    } else {
+      // two levels: sub-segments of k2 rows, as long as the device budget
+      // allows; a first pass keeps the state at the start of each and ends
+      // with the last sub-segment on the device, which is walked at once;
+      // the earlier ones are recomputed from their states
+      const uint64_t span = (uint64_t)(seg_end - seg_start);
+      const uint64_t k2 = sub_segment_rows(span, budget / row);
+      require(k2 >= 1, CHSGA_ERR_OOM,
+              "traceback segment does not fit the byte cap even with two-level checkpoints");
+      const uint64_t nsub = (span + k2 - 1) / k2;
+      TbMatrix mem(c, (k2 + 1) * row);
+      unsigned char* seg = mem.p;
+      DevArr<unsigned char> subs;
+      subs.alloc(nsub * ckb);  // a state is no larger than a row
+      CK(cudaMemcpyAsync(subs.p, ck, ckb, cudaMemcpyHostToDevice, c.st));
+      load_state(seg, subs.p, cudaMemcpyDeviceToDevice);
+      int64_t r0 = seg_start;
+      for (uint64_t j = 1; j < nsub; ++j) {
+        const int64_t r1 = seg_start + (int64_t)(j * k2);
+        const int at = run_rows(r0, r1, seg);
+        unsigned char* d = subs.p + j * ckb;
+        const unsigned char* last = seg + (size_t)(r1 - r0) * row;
+        CK(cudaMemcpyAsync(d, last, W8, cudaMemcpyDeviceToDevice, c.st));
+        CK(cudaMemcpyAsync(d + W8, last + rf, 2 * S, cudaMemcpyDeviceToDevice, c.st));
+        CK(cudaMemcpyAsync(d + W8 + 2 * S, mb.rl[at].p, 2 * S, cudaMemcpyDeviceToDevice, c.st));
+        load_state(seg, d, cudaMemcpyDeviceToDevice);
+        r0 = r1;
+      }
+      // r0 < seg_end: the last sub-segment holds 1..k2 rows after r0
+      run_rows(r0, seg_end, seg);
+      uint32_t v = cur_v;
+      walk_bits(c, seg, r0, seg_end, cur_v, len, path, &v);
+      for (int64_t at = r0; at > seg_start;) {
+        const int64_t s0 = at - (int64_t)k2;
+        load_state(seg, subs.p + (size_t)((s0 - seg_start) / (int64_t)k2) * ckb, cudaMemcpyDeviceToDevice);
+        run_rows(s0, at, seg);
+        walk_bits(c, seg, s0, at, v, len, path, &v);
+        at = s0;
+      }
+      landing = v;
+    }
+    if (!dir.empty() && !keep && seg_start > 0) std::filesystem::remove(ckpt_row_path(dir, seg_start));
+    cur_row = seg_start;
+    cur_v = landing;
+  }
+  path.push_back(dev::WalkOp{0, cur_v, CHSGA_OP_MATCHSUB});
+  if (!dir.empty() && !keep) std::filesystem::remove(ckpt_row_path(dir, 0));
+  fill_result(res, path, best_s);
+}
+
 void traceback(chsga_ctx& c, const char* read, uint32_t len, const chsga_tb_opts* o,
                chsga_tb_result* res) {
-  if (len <= kRow16Max)
+  if (traceback_on_bits(c, len, (o && o->k > 0) ? o->k : 500, o ? o->cap_bytes : 0))
+    traceback_bits(c, read, len, o, res);
+  else if (len <= kRow16Max)
     traceback_rows<uint16_t>(c, read, len, o, res);
   else
     traceback_rows<int32_t>(c, read, len, o, res);
@@ -1420,24 +1746,41 @@ void traceback_batched(chsga_ctx& parent, const char* const* reads, const uint32
   }
   upload_reads(c, rp.data(), rl.data(), nf);  // queue entry i = read i, published below
   c.done_ring.alloc(nf);
-  SlotBufs& b = get_bufs<R, uint16_t>(c, true);
-  reset_slots<R>(c, b, 0);
-  launch_advance<R>(c, b, 0, c.st);
+  // bit rows go straight to the reads' matrices (mat_step); the level-sweep
+  // engine keeps 16-bit rows that k_store_rows copies there
+  const bool bits = traceback_on_bits(c, *std::max_element(rl.begin(), rl.end()));
+  const size_t pitch = c.g->pitch;
+  const uint64_t row_bytes = bits ? bit_row_bytes(c) : pitch * 2;
+  SlotBufs* b = nullptr;
+  BitBufs* mb = nullptr;
+  if (bits) {
+    mb = &get_mat_bufs<R>(c);
+    reset_bit_slots<R>(c, *mb, 0);
+  } else {
+    b = &get_bufs<R, uint16_t>(c, true);
+    reset_slots<R>(c, *b, 0);
+    launch_advance<R>(c, *b, 0, c.st);
+  }
+  dev::StepCtl* const ctl = bits ? mb->ctl.p : b->ctl.p;
   DevArr<uint16_t*> mats;
   mats.alloc(nf);
   CK(cudaMemsetAsync(mats.p, 0, nf * sizeof(uint16_t*), c.st));
-  const size_t pitch = c.g->pitch;
   const RowSink sink{mats.p, pitch};
   constexpr uint32_t per = 8;
-  uint16_t* rows[2] = {reinterpret_cast<uint16_t*>(b.rows[0].p), reinterpret_cast<uint16_t*>(b.rows[1].p)};
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   {
     cudaStream_t cap;
     CK(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
     CK(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-    for (uint32_t i = 0; i < per; ++i)
-      row_step<R, false, uint16_t>(c, b, rows[i & 1], rows[(i + 1) & 1], cap, nullptr, &sink);
+    for (uint32_t i = 0; i < per; ++i) {
+      if (bits) {
+        mat_step<R>(c, *mb, reinterpret_cast<unsigned char* const*>(mats.p), (int)(i & 1), cap);
+      } else {
+        uint16_t* rows[2] = {reinterpret_cast<uint16_t*>(b->rows[0].p), reinterpret_cast<uint16_t*>(b->rows[1].p)};
+        row_step<R, false, uint16_t>(c, *b, rows[i & 1], rows[(i + 1) & 1], cap, nullptr, &sink);
+      }
+    }
     CK(cudaStreamEndCapture(cap, &graph));
     CK(cudaGraphInstantiate(&exec, graph, 0));
     CK(cudaStreamDestroy(cap));
@@ -1497,7 +1840,12 @@ void traceback_batched(chsga_ctx& parent, const char* const* reads, const uint32
       for (uint32_t i = i0; i < i1; ++i) {
         const dev::CompletionRec& r = hring.p[(size_t)k * nf + i];
         const uint32_t id = (uint32_t)r.id, len = rl[id], j = i - i0;
-        if (len > 1)
+        if (len > 1 && bits)
+          dev::k_walk_bits<<<1, 32, 0, c.side>>>(c.g->gp, c.g->bg, reinterpret_cast<unsigned char*>(hm[id]),
+                                                  row_bytes, 0, (long long)len - 1, r.vertex, c.reads.p + roff[id],
+                                                  ops_buf.p + (size_t)j * max_ops, (uint32_t)max_ops, wout.p + j,
+                                                  match_n(c));
+        else if (len > 1)
           dev::k_walk<uint16_t><<<1, 1, 0, c.side>>>(c.g->gp, hm[id], pitch, 0, (long long)len - 1,
                                                       r.vertex, c.reads.p + roff[id],
                                                       ops_buf.p + (size_t)j * max_ops, (uint32_t)max_ops,
@@ -1528,7 +1876,7 @@ void traceback_batched(chsga_ctx& parent, const char* const* reads, const uint32
         fill_result(&out[idx[id]], path, r.score);
         CK(cudaFreeAsync(hm[id], c.side));
         hm[id] = nullptr;
-        used -= (uint64_t)len * pitch * 2;
+        used -= (uint64_t)len * row_bytes;
       }
     }
     hdone = st.done;
@@ -1537,20 +1885,20 @@ void traceback_batched(chsga_ctx& parent, const char* const* reads, const uint32
     while (hdone < nf) {
       const uint32_t pub0 = next;
       while (next < nf) {
-        const uint64_t mb = (uint64_t)rl[next] * pitch * 2;
+        const uint64_t need = (uint64_t)rl[next] * row_bytes;
         // always admit when nothing else holds a matrix, so the loop progresses
-        if (used + mb > budget && used > 0) break;
+        if (used + need > budget && used > 0) break;
         void* p = nullptr;
-        CK(cudaMallocAsync(&p, mb, c.st));
+        CK(cudaMallocAsync(&p, need, c.st));
         hm[next] = static_cast<uint16_t*>(p);
         dev::k_set_ptr<<<1, 1, 0, c.st>>>(mats.p, next, hm[next]);
-        used += mb;
+        used += need;
         ++next;
       }
-      if (next > pub0) k_publish<<<1, 1, 0, c.st>>>(b.ctl.p, next);
+      if (next > pub0) k_publish<<<1, 1, 0, c.st>>>(ctl, next);
       const int k = (int)(launched & 1);
       CK(cudaGraphLaunch(exec, c.st));
-      CK(cudaMemcpyAsync(hctl.p + k, b.ctl.p, sizeof(dev::StepCtl), cudaMemcpyDeviceToHost, c.st));
+      CK(cudaMemcpyAsync(hctl.p + k, ctl, sizeof(dev::StepCtl), cudaMemcpyDeviceToHost, c.st));
       CK(cudaMemcpyAsync(hring.p + (size_t)k * nf, c.done_ring.p, nf * sizeof(dev::CompletionRec),
                          cudaMemcpyDeviceToHost, c.st));
       CK(cudaEventRecord(ev[k], c.st));
@@ -2037,8 +2385,7 @@ class ScoreLaneImpl final : public ScoreLane {
     if (use_bits_) {
       bb_ = &get_bit_bufs<R, ST>(c);
       ctl_ = bb_->ctl.p;
-      reset_bit_slots<R>(c, *bb_, 0);
-      bit_admit<R>(c, *bb_, c.st);  // every slot idle
+      reset_bit_slots<R>(c, *bb_, 0);  // every slot idle
     } else {
       b_ = &get_bufs<R, ST>(c, true);
       ctl_ = b_->ctl.p;
@@ -2220,10 +2567,14 @@ chsga_ctx* fork_context(chsga_ctx& p) {
 }
 
 uint64_t traceback_device_bytes(const chsga_ctx& c, uint32_t len, const chsga_tb_opts* o) {
-  // rows as traceback_rows stores them; the path choice counts int32 rows
-  const uint64_t pb = (uint64_t)c.g->pitch * (len <= kRow16Max ? 2 : 4), row_bytes = (uint64_t)c.g->L.N * 4;
+  // 16- or 32-bit rows, the plan budgets are sized by; bit rows where they
+  // are larger than that (short labels), else they leave some of it unused.
+  // The path choice counts int32 rows
+  uint64_t pb = (uint64_t)c.g->pitch * (len <= kRow16Max ? 2 : 4);
+  const uint64_t row_bytes = (uint64_t)c.g->L.N * 4;
   const int64_t k = (o && o->k > 0) ? o->k : 500;
   const uint64_t cap = (o && o->cap_bytes) ? o->cap_bytes : c.cap;
+  if (traceback_on_bits(c, len, k, cap)) pb = std::max<uint64_t>(pb, bit_row_bytes(c));
   const uint64_t read = (len + 255) / 256 * 256;
   if ((uint64_t)len * row_bytes <= cap) return ((uint64_t)len + 1) * pb + read;
   // checkpointed: three forward rows, then the largest recompute segment
@@ -2467,7 +2818,8 @@ chsga_status chsga_align_traceback_batched(chsga_ctx* c, const char* const* read
       // `slots` at a time; a group whose matrices are large runs with fewer
       // slots (idle slots would still cost a full row-step each)
       const uint64_t mem = (uint64_t)(device_free_bytes(*c) * 0.6);
-      const uint64_t pitch_b = (uint64_t)c->g->pitch * 2;
+      // (bit rows or 16-bit rows, as traceback_batched chooses)
+      const uint64_t pitch_b = traceback_on_bits(*c, 1) ? bit_row_bytes(*c) : (uint64_t)c->g->pitch * 2;
       size_t g0 = 0;
       while (g0 < full.size()) {
         const uint64_t mb = (uint64_t)lens[full[g0]] * pitch_b;  // the group's largest matrix

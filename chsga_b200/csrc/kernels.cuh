@@ -159,7 +159,6 @@ struct StepCtl {        // device-resident control block
   uint32_t steps;       // row-steps with work
   uint32_t error;       // nonzero: a bounded device-side wait gave up
   uint32_t run_next;    // k_row_delta: runs handed out after each warp's first (k_advance resets it)
-  uint32_t arrive;      // bit-row kernels: blocks of the launch that are done (bits_advance resets it)
 };
 
 template <int R>

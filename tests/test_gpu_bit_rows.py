@@ -38,3 +38,34 @@ def test_bit_rows_match_oracle(tmp_path, name, match_n):
             got = with_n.align_scores_batched(reads, slots=slots, row_bits=row_bits)
             np.testing.assert_array_equal(got, want, err_msg=f"{slots} slots, {row_bits} bits")
     with_n.close()
+
+
+@pytest.mark.parametrize("name", sorted(GRAPHS))
+def test_bit_row_tracebacks_equal_level_sweeps(tmp_path, monkeypatch, name):
+    """Paths from bit rows (full matrix, checkpoints, two-level segments,
+    batched) are the level-sweep engine's, op for op, and score the optimum."""
+    g, files = gen_graph(tmp_path, name, **GRAPHS[name])
+    reads = g.gen_reads(5, 19, 60, 140, sub_rate=0.03, indel_rate=0.05).to_list() + [b"A", b"T" * 45]
+    n = g.view().num_chars
+    want = orc.Oracle(files).scores(reads)
+    labels = open(files[3], "rb").read().replace(b"\n", b"")
+    monkeypatch.setenv("CHSGA_ROW_KERNEL", "direct")
+    sweeps = cb.Context(0).load(g)
+    monkeypatch.delenv("CHSGA_ROW_KERNEL")
+    bits = cb.Context(0).load(g)
+    tight = cb.Context(0, hbm_cap_bytes=16 * 4 * n).load(g)
+    for rd, w in zip(reads, want):
+        ops, score, ck = sweeps.align_traceback(rd)
+        assert score == w and not ck
+        for ctx, k, cap in ((bits, 500, 0), (bits, 13, 4 * n), (tight, 100, 0)):
+            got, gs, _ = ctx.align_traceback(rd, k=k, cap_bytes=cap)
+            assert gs == w
+            if len(rd) > 1:
+                assert orc.rescore(got, rd, labels) == (w, len(rd) - 1)
+            np.testing.assert_array_equal(got, ops)
+    for slots in (4, 64):
+        for (got, gs, _), rd, w in zip(bits.align_traceback_batched(reads, slots=slots), reads, want):
+            assert gs == w
+            np.testing.assert_array_equal(got, sweeps.align_traceback(rd)[0])
+    for c in (sweeps, bits, tight):
+        c.close()
