@@ -43,7 +43,7 @@ struct BitGraph {
   const uint2* ent16;     // {source, weight for M | weight for F << 16}, 0xFFFF = none
   const uint4* lab;
   const uint8_t* by_list;
-  const uint8_t* by_len;  // of the kernel's window
+  const uint8_t* by_len;
   const uint32_t* sv_off;
   const uint32_t* lab4;
   uint32_t N;
@@ -281,8 +281,16 @@ __global__ void __launch_bounds__(NT, CHSGA_WORDS_THREADS / NT) k_row_words(BitA
     wout = static_cast<uint2*>(a.bits) + r;
   }
   const uint32_t mask = (w >> SW_MASK_SHIFT) & SW_MASK;
-  for (; i - threadIdx.x / R < g.S && (w & (SW_ACTIVE | SW_DRAIN)); i += gridDim.x * VB, fetch()) {
-    if (i >= g.S) break;
+  // turn t of block b: group (b + t) mod n of the turn's n groups (a window's
+  // groups go from long to short lists)
+  uint32_t gb = blockIdx.x;
+  for (uint32_t turn0 = 0; turn0 < g.S && (w & (SW_ACTIVE | SW_DRAIN)); turn0 += gridDim.x * VB) {
+    if (turn0) {
+      gb = gb + 1 < gridDim.x ? gb + 1 : 0;
+      i = turn0 + gb * VB + threadIdx.x / R;
+      fetch();
+    }
+    if (i >= g.S) continue;
     const uint32_t len = rec.y & 0x1FFFFFFFu, key = rec.y >> 29;
     const uint32_t nb = rec.w & 0xFFu, nm = (rec.w >> 8) & 0xFFu, nf = (rec.w >> 16) & 0xFFu;
     const uint32_t nw = (len + 30) / 32;
@@ -577,11 +585,11 @@ __global__ void __launch_bounds__(32) k_walk_bits(GraphPtrs g, BitGraph bg, cons
 // char of 32 slots is a handful of logic operations, where the packed 16-bit
 // update spends tens of instructions.
 //
-// A block takes a window of 8192 / R vertices in three passes:
-//   1  thread = (vertex, 8 slots): closure and first char in 16-bit pairs;
-//      the gap RF - F, the change T - F and rare cases leave as bytes
-//   2  thread = (vertex, 32 slots), vertices by length: the chain
-//   3  thread = (vertex, 8 slots): last scores
+// A warp takes a group of vertices in three passes:
+//   1  lane = (vertex, 8 slots): closure and first char in 16-bit pairs; the
+//      gap RF - F, the change T - F and rare cases leave as bytes
+//   2  lane = (vertex, 32 slots): the chain
+//   3  lane = (vertex, 8 slots): last scores
 // The gap of a vertex that the line lowers is a two-bit counter per slot; a
 // larger gap (none was seen on variation graphs; gaps of 1 and 2 are common)
 // and a chain to be lowered under its own first score take a scalar pass
@@ -628,7 +636,7 @@ __device__ __forceinline__ uint32_t nonzero8(const uint4& x) {
 
 // Lowers slot bit `bit` of the n chars at p (stride W word pairs) under a
 // line that starts `gap` below their left neighbour.
-__device__ __noinline__ void line_slot(uint2* p, int W, uint32_t n, uint32_t bit, uint32_t gap) {
+__device__ __forceinline__ void line_slot(uint2* p, int W, uint32_t n, uint32_t bit, uint32_t gap) {
   for (uint32_t k = 0; k < n && gap; ++k, p += W) {
     uint2 x = *p;
     if (x.x & bit) continue;
@@ -644,105 +652,141 @@ __device__ __noinline__ void line_slot(uint2* p, int W, uint32_t n, uint32_t bit
   }
 }
 
-#ifndef CHSGA_SLICED_BLOCKS
-#define CHSGA_SLICED_BLOCKS 4  // blocks per SM the register budget is sized for (build-time tuning)
+#ifndef CHSGA_SLICED_WARPS
+#define CHSGA_SLICED_WARPS 32  // warps per SM the register budget is sized for (build-time tuning)
 #endif
+#ifndef CHSGA_SLICED_U
+#define CHSGA_SLICED_U 3  // gathers in flight (build-time tuning)
+#endif
+constexpr int kSlicedThreads = 128;
+
 __device__ __forceinline__ uint4 viaddmin4(const uint4& a, uint32_t w, const uint4& c) {  // min(a + w, c), no half wraps
   return make_uint4(__viaddmin_u16x2(a.x, w, c.x), __viaddmin_u16x2(a.y, w, c.y), __viaddmin_u16x2(a.z, w, c.z),
                     __viaddmin_u16x2(a.w, w, c.w));
 }
+enum { G0, G1, VP, VN, GBIG, LOW, ENDC, NPL };
 
-enum { G0, G1, VP, VN, GBIG, LOW, NPL };
-
-// Shared memory of a k_row_sliced block: K times 256 (vertex, 8 slots) items.
+// Shared memory of a k_row_sliced block. Every warp works for itself on VB
+// vertices at a time: K (vertex, 8 slots) items a lane.
 template <int R, int K>
 struct SlicedShared {
-  static constexpr int C = R / 8, W = R / 32, NT = 256, VB = K * NT / C;
-  uint16_t F[VB * R];
-  uint16_t mis16[8][R];
+  static constexpr int C = R / 8, W = R / 32, NT = kSlicedThreads, NW = NT / 32, VB = K * 32 / C;
+  uint16_t F[NW][VB * R];
+  uint16_t mis16[5][R];
   uint16_t init[R];
-  uint8_t P[NPL][VB * C];
-  uint32_t mis[8 * W], keep[W], end[W], word[R];
-  unsigned long long best[4 * R];
+  uint16_t lim[2][R];  // scores to reach: last row, drain
+  unsigned long long best[2][R];
+  uint8_t P[NW][NPL][VB * C];
+  uint32_t mis[8 * W], keep[W], end[W], drain[W], word[R];
 };
 
-// The windows of one block. WIDE: some read is so long that a sum of a score
+// bit j of the result: value j of x (8 slots) is at most that of y
+__device__ __forceinline__ uint32_t at_most8(const uint4& x, const uint4& y) {
+  const uint4 m = min4(x, y);
+  return ~nonzero8(make_uint4(x.x ^ m.x, x.y ^ m.y, x.z ^ m.z, x.w ^ m.w)) & 0xFFu;
+}
+
+// The vertices of one warp. WIDE: some read is so long that a sum of a score
 // and a weight may leave 16 bits (saturating sums).
 template <int R, int K, bool WIDE>
-__device__ __forceinline__ void sliced_windows(const BitArgs& a, const HeadFlags& hf, SlicedShared<R, K>& sh) {
-  constexpr int C = R / 8, W = R / 32, NT = 256, VB = K * NT / C;
+__device__ __forceinline__ void sliced_warp(const BitArgs& a, const HeadFlags& hf, SlicedShared<R, K>& sh) {
+  using Shared = SlicedShared<R, K>;
+  constexpr int C = Shared::C, W = Shared::W, NW = Shared::NW, VB = Shared::VB;
   constexpr uint32_t ONES = 0x00010001u;
   const BitGraph& g = a.g;
+  const uint32_t lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  uint16_t* const sF = sh.F[wp];
+  uint8_t(*const sP)[VB * C] = sh.P[wp];
   const uint16_t* RFin = static_cast<const uint16_t*>(a.RFin);
   const uint16_t* RLin = static_cast<const uint16_t*>(a.RLin);
   uint16_t* RFout = static_cast<uint16_t*>(a.RFout);
   uint16_t* RLout = static_cast<uint16_t*>(a.RLout);
   const uint4 zero = make_uint4(0, 0, 0, 0), one = make_uint4(ONES, ONES, ONES, ONES);
-  for (uint32_t v0 = blockIdx.x * VB; v0 < g.S; v0 += gridDim.x * VB) {
+  // A block's warps share a window of NW * VB consecutive vertices (their
+  // lists and in-edges mostly stay near, so the warps meet in L1) and take
+  // its groups by label length, another one each turn.
+  constexpr uint32_t WIN = NW * VB;
+  uint32_t turn = 0;
+  for (uint32_t w0 = blockIdx.x * WIN; w0 < g.S; w0 += gridDim.x * WIN, ++turn) {
+    const uint32_t v0 = w0 + ((wp + turn) % NW) * VB;
+    if (v0 >= g.S) continue;
+    // lane v holds vertex v of the warp's group
     const uint32_t nv = min((uint32_t)VB, g.S - v0);
+    uint32_t my_s = 0;
+    if (lane < nv) my_s = K == 4 ? CHSGA_CHK(w0 + __ldg(g.by_len + v0 + lane), g.S, 24) : v0 + lane;
     // ---- pass 1
-    for (uint32_t it = threadIdx.x; it < nv * C; it += NT) {
-      const uint32_t vl = it / C, q = it % C, s = v0 + vl;
+    constexpr int U = CHSGA_SLICED_U;  // gathers in flight
+#pragma unroll 1
+    for (int j = 0; j < K; ++j) {
+      const uint32_t it = lane + 32 * j, vl = it / C, q = it % C;
+      const uint32_t s = __shfl_sync(0xFFFFFFFFu, my_s, vl);
+      if (vl >= nv) continue;
       const uint4 rec = __ldg(g.rec + s);
-      const uint32_t key = rec.y >> 29;
-      const size_t so = (size_t)s * R + 8 * q;
-      const uint4 rf = __ldg(reinterpret_cast<const uint4*>(RFin + so));
+      const uint32_t ry = rec.y;
       uint32_t k0 = rec.z, k1 = k0 + (rec.w & 0xFFu) + ((rec.w >> 8) & 0xFFu) + ((rec.w >> 16) & 0xFFu);
       CHSGA_CHK_RANGE(k0, k1, g.n_ent, 21);
+      const uint32_t key = ry >> 29;
+      const size_t so = (size_t)s * R + 8 * q;
+      const uint4 rf = __ldg(reinterpret_cast<const uint4*>(RFin + so));
       const uint4 d = *reinterpret_cast<const uint4*>(&sh.mis16[key][8 * q]);
-      uint4 F = rf, M, T;
-      constexpr int U = 4;
-      {
-        // no source: above every score, and one more does not wrap
-        const uint32_t none = WIDE ? 0xFFFFFFFFu : 0x80008000u;
-        M = make_uint4(none, none, none, none);
-        for (uint32_t k = k0; k < k1; k += U) {
-          uint2 e[U];
-          uint4 x[U];
+      const uint16_t* rl = RLin + 8 * q;
+      uint4 F = rf;
+      // no source: above every score, and one more does not wrap
+      const uint32_t none = WIDE ? 0xFFFFFFFFu : 0x80008000u;
+      uint4 M = make_uint4(none, none, none, none), T;
+      for (uint32_t k = k0; k < k1; k += U) {
+        uint2 e[U];
+        uint4 x[U];
 #pragma unroll
-          for (int u = 0; u < U; ++u)
-            if (k + u < k1) e[u] = __ldg(g.ent16 + k + u);
+        for (int u = 0; u < U; ++u)
+          if (k + u < k1) e[u] = __ldg(g.ent16 + k + u);
 #pragma unroll
-          for (int u = 0; u < U; ++u)
-            if (k + u < k1)
-              x[u] = __ldg(reinterpret_cast<const uint4*>(RLin + (size_t)CHSGA_CHK(e[u].x, g.S, 22) * R + 8 * q));
+        for (int u = 0; u < U; ++u)
+          if (k + u < k1) x[u] = __ldg(reinterpret_cast<const uint4*>(rl + (size_t)CHSGA_CHK(e[u].x, g.S, 22) * R));
 #pragma unroll
-          for (int u = 0; u < U; ++u)
-            if (k + u < k1) {
-              const uint32_t ww = WIDE ? e[u].y : __vminu2(e[u].y, 0x80008000u);
-              const uint32_t wm = __byte_perm(ww, 0, 0x1010), wf = __byte_perm(ww, 0, 0x3232);
-              if (WIDE) {
-                M = min4(M, addw4(x[u], wm));
-                F = min4(F, addw4(x[u], wf));
-              } else {
-                M = viaddmin4(x[u], wm, M);
-                F = viaddmin4(x[u], wf, F);
-              }
+        for (int u = 0; u < U; ++u)
+          if (k + u < k1) {
+            const uint32_t ww = WIDE ? e[u].y : __vminu2(e[u].y, 0x80008000u);
+            const uint32_t wm = __byte_perm(ww, 0, 0x1010), wf = __byte_perm(ww, 0, 0x3232);
+            if (WIDE) {
+              M = min4(M, addw4(x[u], wm));
+              F = min4(F, addw4(x[u], wf));
+            } else {
+              M = viaddmin4(x[u], wm, M);
+              F = viaddmin4(x[u], wf, F);
             }
-        }
-        const uint4 F1 = make_uint4(F.x + ONES, F.y + ONES, F.z + ONES, F.w + ONES);
-        if (WIDE)
-          T = min4(F1, add4(M, d));
-        else
-          T = make_uint4(__viaddmin_u16x2(M.x, d.x, F1.x), __viaddmin_u16x2(M.y, d.y, F1.y),
-                         __viaddmin_u16x2(M.z, d.z, F1.z), __viaddmin_u16x2(M.w, d.w, F1.w));
+          }
       }
+      const uint4 F1 = make_uint4(F.x + ONES, F.y + ONES, F.z + ONES, F.w + ONES);
+      if (WIDE)
+        T = min4(F1, add4(M, d));
+      else
+        T = make_uint4(__viaddmin_u16x2(M.x, d.x, F1.x), __viaddmin_u16x2(M.y, d.y, F1.y),
+                       __viaddmin_u16x2(M.z, d.z, F1.z), __viaddmin_u16x2(M.w, d.w, F1.w));
       uint4 in = zero;
       if (hf.init) {
         in = *reinterpret_cast<const uint4*>(sh.init + 8 * q);
         T = sel4(d, T, in);
       }
       *reinterpret_cast<uint4*>(RFout + so) = T;
-      *reinterpret_cast<uint4*>(sh.F + vl * R + 8 * q) = F;
+      *reinterpret_cast<uint4*>(sF + vl * R + 8 * q) = F;
       if (hf.drain) {
-        const uint32_t f = __ldg(g.sv_off + s), fw[4] = {F.x, F.y, F.z, F.w};
-#pragma unroll
-        for (int v = 0; v < 8; ++v) {
-          const uint32_t w = sh.word[8 * q + v];
-          if (w & SW_DRAIN)
-            atomicMin(&sh.best[((w >> SW_PAR_SHIFT) + 3u & 3u) * R + 8 * q + v],
-                      pack_min((int)((fw[v >> 1] >> (16 * (v & 1))) & 0xFFFFu), f));
+        uint32_t m = at_most8(F, *reinterpret_cast<const uint4*>(&sh.lim[1][8 * q]));
+        m &= sh.drain[q >> 2] >> (8 * (q & 3));
+        if (m) {
+          const uint32_t f = __ldg(g.sv_off + s);
+          for (; m; m &= m - 1) {
+            const int v = __ffs(m) - 1;
+            atomicMin(&sh.best[1][8 * q + v], pack_min(sF[vl * R + 8 * q + v], f));
+          }
         }
+      }
+      if (hf.end) {
+        // a chain falls by at most one a char: most vertices stay above the best so far
+        const uint32_t n = ((ry & 0x1FFFFFFFu) - 1) * ONES;
+        const uint4 lo = make_uint4(__vsubus2(T.x, n), __vsubus2(T.y, n), __vsubus2(T.z, n), __vsubus2(T.w, n));
+        sP[ENDC][it] = (uint8_t)(at_most8(lo, *reinterpret_cast<const uint4*>(&sh.lim[0][8 * q])) &
+                                 (sh.end[q >> 2] >> (8 * (q & 3))));
       }
       // chain start: not below F - 1 (max(T + 1, F) - 1; no half wraps)
       const uint4 T1 = max4(make_uint4(T.x + ONES, T.y + ONES, T.z + ONES, T.w + ONES), F);  // + 1
@@ -761,152 +805,186 @@ __device__ __forceinline__ void sliced_windows(const BitArgs& a, const HeadFlags
       }
       planes2(gap, g0, g1);
       planes2(ch, c0, c1);
-      const uint32_t at = vl * C + q;
-      sh.P[G0][at] = (uint8_t)g0;
-      sh.P[G1][at] = (uint8_t)g1;
-      sh.P[VP][at] = (uint8_t)c1;
-      sh.P[VN][at] = (uint8_t)(~(c0 | c1));
-      sh.P[GBIG][at] = (uint8_t)big;
-      sh.P[LOW][at] = (low.x | low.y | low.z | low.w) ? (uint8_t)nonzero8(low) : (uint8_t)0;
+      sP[G0][it] = (uint8_t)g0;
+      sP[G1][it] = (uint8_t)g1;
+      sP[VP][it] = (uint8_t)c1;
+      sP[VN][it] = (uint8_t)(~(c0 | c1));
+      sP[GBIG][it] = (uint8_t)big;
+      sP[LOW][it] = (low.x | low.y | low.z | low.w) ? (uint8_t)nonzero8(low) : (uint8_t)0;
     }
-    __syncthreads();
+    __syncwarp();
     // ---- pass 2
-    for (uint32_t t = threadIdx.x; t < nv * W; t += NT) {
-      const uint32_t vi = t / W, w = t % W;
-      const uint32_t vl = K == 4 ? CHSGA_CHK((uint32_t)__ldg(g.by_len + v0 + vi), nv, 24) : vi;
-      const uint32_t s = v0 + vl;
-      uint32_t f = __ldg(g.sv_off + s), e = __ldg(g.sv_off + s + 1);
-      CHSGA_CHK_CHARS(f, e, g.N, 1);
-      const uint32_t n = e - f - 1;  // chain chars
-      uint2* z = static_cast<uint2*>(a.bits) + (size_t)(f + 1) * W + w;
-      auto plane = [&](int p) { return reinterpret_cast<const uint32_t*>(sh.P[p])[vl * W + w]; };
-      if (n) {
-        uint32_t vp = plane(VP), vn = plane(VN);
-        const uint32_t keep = sh.keep[w];
-        uint32_t g0 = plane(G0), g1 = plane(G1);
-        for (uint32_t big = plane(GBIG); big; big &= big - 1) {
-          const uint32_t b = __ffs(big) - 1, r = 32 * w + b;
-          line_slot(z, W, n, 1u << b, (uint32_t)RFin[(size_t)s * R + r] - sh.F[vl * R + r]);
-        }
-        // label keys, 8 chars a word
-        const uint32_t* kp = g.lab4 + ((f + 1) >> 3);
-        const uint32_t ks = ((f + 1) & 7u) * 4u;
-        uint32_t klo = __ldg(kp);
-        constexpr int U = 8;
-        for (uint32_t c = 0; c < n; c += U) {
-          const uint32_t khi = __ldg(++kp);
-          const uint32_t keys = __funnelshift_r(klo, khi, ks);
-          klo = khi;
-          uint2 x[U];
-#pragma unroll
-          for (int u = 0; u < U; ++u)
-            if (c + u < n) x[u] = z[u * W];
-#pragma unroll
-          for (int u = 0; u < U; ++u)
-            if (c + u < n) {
-              const uint32_t d = sh.mis[((keys >> (4 * u)) & 7u) * W + w];
-              const uint32_t p = x[u].x, m = x[u].y;
-              // the previous row under its line (row 0 slots have none)
-              const uint32_t t0 = g0 & ~m;
-              const uint32_t hp = (p & keep) | g1 | t0;
-              const uint32_t hn = m & keep & ~(g1 | g0);
-              const uint32_t b = g1 & ~(g0 ^ m);
-              g1 &= p | t0;
-              g0 = (p & g0) | (~p & b);
-              // the new score is 1 above the previous row's left neighbour, else level with it
-              const uint32_t t1 = d & ~(vn | hn);
-              const uint32_t op = vn | (t1 & ~vp), om = vp & ~t1;
-              vp = hn | (t1 & ~hp);
-              vn = hp & ~t1;
-              z[u * W] = make_uint2(op, om);
-            }
-          z += U * W;
-        }
-        z = static_cast<uint2*>(a.bits) + (size_t)(f + 1) * W + w;
-        for (uint32_t lb = plane(LOW); lb; lb &= lb - 1) {
-          const uint32_t b = __ffs(lb) - 1, r = 32 * w + b;
-          line_slot(z, W, n, 1u << b, (uint32_t)sh.F[vl * R + r] - 1u - RFout[(size_t)s * R + r]);
-        }
-        reinterpret_cast<uint32_t*>(sh.P[VP])[vl * W + w] = vp;
-        reinterpret_cast<uint32_t*>(sh.P[VN])[vl * W + w] = vn;
-      }
-      if (hf.end) {
-        for (uint32_t eb = sh.end[w]; eb; eb &= eb - 1) {
-          const uint32_t b = __ffs(eb) - 1, r = 32 * w + b;
-          int cur = RFout[(size_t)s * R + r], bm = cur;
-          uint32_t bc = f;
-          for (uint32_t c = 0; c < n; ++c) {
-            const uint2 x = z[(size_t)c * W];
-            cur += (int)((x.x >> b) & 1u) - (int)((x.y >> b) & 1u);
-            if (cur < bm) {
-              bm = cur;
-              bc = f + 1 + c;
-            }
+    {
+      const uint32_t vl = lane / W, w = lane % W;
+      const uint32_t s = __shfl_sync(0xFFFFFFFFu, my_s, vl % VB);
+      if (vl < nv) {
+        uint32_t f = __ldg(g.sv_off + s), e = __ldg(g.sv_off + s + 1);
+        CHSGA_CHK_CHARS(f, e, g.N, 1);
+        const uint32_t n = e - f - 1;  // chain chars
+        uint2* const z0 = static_cast<uint2*>(a.bits) + (size_t)(f + 1) * W + w;
+        auto plane = [&](int p) { return reinterpret_cast<const uint32_t*>(sP[p])[vl * W + w]; };
+        if (n) {
+          uint32_t vp = plane(VP), vn = plane(VN);
+          const uint32_t keep = sh.keep[w];
+          uint32_t g0 = plane(G0), g1 = plane(G1);
+          for (uint32_t big = plane(GBIG); big; big &= big - 1) {
+            const uint32_t b = __ffs(big) - 1, r = 32 * w + b;
+            line_slot(z0, W, n, 1u << b, (uint32_t)RFin[(size_t)s * R + r] - sF[vl * R + r]);
           }
-          atomicMin(&sh.best[((sh.word[r] >> SW_PAR_SHIFT) & 3u) * R + r], pack_min(bm, bc));
+          const uint32_t* kp = g.lab4 + ((f + 1) >> 3);  // label keys, 8 chars a word
+          const uint32_t ks = ((f + 1) & 7u) * 4u;
+          uint32_t klo = __ldg(kp);
+          // chars whose words load together: a lone group of vertices waits for
+          // each load, many groups lose more to the chars past the last
+          constexpr int U2 = K == 1 ? 8 : 4;
+          uint32_t keys = 0, c = 0;
+          uint2* z = z0;
+          auto one = [&](uint2* at, const uint2& x, uint32_t key) {
+            const uint32_t d = sh.mis[key * W + w];
+            const uint32_t p = x.x, m = x.y;
+            // the previous row under its line (row 0 slots have none)
+            const uint32_t t0 = g0 & ~m;
+            const uint32_t hp = (p & keep) | g1 | t0;
+            const uint32_t hn = m & keep & ~(g1 | g0);
+            const uint32_t b = g1 & ~(g0 ^ m);
+            g1 &= p | t0;
+            g0 = (p & g0) | (~p & b);
+            // the new score is 1 above the previous row's left neighbour, else level with it
+            const uint32_t t1 = d & ~(vn | hn);
+            const uint32_t op = vn | (t1 & ~vp), om = vp & ~t1;
+            vp = hn | (t1 & ~hp);
+            vn = hp & ~t1;
+            *at = make_uint2(op, om);
+          };
+          auto next_keys = [&] {  // of the chars c .. c + 7, when c is a multiple of 8
+            const uint32_t khi = __ldg(++kp);
+            keys = __funnelshift_r(klo, khi, ks);
+            klo = khi;
+          };
+          for (; c < n; c += U2, z += U2 * W) {
+            uint2 x[U2];
+#pragma unroll
+            for (int u = 0; u < U2; ++u)
+              if (c + u < n) x[u] = z[u * W];
+            if (U2 == 4 && (c & 4u))
+              keys >>= 16;
+            else
+              next_keys();
+#pragma unroll
+            for (int u = 0; u < U2; ++u)
+              if (c + u < n) one(z + u * W, x[u], (keys >> (4 * u)) & 7u);
+          }
+          for (uint32_t lb = plane(LOW); lb; lb &= lb - 1) {
+            const uint32_t b = __ffs(lb) - 1, r = 32 * w + b;
+            line_slot(z0, W, n, 1u << b, (uint32_t)sF[vl * R + r] - 1u - RFout[(size_t)s * R + r]);
+          }
+          reinterpret_cast<uint32_t*>(sP[VP])[vl * W + w] = vp;
+          reinterpret_cast<uint32_t*>(sP[VN])[vl * W + w] = vn;
+        }
+        if (hf.end) {
+          for (uint32_t eb = plane(ENDC); eb; eb &= eb - 1) {
+            const uint32_t b = __ffs(eb) - 1, r = 32 * w + b;
+            int cur = RFout[(size_t)s * R + r], bm = cur;
+            uint32_t bc = f;
+            for (uint32_t c = 0; c < n; ++c) {
+              const uint2 x = z0[(size_t)c * W];
+              cur += (int)((x.x >> b) & 1u) - (int)((x.y >> b) & 1u);
+              if (cur < bm) {
+                bm = cur;
+                bc = f + 1 + c;
+              }
+            }
+            atomicMin(&sh.best[0][r], pack_min(bm, bc));
+          }
         }
       }
     }
-    __syncthreads();
+    __syncwarp();
     // ---- pass 3 (first + len - 1 stays below 2^16: the kernel runs up to 512 chars)
-    for (uint32_t it = threadIdx.x; it < nv * C; it += NT) {
-      const uint32_t vl = it / C, q = it % C, s = v0 + vl;
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const uint32_t it = lane + 32 * j, vl = it / C, q = it % C;
+      const uint32_t s = __shfl_sync(0xFFFFFFFFu, my_s, vl);
+      if (vl >= nv) continue;
       const uint32_t len = __ldg(&g.rec[s].y) & 0x1FFFFFFFu;
       const size_t so = (size_t)s * R + 8 * q;
       uint4 o;
       if (len == 1) {
         o = *reinterpret_cast<const uint4*>(RFout + so);
       } else {
-        const uint32_t lw = (len - 1) * ONES, at = vl * C + q;
-        o = viaddmin4(*reinterpret_cast<const uint4*>(sh.F + vl * R + 8 * q), lw,
+        const uint32_t lw = (len - 1) * ONES;
+        o = viaddmin4(*reinterpret_cast<const uint4*>(sF + vl * R + 8 * q), lw,
                       __ldg(reinterpret_cast<const uint4*>(RLin + so)));
         if (hf.init) o = sel4(zero, o, *reinterpret_cast<const uint4*>(sh.init + 8 * q));
-        const uint4 p = unplane(sh.P[VP][at]), m = unplane(sh.P[VN][at]);
+        const uint4 p = unplane(sP[VP][it]), m = unplane(sP[VN][it]);
         o = make_uint4(o.x + p.x - m.x, o.y + p.y - m.y, o.z + p.z - m.z, o.w + p.w - m.w);
-        if (sh.P[LOW][at]) o = viaddmin4(*reinterpret_cast<const uint4*>(RFout + so), lw, o);
+        if (sP[LOW][it]) o = viaddmin4(*reinterpret_cast<const uint4*>(RFout + so), lw, o);
       }
       *reinterpret_cast<uint4*>(RLout + so) = o;
     }
-    __syncthreads();  // the next window reuses the shared arrays
+    if (hf.end) {
+      // hand the best so far to the other blocks and take theirs
+      for (int r = (int)lane; r < R; r += 32) {
+        const unsigned long long b = *(volatile unsigned long long*)&sh.best[0][r];
+        if (b == ~0ull) continue;
+        unsigned long long* gb = a.best + ((sh.word[r] >> SW_PAR_SHIFT) & 3u) * R + r;
+        const unsigned long long o = __ldcg(gb);
+        if (b < o) atomicMin(gb, b);
+        sh.lim[0][r] = (uint16_t)min((unsigned long long)0xFFFFu, min(b, o) >> 32);
+      }
+    }
+    __syncwarp();  // the next vertices reuse the warp's arrays
   }
 }
 
 template <int R, int K>
-__global__ void __launch_bounds__(256, CHSGA_SLICED_BLOCKS) k_row_sliced(BitArgs a) {
+__global__ void __launch_bounds__(kSlicedThreads, CHSGA_SLICED_WARPS * 32 / kSlicedThreads) k_row_sliced(BitArgs a) {
   using Shared = SlicedShared<R, K>;
   constexpr int NT = Shared::NT, W = Shared::W;
+  static_assert(R <= NT, "a thread per slot");
   __shared__ __align__(16) Shared sh;
   pdl_wait();
   const HeadFlags hf = bits_head<R>(a, sh.word, nullptr);
   if (!hf.work) return;
   // the step's words: per label key the mismatches of 32 slots, and as 16-bit increments
-  for (int i = threadIdx.x; i < R; i += NT) {
+  if (threadIdx.x < R) {
+    const int i = threadIdx.x;
     const uint32_t w = sh.word[i], m = (w >> SW_MASK_SHIFT) & SW_MASK;
     const bool init = (w & SW_INIT) || !(w & SW_ACTIVE);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      sh.mis16[k][i] = (uint16_t)((m >> k) & 1u);
+      if (k < 5) sh.mis16[k][i] = (uint16_t)((m >> k) & 1u);
       const uint32_t b = __ballot_sync(0xFFFFFFFFu, (m >> k) & 1u);
       if ((i & 31) == 0) sh.mis[k * W + (i >> 5)] = b;
     }
     sh.init[i] = init ? 0xFFFFu : 0u;
-    const uint32_t bk = __ballot_sync(0xFFFFFFFFu, !init), be = __ballot_sync(0xFFFFFFFFu, (w & SW_ENDING) != 0);
+    const uint32_t bk = __ballot_sync(0xFFFFFFFFu, !init), be = __ballot_sync(0xFFFFFFFFu, (w & SW_ENDING) != 0),
+                   bd = __ballot_sync(0xFFFFFFFFu, (w & SW_DRAIN) != 0);
     if ((i & 31) == 0) {
       sh.keep[i >> 5] = bk;
       sh.end[i >> 5] = be;
+      sh.drain[i >> 5] = bd;
     }
+    sh.best[0][i] = sh.best[1][i] = ~0ull;
+    sh.lim[0][i] = 0xFFFFu;
+    // a draining read's raw minimum is known: only scores that reach it count
+    if (hf.drain)
+      sh.lim[1][i] = (uint16_t)min((unsigned long long)0xFFFFu,
+                                   __ldcg(a.best + (((w >> SW_PAR_SHIFT) + 3u) & 3u) * R + i) >> 32);
   }
-  const bool ends = hf.end || hf.drain;
-  if (ends)
-    for (int i = threadIdx.x; i < 4 * R; i += NT) sh.best[i] = ~0ull;
   __syncthreads();
   if (hf.wide)
-    sliced_windows<R, K, true>(a, hf, sh);
+    sliced_warp<R, K, true>(a, hf, sh);
   else
-    sliced_windows<R, K, false>(a, hf, sh);
-  if (ends) {
-    for (int i = threadIdx.x; i < 4 * R; i += NT)
-      if (sh.best[i] != ~0ull) atomicMin(a.best + i, sh.best[i]);
+    sliced_warp<R, K, false>(a, hf, sh);
+  if (hf.end || hf.drain) {
+    __syncthreads();
+    if (threadIdx.x < R) {
+      const int i = threadIdx.x;
+      const uint32_t par = (sh.word[i] >> SW_PAR_SHIFT) & 3u;
+      if (sh.best[0][i] != ~0ull) atomicMin(a.best + par * R + i, sh.best[0][i]);
+      if (sh.best[1][i] != ~0ull) atomicMin(a.best + ((par + 3u) & 3u) * R + i, sh.best[1][i]);
+    }
   }
 }
 

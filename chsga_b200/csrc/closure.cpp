@@ -231,7 +231,7 @@ HostClosure build_closure(const HostLayout& L) {
   };
   windows(c.by_list, 256, [&](int64_t s) { return e_cnt[s + 1] - e_cnt[s]; });
   for (int i = 0; i < 3; ++i)
-    windows(c.by_len[i], 64u << i, [&](int64_t s) { return L.sv_off[s + 1] - L.sv_off[s]; });
+    windows(c.by_len[i], 32u << i, [&](int64_t s) { return L.sv_off[s + 1] - L.sv_off[s]; });
   c.ok = true;
   return c;
 }

@@ -56,7 +56,7 @@ struct HostClosure {
   // 0xFFFF = no such entry (or a weight no 16-bit score can win with)
   std::vector<uint32_t> ent16;
   // order of the vertices inside every window of 256 by list length, and
-  // inside every window of 64, 128 and 256 by label length (local indexes)
+  // inside every window of 32, 64 and 128 by label length (local indexes)
   std::vector<uint8_t> by_list;
   std::vector<uint8_t> by_len[3];
 };

@@ -163,7 +163,7 @@ struct LoadedGraph {
   std::unique_ptr<TopDev> top;
   dev::T1Ptrs t1{};  // ntiles = 0: some vertex is too long for k_row_t1
   bool bits = false;       // the closure lists exist: rows can run on the bit-row kernels
-  dev::BitGraph bg{};      // by_len is set per kernel
+  dev::BitGraph bg{};
   size_t pitch = 0;  // traceback matrix row stride (elements), 16-byte aligned rows
   bool nul_label = false;
   bool n_label = false;  // some label byte is 'N'
@@ -805,17 +805,19 @@ void bit_step(chsga_ctx& c, BitBufs& b, int par, cudaStream_t s) {
   const uint32_t S = c.g->L.S;
   if constexpr (R >= 32 && std::is_same_v<ST, uint16_t>) {
     if (bits_sliced<R, ST>(c)) {
-      a.g.by_len = c.g->gd.cl_by_len[R == 128 ? 0 : R == 64 ? 1 : 2].p;
-      // windows of 8192 / R vertices where they fill the device, else a
-      // quarter of that: a small graph's row-step is as long as one block's
       auto launch = [&](auto kern, uint32_t VB) {
-        const uint32_t wins = (S + VB - 1) / VB;
-        chain_launch(c, kern, std::min(wins, resident_blocks(c, (const void*)kern, 256)), 256, 0, s, a);
+        const uint32_t blocks = (S + VB - 1) / VB;
+        chain_launch(c, kern, std::min(blocks, resident_blocks(c, (const void*)kern, dev::kSlicedThreads)),
+                     dev::kSlicedThreads, 0, s, a);
       };
-      if (S >= 8192 / R * 2u * (uint32_t)c.num_sms)
-        launch(dev::k_row_sliced<R, 4>, 8192 / R);
+      using S4 = dev::SlicedShared<R, 4>;
+      using S1 = dev::SlicedShared<R, 1>;
+      // four items a lane where that gives every warp of the device work
+      a.g.by_len = c.g->gd.cl_by_len[R == 128 ? 0 : R == 64 ? 1 : 2].p;
+      if (S >= (uint32_t)S4::VB * 16u * (uint32_t)c.num_sms)
+        launch(dev::k_row_sliced<R, 4>, S4::VB * S4::NW);
       else
-        launch(dev::k_row_sliced<R, 1>, 2048 / R);
+        launch(dev::k_row_sliced<R, 1>, S1::VB * S1::NW);
       return;
     }
   }
