@@ -35,18 +35,19 @@ constexpr uint32_t SW_DRAIN = 1u << 13;     // the slot's previous read takes it
 constexpr uint32_t SW_PAR_SHIFT = 14;       // bits 14..15: which of the slot's four minima its read uses
 constexpr uint32_t kBitsNarrowMax = 32767;  // longest read whose sums need no saturation
 
-struct BitGraph {
-  uint32_t S, n_ent;
+struct BitGraph {  // closure.hpp
+  uint32_t S, N, n_ent, n_went, heavy;
   uint64_t words;
-  const uint4* rec;       // closure.hpp
-  const uint2* ent;       // {source, weight}
-  const uint2* ent16;     // {source, weight for M | weight for F << 16}, 0xFFFF = none
-  const uint4* lab;
-  const uint8_t* by_list;
-  const uint8_t* by_len;
+  const uint4* rec;
+  const uint2* ent16;
+  const uint8_t* by_len;  // of the kernel's window
   const uint32_t* sv_off;
   const uint32_t* lab4;
-  uint32_t N;
+  const uint32_t* pos;
+  const uint2* wsv;
+  const uint4* wrec;
+  const uint2* went;
+  const uint4* lab;
 };
 
 // Where a slot's previous and current rows lie in its read's matrix
@@ -61,6 +62,7 @@ struct SlotRows {
 struct BitState {
   SlotState s[128];
   SlotRows rows[128];  // traceback
+  uint32_t next[128];  // the slot's read base after the row's, when there is one
   uint32_t q_head, pad[3];
 };
 
@@ -111,11 +113,12 @@ __device__ __forceinline__ HeadFlags bits_head(const BitArgs& a, uint32_t* word,
   SlotState st{};
   SlotRows sr{nullptr, nullptr};
   bool need = false, wide = false;
-  uint32_t drain = 0, par = 0, q_head = 0, avail = 0;
+  uint32_t drain = 0, par = 0, q_head = 0, avail = 0, byte = 0;
   unsigned before = 0;
   if (wp < NW) {
     if (r < R) {
       st = a.st_in->s[r];
+      byte = a.st_in->next[r];
       q_head = a.st_in->q_head;
       avail = a.ctl->q_count - q_head;
       par = st.pad & 3u;
@@ -171,11 +174,12 @@ __device__ __forceinline__ HeadFlags bits_head(const BitArgs& a, uint32_t* word,
         st.len = q.len;
         st.row = 0;
         st.id = q.id;
+        byte = a.reads[q.off];
         if (first) a.res_t0[q.id] = global_ns();
       }
       if (st.id >= 0) {
-        const int byte = a.reads[st.off + st.row];
-        w = base_code(byte, a.special) | (mismatch_mask(byte, a.special, a.match_n) << SW_MASK_SHIFT) | SW_ACTIVE;
+        w = base_code((int)byte, a.special) | (mismatch_mask((int)byte, a.special, a.match_n) << SW_MASK_SHIFT) |
+            SW_ACTIVE;
         w |= st.row == 0 ? SW_INIT : SW_CLOSURE;
         if (st.row + 1 == st.len) w |= SW_ENDING;
         if (a.mats) sr.cur = a.mats[st.id] + (size_t)st.row * a.pitch;
@@ -187,6 +191,9 @@ __device__ __forceinline__ HeadFlags bits_head(const BitArgs& a, uint32_t* word,
       if (first) {
         st.pad = drain << 2 | par;
         a.st_out->s[r] = st;
+        // fetched here, where nothing waits for it, the base is part of the
+        // state the next launch starts from
+        if (st.id >= 0 && st.row + 1 < st.len) a.st_out->next[r] = a.reads[st.off + st.row + 1];
         if (a.mats) a.st_out->rows[r] = sr;
         if (r == 0) a.st_out->q_head = q_head + (total < avail ? total : avail);
       }
@@ -222,18 +229,21 @@ __host__ __device__ constexpr size_t bits_row_bytes(uint64_t words, uint32_t S) 
 // words of 32 chars. Slots are interleaved (RF[s * R + r], word w of slot r at
 // w * R + r), so the gathers of neighbouring slots share sectors; with MAT
 // every slot is blockIdx.y of a one-slot launch with rows in its read's
-// matrix. Vertices of a 256-vertex window are taken by list length, so a
-// warp's lists end together.
+// matrix. Vertices are in the order of closure.hpp (windows by list length),
+// so a warp's lists end together and its loads of records, entries, labels
+// and bits lie side by side.
 // ---------------------------------------------------------------------------
 #ifndef CHSGA_WORDS_THREADS
-#define CHSGA_WORDS_THREADS 1280  // threads per SM the register budget is sized for (build-time tuning)
+#define CHSGA_WORDS_THREADS 1024  // threads per SM the register budget is sized for (build-time tuning)
 #endif
-template <int R, typename ST, int H, int NT>
+// P = lanes that share a long list (for every slot).
+template <int R, typename ST, int H, int NT, int P>
 __global__ void __launch_bounds__(NT, CHSGA_WORDS_THREADS / NT) k_row_words(BitArgs a) {
   constexpr bool MAT = H > 0;
   constexpr int SLOTS = MAT ? H : R;
   static_assert(!MAT || (R == 1 && sizeof(ST) == 2), "matrix rows hold one slot each, 16 bits");
   static_assert(NT >= (SLOTS < 32 ? 32 : SLOTS), "the head needs a thread per slot");
+  static_assert(P == 1 || R * P <= 32, "a list's lanes lie in one warp");
   using bits::PN;
   constexpr int VB = NT / R;  // vertices per block and turn
   const BitGraph& g = a.g;
@@ -241,20 +251,48 @@ __global__ void __launch_bounds__(NT, CHSGA_WORDS_THREADS / NT) k_row_words(BitA
   __shared__ SlotRows s_rows[MAT ? SLOTS : 1];
   __shared__ unsigned long long s_min[4 * R];
   const int r = (int)(threadIdx.x % R);  // of this block's slots
-  uint32_t i = blockIdx.x * VB + threadIdx.x / R;  // position in the windows' order
-  uint32_t s = 0;
+  constexpr int U = R == 1 ? 8 : 4;  // entries and gathers in flight: a short list in one go
+  // items: P parts of every long list, rounded up to whole blocks, then the
+  // vertices with short lists
+  const uint32_t hparts = (g.heavy * P + VB - 1) / VB * VB, items = hparts + (g.S - g.heavy);
+  uint32_t i = 0, part = 0, n = 0, stride = 32;  // position of the vertex; this lane's entries
+  uint2 sv = make_uint2(0, 0);                   // the vertex, its first char
+  bool mine = false;
   uint4 rec = make_uint4(0, 1, 0, 0);
-  auto fetch = [&] {
-    if (i < g.S) {
-      s = CHSGA_CHK((i & ~255u) + __ldg(g.by_list + i), g.S, 20);
-      rec = __ldg(g.rec + s);
+  uint2 e[U];
+  auto entries = [&](uint32_t k) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k + u < n) e[u] = __ldg(g.went + CHSGA_CHK(rec.z + part + stride * (k + u), g.n_went, 21));
+  };
+  auto fetch = [&](uint32_t item) {
+    const bool long_list = item < hparts;
+    i = long_list ? item / P : item - hparts + g.heavy;
+    part = long_list ? item % P : 0;
+    mine = item < items && (!long_list || i < g.heavy);
+    n = 0;
+    if (mine) {
+      rec = __ldg(g.wrec + i);
+      sv = __ldg(g.wsv + i);
+      sv.x = CHSGA_CHK(sv.x, g.S, 20);
+      stride = long_list ? P : 32;
+      n = long_list ? (rec.w > part ? (rec.w - part + P - 1) / P : 0) : rec.w;
+      entries(0);
     }
   };
-  fetch();
+  fetch(blockIdx.x * VB + threadIdx.x / R);
   pdl_wait();
   for (int k = threadIdx.x; k < 4 * R; k += NT) s_min[k] = ~0ull;
   const HeadFlags hf = bits_head<SLOTS>(a, s_word, MAT ? s_rows : nullptr);
   if (!hf.work) return;
+  if (hf.drain) {
+    // a draining read's raw minimum is known: only scores that reach it count
+    if (threadIdx.x < R) {
+      const uint32_t q = MAT ? blockIdx.y : threadIdx.x, p = ((s_word[q] >> SW_PAR_SHIFT) + 3u) & 3u;
+      if (s_word[q] & SW_DRAIN) s_min[p * R + threadIdx.x] = __ldcg(a.best + p * SLOTS + q);
+    }
+    __syncthreads();
+  }
   const uint32_t w = s_word[MAT ? blockIdx.y : r];
   const bool init = (w & SW_INIT) != 0;
   const uint32_t par = (w >> SW_PAR_SHIFT) & 3u;
@@ -284,55 +322,76 @@ __global__ void __launch_bounds__(NT, CHSGA_WORDS_THREADS / NT) k_row_words(BitA
   // turn t of block b: group (b + t) mod n of the turn's n groups (a window's
   // groups go from long to short lists)
   uint32_t gb = blockIdx.x;
-  for (uint32_t turn0 = 0; turn0 < g.S && (w & (SW_ACTIVE | SW_DRAIN)); turn0 += gridDim.x * VB) {
+  for (uint32_t turn0 = 0; turn0 < items && (w & (SW_ACTIVE | SW_DRAIN)); turn0 += gridDim.x * VB) {
     if (turn0) {
       gb = gb + 1 < gridDim.x ? gb + 1 : 0;
-      i = turn0 + gb * VB + threadIdx.x / R;
-      fetch();
+      fetch(turn0 + gb * VB + threadIdx.x / R);
     }
-    if (i >= g.S) continue;
+    const bool long_list = turn0 + gb * VB < hparts;  // the same for the whole block
+    if (!long_list && !mine) continue;
     const uint32_t len = rec.y & 0x1FFFFFFFu, key = rec.y >> 29;
-    const uint32_t nb = rec.w & 0xFFu, nm = (rec.w >> 8) & 0xFFu, nf = (rec.w >> 16) & 0xFFu;
     const uint32_t nw = (len + 30) / 32;
     const int delta = (int)((mask >> key) & 1u);
+    // the first word's labels and bits load beside the gathers
+    uint4 lb = make_uint4(0, 0, 0, 0);
+    uint2 old = make_uint2(0, 0);
+    if (mine && part == 0 && nw) {
+      const size_t wi = (size_t)CHSGA_CHK(rec.x, g.words, 23);
+      lb = __ldg(g.lab + wi);
+      if (!init) old = win[wi * R];
+    }
     // closure of the previous row (a no-op on row 0: its scores are 0 and 1
     // and every weight is at least 1)
     int rf = 0, F = 0, M = 0x3fffffff, dl = 0;
     if (!init || (w & SW_DRAIN)) {
-      rf = (int)__ldg(RFin + (size_t)s * R);
-      dl = (int)__ldg(RLin + (size_t)s * R);
-      uint32_t k0 = rec.z, k1 = k0 + nb + nm + nf;
-      CHSGA_CHK_RANGE(k0, k1, g.n_ent, 21);
-      const uint32_t kb = k0 + nb, km = kb + nm;
+      if (mine) {
+        rf = (int)__ldg(RFin + (size_t)sv.x * R);
+        dl = (int)__ldg(RLin + (size_t)sv.x * R);
+      }
       F = rf;
-      constexpr int U = 4;  // gathers in flight
-      for (uint32_t k = k0; k < k1; k += U) {
-        uint2 e[U];
+      for (uint32_t k = 0; k < n; k += U) {
+        if (k) entries(k);
         int x[U];
 #pragma unroll
         for (int u = 0; u < U; ++u)
-          if (k + u < k1) e[u] = __ldg(g.ent + k + u);
+          if (k + u < n) x[u] = (int)__ldg(RLin + (size_t)CHSGA_CHK(e[u].x & 0x3FFFFFFFu, g.S, 22) * R) + (int)e[u].y;
 #pragma unroll
         for (int u = 0; u < U; ++u)
-          if (k + u < k1) x[u] = (int)__ldg(RLin + (size_t)CHSGA_CHK(e[u].x, g.S, 22) * R) + (int)e[u].y;
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (k + u < k1) {
-            if (k + u < km) M = min(M, x[u]);
-            if (k + u < kb || k + u >= km) F = min(F, x[u] + (k + u < kb ? 1 : 0));
+          if (k + u < n) {
+            const uint32_t cls = e[u].x >> 30;  // 0 both, 1 M only, 2 F only
+            if (cls != 2) M = min(M, x[u]);
+            if (cls != 1) F = min(F, x[u] + (cls ? 0 : 1));
           }
       }
-      if constexpr (MAT) Fout[s] = (ST)F;
-      if (w & SW_DRAIN) atomicMin(&s_min[((par + 3u) & 3u) * R + r], pack_min(F, __ldg(g.sv_off + s)));
+      if (P > 1 && long_list) {
+        // a list's lanes for one slot lie R apart and take the same way here
+        // (other slots' lanes may not)
+        const uint32_t lane = threadIdx.x & 31u;
+        unsigned lanes = 0;
+#pragma unroll
+        for (int p = 0; p < P; ++p) lanes |= 1u << (p * R);
+        lanes <<= lane / (R * P) * (R * P) + lane % R;
+#pragma unroll
+        for (int o = R; o < R * P; o <<= 1) {
+          F = min(F, __shfl_xor_sync(lanes, F, o));
+          M = min(M, __shfl_xor_sync(lanes, M, o));
+        }
+      }
+      if (!mine || part) continue;
+      if constexpr (MAT) Fout[sv.x] = (ST)F;
+      if (w & SW_DRAIN) {
+        const unsigned long long b = pack_min(F, sv.y);
+        if (b < s_min[((par + 3u) & 3u) * R + r]) atomicMin(&s_min[((par + 3u) & 3u) * R + r], b);
+      }
     }
-    if (w & SW_ACTIVE) {
+    if ((w & SW_ACTIVE) && mine && part == 0) {
       int T, last;
       if (init) {
         T = delta;
         uint32_t left = (uint32_t)delta;
         for (uint32_t j = 0; j < nw; ++j) {
           const size_t wi = (size_t)CHSGA_CHK(rec.x + j, g.words, 23);
-          const uint4 lb = __ldg(g.lab + wi);
+          if (j) lb = __ldg(g.lab + wi);
           const PN x = bits::first_row(bits::mismatch_word(lb.x, lb.y, lb.z, mask), left, min(31u, len - 2 - 32 * j));
           wout[wi * R] = make_uint2(x.p, x.n);
         }
@@ -344,8 +403,10 @@ __global__ void __launch_bounds__(NT, CHSGA_WORDS_THREADS / NT) k_row_words(BitA
         int h = Tc - F;
         for (uint32_t j = 0; j < nw; ++j) {
           const size_t wi = (size_t)CHSGA_CHK(rec.x + j, g.words, 23);
-          const uint4 lb = __ldg(g.lab + wi);
-          const uint2 old = win[wi * R];
+          if (j) {
+            lb = __ldg(g.lab + wi);
+            old = win[wi * R];
+          }
           const uint32_t top = min(31u, len - 2 - 32 * j), valid = 0xFFFFFFFFu >> (31 - top);
           PN x = bits::under_line(PN{old.x, old.y}, valid, gap);
           x = bits::step(x, bits::mismatch_word(lb.x, lb.y, lb.z, mask), h, top);
@@ -354,11 +415,13 @@ __global__ void __launch_bounds__(NT, CHSGA_WORDS_THREADS / NT) k_row_words(BitA
         }
         last = len > 1 ? min(min(dl, F + (int)(len - 1)) + h, T + (int)(len - 1)) : T;
       }
-      RFout[(size_t)s * R] = (ST)T;
-      RLout[(size_t)s * R] = (ST)last;
-      if (w & SW_ENDING) {
-        // the raw row's minimum and its first char
-        const uint32_t f = __ldg(g.sv_off + s);
+      RFout[(size_t)sv.x * R] = (ST)T;
+      RLout[(size_t)sv.x * R] = (ST)last;
+      // the raw row's minimum and its first char; a chain falls by at most
+      // one a char, so most vertices cannot reach the block's best so far
+      if ((w & SW_ENDING) &&
+          max(T - (int)(len - 1), 0) <= (int)min(s_min[par * R + r] >> 32, 0x7FFFFFFFull)) {
+        const uint32_t f = sv.y;
         int cur = T, bm = T;
         uint32_t bc = f;
         for (uint32_t j = 0; j < nw; ++j) {
@@ -391,17 +454,16 @@ __global__ void __launch_bounds__(NT, CHSGA_WORDS_THREADS / NT) k_row_words(BitA
 __global__ void __launch_bounds__(256) k_close_row(BitGraph g, const uint2* __restrict__ bits,
                                                    const uint16_t* __restrict__ RF,
                                                    const uint16_t* __restrict__ RL, int* __restrict__ out) {
-  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= g.S) return;
-  const uint4 rec = __ldg(g.rec + s);
-  const uint32_t nb = rec.w & 0xFFu, nm = (rec.w >> 8) & 0xFFu, nf = (rec.w >> 16) & 0xFFu;
-  int F = RF[s], cur = F;
-  for (uint32_t k = rec.z; k < rec.z + nb + nm + nf; ++k) {
-    if (k >= rec.z + nb && k < rec.z + nb + nm) continue;
-    const uint2 e = __ldg(g.ent + k);
-    F = min(F, (int)RL[e.x] + (int)e.y + (k < rec.z + nb ? 1 : 0));
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= g.S) return;
+  const uint4 rec = __ldg(g.wrec + i);
+  const uint2 sv = __ldg(g.wsv + i);
+  int F = RF[sv.x], cur = F;
+  for (uint32_t k = 0; k < rec.w; ++k) {
+    const uint2 e = __ldg(g.went + rec.z + (i < g.heavy ? 1 : 32) * k);
+    if (e.x >> 30 != 1) F = min(F, (int)RL[e.x & 0x3FFFFFFFu] + (int)e.y + (e.x >> 30 ? 0 : 1));
   }
-  const uint32_t f = __ldg(g.sv_off + s), len = rec.y & 0x1FFFFFFFu;
+  const uint32_t f = sv.y, len = rec.y & 0x1FFFFFFFu;
   out[f] = F;
   for (uint32_t k = 0; k + 1 < len; ++k) {
     const uint2 x = bits[rec.x + (k >> 5)];
@@ -430,7 +492,7 @@ struct BitRowView {
   __device__ __forceinline__ uint2 word(long long i, uint32_t w) const {
     return reinterpret_cast<const uint2*>(M + (size_t)i * pitch)[w];
   }
-  // final score of char k of the vertex with record words at wo
+  // final score of char k of vertex s, its words from wo on
   __device__ __forceinline__ int score(long long i, uint32_t s, uint32_t wo, uint32_t k) const {
     int cur = first_raw(i, s);
     const int F = first_final(i, s);
@@ -459,7 +521,7 @@ __global__ void __launch_bounds__(32) k_walk_bits(GraphPtrs g, BitGraph bg, cons
   long long row = row_hi;
   int status = 0, fail_row = 0;
   uint32_t first = g.sv_off[sv], k = start - first;  // char k of vertex sv
-  uint32_t wo = bg.rec[sv].x;
+  uint32_t wo = bg.wrec[bg.pos[sv]].x;  // first word
   // lane j: vertex sv in row held - j (its first word, enough up to char 32)
   long long held = -1;
   int h_rf = 0, h_f = 0;
@@ -509,7 +571,7 @@ __global__ void __launch_bounds__(32) k_walk_bits(GraphPtrs g, BitGraph bg, cons
         int x = 0x3fffffff;
         if (b + lane < e1) {
           u = list[b + lane];
-          const uint4 rec = bg.rec[u];
+          const uint4 rec = bg.wrec[bg.pos[u]];
           kl = (rec.y & 0x1FFFFFFFu) - 1;
           x = v.score(i - row_lo, u, rec.x, kl);
         }
@@ -571,7 +633,7 @@ __global__ void __launch_bounds__(32) k_walk_bits(GraphPtrs g, BitGraph bg, cons
     if (src_sv != sv || found) {  // an in-edge may lead back to the same vertex (cycles)
       sv = src_sv;
       first = g.sv_off[sv];
-      wo = bg.rec[sv].x;
+      wo = bg.wrec[bg.pos[sv]].x;
       if (row > row_lo) hold();
       held_k = k;
     }

@@ -184,34 +184,16 @@ HostClosure build_closure(const HostLayout& L) {
 #pragma omp parallel for schedule(static)
   for (int64_t q = 0; q < chunks; ++q)
     std::copy(e_chunk[q].begin(), e_chunk[q].end(), c.ent.begin() + e_cnt[q * kChunk]);
-  // vertex records and the label planes of the chain chars
-  uint64_t words = 0;
-  for (uint32_t s = 0; s < S; ++s) {
-    const uint32_t len = L.sv_off[s + 1] - L.sv_off[s];
-    c.rec[4 * (size_t)s] = (uint32_t)words;
-    words += (len - 1 + 31) / 32;
-  }
-  c.words = words;
-  c.lab.assign(4 * (size_t)std::max<uint64_t>(words, 1), 0);
-#pragma omp parallel for schedule(static)
-  for (int64_t s = 0; s < (int64_t)S; ++s) {
-    const uint32_t f = L.sv_off[s], len = L.sv_off[s + 1] - f;
-    auto key = [&](uint32_t ch) { return (L.lab4[ch >> 3] >> ((ch & 7) * 4)) & 0xFu; };
-    uint32_t* r = &c.rec[4 * (size_t)s];
-    r[1] = len | key(f) << 29;
-    r[2] = e_cnt[s];
-    for (uint32_t k = 0; k + 1 < len; ++k) {
-      uint32_t* w = &c.lab[4 * ((size_t)r[0] + k / 32)];
-      const uint32_t x = key(f + 1 + k), bit = 1u << (k & 31);
-      if (x & 1) w[0] |= bit;
-      if (x & 2) w[1] |= bit;
-      if (x & 4) w[2] |= bit;
-    }
-  }
+  auto key = [&](uint32_t ch) { return (L.lab4[ch >> 3] >> ((ch & 7) * 4)) & 0xFu; };
+  auto len_of = [&](uint32_t s) { return L.sv_off[s + 1] - L.sv_off[s]; };
   c.ent16.resize(2 * c.ent.size());
 #pragma omp parallel for schedule(static)
   for (int64_t s = 0; s < (int64_t)S; ++s) {
-    const uint32_t n = c.rec[4 * s + 3], kb = e_cnt[s] + (n & 255), km = kb + ((n >> 8) & 255);
+    uint32_t* r = &c.rec[4 * (size_t)s];
+    r[0] = L.sv_off[s];
+    r[1] = len_of((uint32_t)s) | key(L.sv_off[s]) << 29;
+    r[2] = e_cnt[s];
+    const uint32_t n = r[3], kb = e_cnt[s] + (n & 255), km = kb + ((n >> 8) & 255);
     for (uint32_t k = e_cnt[s]; k < e_cnt[s + 1]; ++k) {
       const uint32_t w = std::min<uint32_t>((uint32_t)c.ent[k].w, 0xFFFE), none = 0xFFFF;
       const uint32_t wm = k < km ? w : none, wf = k < kb ? w + 1 : k >= km ? w : none;
@@ -219,19 +201,94 @@ HostClosure build_closure(const HostLayout& L) {
       c.ent16[2 * (size_t)k + 1] = wm | wf << 16;
     }
   }
-  auto windows = [&](std::vector<uint8_t>& out, uint32_t W, auto&& weight) {
+  for (int i = 0; i < 3; ++i) {
+    const uint32_t W = 32u << i;
+    std::vector<uint8_t>& out = c.by_len[i];
     out.resize(S);
 #pragma omp parallel for schedule(static)
     for (int64_t w0 = 0; w0 < (int64_t)S; w0 += W) {
       const uint32_t n = std::min<uint32_t>(W, S - (uint32_t)w0);
       uint8_t* o = &out[w0];
       std::iota(o, o + n, (uint8_t)0);
-      std::stable_sort(o, o + n, [&](uint8_t x, uint8_t y) { return weight(w0 + x) > weight(w0 + y); });
+      std::stable_sort(o, o + n, [&](uint8_t x, uint8_t y) {
+        return len_of((uint32_t)w0 + x) > len_of((uint32_t)w0 + y);
+      });
     }
+  }
+  // the word kernel's order and arrays
+  c.pos.resize(S);
+  std::vector<uint32_t> at(S);
+  auto count = [&](uint32_t s) { return e_cnt[s + 1] - e_cnt[s]; };
+  {
+    uint32_t h = 0;
+    for (uint32_t s = 0; s < S; ++s)
+      if (count(s) > kWordLight) at[h++] = s;
+    c.heavy = h;
+    for (uint32_t s = 0; s < S; ++s)
+      if (count(s) <= kWordLight) at[h++] = s;
+  }
+#pragma omp parallel for schedule(static)
+  for (int64_t w0 = c.heavy; w0 < (int64_t)S; w0 += kWordWindow) {
+    const auto b = at.begin() + w0, e = at.begin() + std::min<int64_t>(S, w0 + kWordWindow);
+    // by list length, then vertices without chain chars together
+    auto rank = [&](uint32_t s) { return 2 * count(s) + (len_of(s) > 1 ? 1u : 0u); };
+    std::stable_sort(b, e, [&](uint32_t x, uint32_t y) { return rank(x) > rank(y); });
+  }
+#pragma omp parallel for schedule(static)
+  for (int64_t i = 0; i < (int64_t)S; ++i) c.pos[at[i]] = (uint32_t)i;
+  c.wsv.resize((size_t)2 * S);
+  c.wrec.resize((size_t)4 * S);
+  // groups of 32 positions, counted from the first short list on
+  const uint32_t groups = c.heavy / 32 + 1 + (S - c.heavy + 31) / 32;
+  auto g_lo = [&](uint32_t q) {  // positions [g_lo(q), g_lo(q + 1))
+    const uint32_t hg = c.heavy / 32 + 1;
+    return q < hg ? std::min(32 * q, c.heavy) : std::min<uint32_t>(S, c.heavy + 32 * (q - hg));
   };
-  windows(c.by_list, 256, [&](int64_t s) { return e_cnt[s + 1] - e_cnt[s]; });
-  for (int i = 0; i < 3; ++i)
-    windows(c.by_len[i], 32u << i, [&](int64_t s) { return L.sv_off[s + 1] - L.sv_off[s]; });
+  std::vector<uint64_t> g_words((size_t)groups + 1, 0), g_ent((size_t)groups + 1, 0);
+  for (uint32_t q = 0; q < groups; ++q) {
+    uint64_t w = 0, n = 0;
+    for (uint32_t i = g_lo(q); i < g_lo(q + 1); ++i) {
+      w += (len_of(at[i]) - 1 + 31) / 32;
+      n = i < c.heavy ? n + count(at[i]) : std::max<uint64_t>(n, 32ull * count(at[i]));
+    }
+    g_words[q + 1] = g_words[q] + w;
+    g_ent[q + 1] = g_ent[q] + n;
+  }
+  if (g_words[groups] >= (1ull << 31) || g_ent[groups] >= (1ull << 31)) return HostClosure{};
+  c.words = g_words[groups];
+  c.lab.assign(4 * (size_t)std::max<uint64_t>(c.words, 1), 0);
+  c.went.assign((size_t)g_ent[groups], EdgeW{0, 0});
+#pragma omp parallel for schedule(static)
+  for (int64_t q = 0; q < (int64_t)groups; ++q) {
+    uint64_t wo = g_words[q], eo = g_ent[q];
+    const uint32_t lo = g_lo((uint32_t)q);
+    for (uint32_t i = lo; i < g_lo((uint32_t)q + 1); ++i) {
+      const uint32_t s = at[i], f = L.sv_off[s], len = len_of(s), n = count(s);
+      const bool heavy = i < c.heavy;
+      uint32_t* r = &c.wrec[4 * (size_t)i];
+      c.wsv[2 * (size_t)i] = s;
+      c.wsv[2 * (size_t)i + 1] = f;
+      r[0] = (uint32_t)wo;
+      r[1] = len | key(f) << 29;
+      r[2] = (uint32_t)(heavy ? eo : eo + (i - lo));
+      r[3] = n;
+      const uint32_t nb = c.rec[4 * (size_t)s + 3] & 255, nm = (c.rec[4 * (size_t)s + 3] >> 8) & 255;
+      for (uint32_t k = 0; k < n; ++k) {
+        const EdgeW& e = c.ent[e_cnt[s] + k];
+        const uint32_t cls = k < nb ? 0u : k < nb + nm ? 1u : 2u;
+        c.went[r[2] + (heavy ? 1 : 32) * (size_t)k] = EdgeW{(int32_t)((uint32_t)e.src | cls << 30), e.w};
+      }
+      if (heavy) eo += n;
+      for (uint32_t k = 0; k + 1 < len; ++k) {
+        uint32_t* w = &c.lab[4 * (wo + k / 32)];
+        const uint32_t x = key(f + 1 + k), bit = 1u << (k & 31);
+        if (x & 1) w[0] |= bit;
+        if (x & 2) w[1] |= bit;
+        if (x & 4) w[2] |= bit;
+      }
+      wo += (len - 1 + 31) / 32;
+    }
+  }
   c.ok = true;
   return c;
 }

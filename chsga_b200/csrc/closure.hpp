@@ -38,27 +38,45 @@ namespace chsga {
 // the level sweeps are kept.
 constexpr uint32_t kClosureMaxList = 192;
 constexpr uint32_t kClosureMaxGrowth = 6;
+constexpr uint32_t kWordWindow = 512, kWordLight = 8;
 
 struct HostClosure {
   bool ok = false;
-  // 4 words per string vertex: first bit word of its chain chars; length |
-  // label key of the first char << 29; first entry; entries of each class
-  // (both | M only << 8 | F only << 16)
+  // 4 words per string vertex: first char; length | label key of the first
+  // char << 29; first entry; entries of each class (both | M only << 8 | F
+  // only << 16)
   std::vector<uint32_t> rec;
   // {source vertex, weight}, classes in that order; the weight counts for M
   // (a "both" entry has weight w + 1 for F), for F-only entries for F
   std::vector<EdgeW> ent;
-  // per bit word the label planes of its 32 chain chars (bit k of word j of
-  // vertex s = char first(s) + 1 + 32 j + k): {code bit 0, code bit 1, special, 0}
+  // the entries for 16-bit rows: {source vertex, weight for M | weight for F
+  // << 16}, 0xFFFF = no such entry (or a weight no 16-bit score can win with)
+  std::vector<uint32_t> ent16;
+  // order of the vertices inside every window of 32, 64 and 128 by label
+  // length (local indexes)
+  std::vector<uint8_t> by_len[3];
+
+  // The one-read-a-word kernel works in an order of its own. Vertices with
+  // more than kWordLight entries come first (several lanes share such a
+  // list); the others follow, by list length inside every window of
+  // kWordWindow vertices, so that the 32 vertices of a warp end together and
+  // lie side by side in these arrays. Everything below is by position in that
+  // order (the scores stay by string vertex, where neighbours are near).
+  //   heavy     vertices of the first kind
+  //   pos       position of string vertex s
+  //   wsv       {string vertex, first char}
+  //   wrec      4 words: first bit word; length | key << 29; first entry; entries
+  //   went      {source vertex | class << 30 (0 both, 1 M only, 2 F only),
+  //             weight}; a long list is contiguous, entry k of a short one is at
+  //             wrec[2] + 32 k (a group of 32 vertices side by side)
+  //   lab       per bit word the label planes of its 32 chain chars (bit k of
+  //             word j = char first + 1 + 32 j + k): {code bit 0, code bit 1,
+  //             special, 0}
+  uint32_t heavy = 0;
+  std::vector<uint32_t> pos, wsv, wrec;
+  std::vector<EdgeW> went;
   std::vector<uint32_t> lab;
   uint64_t words = 0;
-  // the entries for 16-bit rows: {source, weight for M | weight for F << 16},
-  // 0xFFFF = no such entry (or a weight no 16-bit score can win with)
-  std::vector<uint32_t> ent16;
-  // order of the vertices inside every window of 256 by list length, and
-  // inside every window of 32, 64 and 128 by label length (local indexes)
-  std::vector<uint8_t> by_list;
-  std::vector<uint8_t> by_len[3];
 };
 
 HostClosure build_closure(const HostLayout& L);

@@ -101,9 +101,10 @@ struct GraphDev {
   DevArr<uint8_t> t1_heads;
   DevArr<uint32_t> delta_order;    // k_row_delta: runs of 32 string vertices by decreasing char count
   // bit-row kernels (closure.hpp)
-  DevArr<uint4> cl_rec, cl_lab;
-  DevArr<uint2> cl_ent, cl_ent16;
-  DevArr<uint8_t> cl_by_list, cl_by_len[3];
+  DevArr<uint4> cl_rec, cl_wrec, cl_lab;
+  DevArr<uint2> cl_ent16, cl_went, cl_wsv;
+  DevArr<uint8_t> cl_by_len[3];
+  DevArr<uint32_t> cl_pos;
 };
 
 struct TopDev {
@@ -821,15 +822,23 @@ void bit_step(chsga_ctx& c, BitBufs& b, int par, cudaStream_t s) {
       return;
     }
   }
-  auto launch = [&](auto kern, uint32_t threads) {
-    const uint32_t VB = threads / R;
-    chain_launch(c, kern, std::min((S + VB - 1) / VB, resident_blocks(c, (const void*)kern, (int)threads)), threads, 0, s, a);
+  auto launch = [&](auto kern, uint32_t threads, uint32_t P) {
+    const uint32_t VB = threads / R, items = S + c.g->bg.heavy * (P - 1);
+    chain_launch(c, kern, std::min((items + VB - 1) / VB + 1, resident_blocks(c, (const void*)kern, (int)threads)),
+                 threads, 0, s, a);
   };
+  // Fewer threads a block where blocks of 256 would leave SMs idle. Lanes that
+  // share long lists shorten the longest chain of loads, which is a row-step's
+  // time on a small graph (8 slots, 100 kbp: 10.3 us without, 7.4 with four
+  // lanes), but cost idle lanes once the device is full (5 Mbp: 87 and 101 us).
+  constexpr int P = R <= 8 ? 4 : R <= 16 ? 2 : 1;
   if constexpr (R <= 64) {
-    // fewer threads a block where blocks of 256 would leave SMs idle
-    if ((uint64_t)S * R < 256ull * 2 * c.num_sms) return launch(dev::k_row_words<R, ST, 0, 64>, 64);
+    if ((uint64_t)S * R < 256ull * 2 * c.num_sms) return launch(dev::k_row_words<R, ST, 0, 64, P>, 64, P);
   }
-  launch(dev::k_row_words<R, ST, 0, 256>, 256);
+  if constexpr (R >= 8 && P > 1) {
+    if ((uint64_t)S * R > 2'000'000) return launch(dev::k_row_words<R, ST, 0, 256, 1>, 256, 1);
+  }
+  launch(dev::k_row_words<R, ST, 0, 256, P>, 256, P);
 }
 
 // Buffers of H slots whose rows go to their reads' matrices (traceback): the
@@ -856,12 +865,13 @@ void mat_step(chsga_ctx& c, BitBufs& b, unsigned char* const* mats, int par, cud
   const uint32_t S = c.g->L.S;
   auto launch = [&](auto kern, uint32_t threads) {
     const uint32_t res = std::max(1u, resident_blocks(c, (const void*)kern, (int)threads) / H);
-    chain_launch(c, kern, dim3(std::min((S + threads - 1) / threads, res), H), threads, 0, s, a);
+    const uint32_t items = S + c.g->bg.heavy * 3;
+    chain_launch(c, kern, dim3(std::min((items + threads - 1) / threads + 1, res), H), threads, 0, s, a);
   };
   if ((uint64_t)S * H < 256ull * 2 * c.num_sms)
-    launch(dev::k_row_words<1, uint16_t, H, 64>, 64);
+    launch(dev::k_row_words<1, uint16_t, H, 64, 4>, 64);
   else
-    launch(dev::k_row_words<1, uint16_t, H, 256>, 256);
+    launch(dev::k_row_words<1, uint16_t, H, 256, 4>, 256);
 }
 
 // Every slot idle, q_count reads queued.
@@ -870,6 +880,7 @@ void reset_bit_slots(chsga_ctx& c, BitBufs& b, uint32_t q_count) {
   std::vector<dev::BitState> st(1);
   for (auto& x : st[0].s) x = dev::SlotState{0, 0, 0, -1, 0};
   for (auto& x : st[0].rows) x = dev::SlotRows{nullptr, nullptr};
+  for (auto& x : st[0].next) x = 0;
   st[0].q_head = 0;
   CK(cudaMemcpyAsync(b.state.p, st.data(), sizeof(dev::BitState), cudaMemcpyHostToDevice, c.st));
   dev::StepCtl ctl{};
@@ -1079,21 +1090,40 @@ void upload_graph(chsga_ctx& c, const chsga_graph_host& g) {
   {
     const HostClosure cl = build_closure(L);
     if (cl.ok) {
-      d.cl_rec.upload(to4(cl.rec), s);
-      d.cl_lab.upload(to4(cl.lab), s);
-      std::vector<uint2> ent(cl.ent.size()), ent16(cl.ent.size());
-      if (!ent.empty()) {
-        std::memcpy(ent.data(), cl.ent.data(), ent.size() * sizeof(uint2));
-        std::memcpy(ent16.data(), cl.ent16.data(), ent.size() * sizeof(uint2));
-      }
-      d.cl_ent.upload(ent, s);
-      d.cl_ent16.upload(ent16, s);
-      d.cl_by_list.upload(cl.by_list, s);
+      auto as4 = [&](DevArr<uint4>& to, const std::vector<uint32_t>& v) {
+        to.alloc(v.size() / 4);
+        CK(cudaMemcpyAsync(to.p, v.data(), v.size() * 4, cudaMemcpyHostToDevice, s));
+      };
+      auto as2 = [&](DevArr<uint2>& to, const void* v, size_t n) {
+        to.alloc(n);
+        if (n) CK(cudaMemcpyAsync(to.p, v, n * sizeof(uint2), cudaMemcpyHostToDevice, s));
+      };
+      as4(d.cl_rec, cl.rec);
+      as4(d.cl_wrec, cl.wrec);
+      as4(d.cl_lab, cl.lab);
+      as2(d.cl_ent16, cl.ent16.data(), cl.ent16.size() / 2);
+      as2(d.cl_went, cl.went.data(), cl.went.size());
+      d.cl_pos.upload(cl.pos, s);
+      as2(d.cl_wsv, cl.wsv.data(), cl.wsv.size() / 2);
       for (int i = 0; i < 3; ++i) d.cl_by_len[i].upload(cl.by_len[i], s);
       CK(cudaStreamSynchronize(s));  // the host vectors die with this scope
       lg->bits = true;
-      lg->bg = dev::BitGraph{L.S, (uint32_t)cl.ent.size(), cl.words, d.cl_rec.p, d.cl_ent.p, d.cl_ent16.p, d.cl_lab.p,
-                             d.cl_by_list.p, nullptr, d.sv_off.p, d.lab4.p, L.N};
+      dev::BitGraph& b = lg->bg;
+      b.S = L.S;
+      b.N = L.N;
+      b.n_ent = (uint32_t)(cl.ent16.size() / 2);
+      b.n_went = (uint32_t)cl.went.size();
+      b.heavy = cl.heavy;
+      b.words = cl.words;
+      b.rec = d.cl_rec.p;
+      b.ent16 = d.cl_ent16.p;
+      b.sv_off = d.sv_off.p;
+      b.lab4 = d.lab4.p;
+      b.pos = d.cl_pos.p;
+      b.wsv = d.cl_wsv.p;
+      b.wrec = d.cl_wrec.p;
+      b.went = d.cl_went.p;
+      b.lab = d.cl_lab.p;
     }
   }
   lg->nul_label = false;
@@ -1620,6 +1650,8 @@ void traceback_bits(chsga_ctx& c, const char* read, uint32_t len, const chsga_tb
     std::vector<dev::BitState> st(1);
     for (auto& x : st[0].s) x = dev::SlotState{0, 0, 0, -1, 0};
     for (auto& x : st[0].rows) x = dev::SlotRows{nullptr, nullptr};
+    for (auto& x : st[0].next) x = 0;
+    st[0].next[0] = (unsigned char)read[a + 1];
     st[0].s[0] = dev::SlotState{0, (uint32_t)(z + 1), (uint32_t)a, 0, 0};
     st[0].rows[0].cur = mat;
     st[0].q_head = 0;
