@@ -13,12 +13,13 @@
 // with W[i][j] the weight from input i to unit j.
 //
 // Loss: L = 1/(2B) * sum_b sum_j (o_bj - t_bj)^2 over a batch of B, t the
-// standardised log targets. Kernels (one thread per sample unless noted):
-//   k_cm_forward   standardise, three layers; keeps x^, h1, h2, dL/do
-//   k_cm_backward  dz2 = (W3 dL/do) * [h2 > 0], dz1 = (W2 dz2) * [h1 > 0]
+// standardised log targets. Kernels:
+//   k_cm_sample    one thread per (sample, hidden unit): standardise, three
+//                  layers (keeps x^, h1, h2, dL/do), then
+//                  dz2 = (W3 dL/do) * [h2 > 0], dz1 = (W2 dz2) * [h1 > 0]
 //   k_cm_wgrad     one thread per parameter: sums activation x delta over
-//                  the batch in sample order (deterministic, no atomics)
-//   k_cm_adam      Adam update, one thread per parameter
+//                  the batch in sample order (deterministic, no atomics) and
+//                  makes the Adam update
 //   k_cm_loss      one block: the batch loss in a fixed reduction order
 #include <cuda_runtime.h>
 
@@ -55,106 +56,91 @@ static_assert(NPARAM == CHSGA_CM_NUM_PARAMS, "parameter count");
            std::string(#x) + ": " + cudaGetErrorString(e_));                                \
   } while (0)
 
-// Forward for samples idx[0..n) (idx == nullptr: 0..n-1). X raw features
-// [*, F]; Y raw targets [*, O] or nullptr (inference). Outputs per batch
-// position b: xn[b][F], h1[b][H], h2[b][H] (when non-null), o[b][O] in
-// standardised log units, and d[b][O] = (o - t) / n when Y is given.
-__global__ void __launch_bounds__(128) k_cm_forward(const float* __restrict__ P,
-                                                    const float* __restrict__ norm,
-                                                    const float* __restrict__ X,
-                                                    const float* __restrict__ Y,
-                                                    const uint32_t* __restrict__ idx, uint32_t n,
-                                                    float* __restrict__ xn, float* __restrict__ h1,
-                                                    float* __restrict__ h2, float* __restrict__ o,
-                                                    float* __restrict__ d) {
-  __shared__ float sP[NPARAM];
-  __shared__ float sN[NNORM];
-  for (int i = threadIdx.x; i < NPARAM; i += blockDim.x) sP[i] = P[i];
-  for (int i = threadIdx.x; i < NNORM; i += blockDim.x) sN[i] = norm[i];
+// Forward and, with targets, backward for samples idx[0..n) (idx == nullptr:
+// 0..n-1), kCmSamples samples a block and one thread per (sample, hidden
+// unit). X raw features [*, F]; Y raw targets [*, O] or nullptr (inference).
+// Outputs per batch position b: o[b][O] in standardised log units; with Y
+// also xn[b][F], h1[b][H], h2[b][H], d[b][O] = (o - t) / n, dz1[b][H],
+// dz2[b][H].
+//
+// A batch of 64 has 64 samples: with a thread per sample the two layers were
+// 8,000 dependent operations on two warps (about 40 us of a 60 us step). Every
+// sum still runs over its inputs in their order in one thread, so the results
+// are the same bit for bit.
+constexpr int kCmSamples = 4;
+__global__ void __launch_bounds__(kCmSamples* H) k_cm_sample(
+    const float* __restrict__ P, const float* __restrict__ norm, const float* __restrict__ X,
+    const float* __restrict__ Y, const uint32_t* __restrict__ idx, uint32_t n, float* __restrict__ xn,
+    float* __restrict__ h1, float* __restrict__ h2, float* __restrict__ o, float* __restrict__ d,
+    float* __restrict__ dz1, float* __restrict__ dz2) {
+  __shared__ float sW2[H][H + 1];  // rows a word apart in the banks: read by row and by column
+  __shared__ float sa[kCmSamples][H], sz[kCmSamples][H], sg[kCmSamples][O];
+  const int q = threadIdx.x / H, j = threadIdx.x % H;
+  const uint32_t b = blockIdx.x * kCmSamples + q;
+  for (int i = threadIdx.x; i < H * H; i += kCmSamples * H) sW2[i / H][i % H] = P[OFF_W2 + i];
+  if (b < n) {
+    const uint32_t s = idx ? idx[b] : b;
+    float a = P[OFF_B1 + j];
+#pragma unroll
+    for (int i = 0; i < F; ++i) {
+      const float x = (X[(size_t)s * F + i] - norm[i]) / norm[F + i];
+      if (Y && j == i) xn[(size_t)b * F + i] = x;
+      a = fmaf(x, P[OFF_W1 + i * H + j], a);
+    }
+    sa[q][j] = fmaxf(a, 0.f);
+  }
   __syncthreads();
-  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
-  const uint32_t s = idx ? idx[b] : b;
-  float x[F];
-#pragma unroll
-  for (int i = 0; i < F; ++i) {
-    x[i] = (X[(size_t)s * F + i] - sN[i]) / sN[F + i];
-    if (xn) xn[(size_t)b * F + i] = x[i];
+  if (b < n) {
+    float z = P[OFF_B2 + j];
+#pragma unroll 16
+    for (int i = 0; i < H; ++i) z = fmaf(sa[q][i], sW2[i][j], z);
+    sz[q][j] = fmaxf(z, 0.f);
   }
-  float a1[H];
-#pragma unroll
-  for (int j = 0; j < H; ++j) a1[j] = sP[OFF_B1 + j];
-#pragma unroll
-  for (int i = 0; i < F; ++i)
-#pragma unroll
-    for (int j = 0; j < H; ++j) a1[j] = fmaf(x[i], sP[OFF_W1 + i * H + j], a1[j]);
-#pragma unroll
-  for (int j = 0; j < H; ++j) {
-    a1[j] = fmaxf(a1[j], 0.f);
-    if (h1) h1[(size_t)b * H + j] = a1[j];
-  }
-  float out[O];
-#pragma unroll
-  for (int k = 0; k < O; ++k) out[k] = sP[OFF_B3 + k];
-  // layer 2 one unit at a time, folded straight into layer 3
-  for (int j = 0; j < H; ++j) {
-    float z = sP[OFF_B2 + j];
-#pragma unroll
-    for (int i = 0; i < H; ++i) z = fmaf(a1[i], sP[OFF_W2 + i * H + j], z);
-    z = fmaxf(z, 0.f);
-    if (h2) h2[(size_t)b * H + j] = z;
-#pragma unroll
-    for (int k = 0; k < O; ++k) out[k] = fmaf(z, sP[OFF_W3 + j * O + k], out[k]);
-  }
-#pragma unroll
-  for (int k = 0; k < O; ++k) {
-    o[(size_t)b * O + k] = out[k];
-    if (Y && d) {
-      const float t = (logf(Y[(size_t)s * O + k]) - sN[2 * F + k]) / sN[2 * F + O + k];
-      d[(size_t)b * O + k] = (out[k] - t) / (float)n;
+  __syncthreads();
+  if (b < n && j < O) {
+    const uint32_t s = idx ? idx[b] : b;
+    float out = P[OFF_B3 + j];
+#pragma unroll 16
+    for (int i = 0; i < H; ++i) out = fmaf(sz[q][i], P[OFF_W3 + i * O + j], out);
+    o[(size_t)b * O + j] = out;
+    if (Y) {
+      const float t = (logf(Y[(size_t)s * O + j]) - norm[2 * F + j]) / norm[2 * F + O + j];
+      const float g = (out - t) / (float)n;
+      d[(size_t)b * O + j] = g;
+      sg[q][j] = g;
     }
   }
-}
-
-__global__ void __launch_bounds__(128) k_cm_backward(const float* __restrict__ P,
-                                                     const float* __restrict__ h1,
-                                                     const float* __restrict__ h2,
-                                                     const float* __restrict__ d, uint32_t n,
-                                                     float* __restrict__ dz1,
-                                                     float* __restrict__ dz2) {
-  __shared__ float sW2[H * H];
-  __shared__ float sW3[H * O];
-  for (int i = threadIdx.x; i < H * H; i += blockDim.x) sW2[i] = P[OFF_W2 + i];
-  for (int i = threadIdx.x; i < H * O; i += blockDim.x) sW3[i] = P[OFF_W3 + i];
+  if (!Y) return;
   __syncthreads();
-  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
-  float g[O];
-#pragma unroll
-  for (int k = 0; k < O; ++k) g[k] = d[(size_t)b * O + k];
-  float e2[H];
-#pragma unroll
-  for (int j = 0; j < H; ++j) {
+  const float a1 = sa[q][j], z2 = sz[q][j];
+  __syncthreads();
+  if (b < n) {
     float v = 0.f;
 #pragma unroll
-    for (int k = 0; k < O; ++k) v = fmaf(sW3[j * O + k], g[k], v);
-    e2[j] = h2[(size_t)b * H + j] > 0.f ? v : 0.f;
-    dz2[(size_t)b * H + j] = e2[j];
+    for (int k = 0; k < O; ++k) v = fmaf(P[OFF_W3 + j * O + k], sg[q][k], v);
+    v = z2 > 0.f ? v : 0.f;
+    h1[(size_t)b * H + j] = a1;
+    h2[(size_t)b * H + j] = z2;
+    dz2[(size_t)b * H + j] = v;
+    sz[q][j] = v;
   }
-  for (int i = 0; i < H; ++i) {
+  __syncthreads();
+  if (b < n) {
     float v = 0.f;
-#pragma unroll
-    for (int j = 0; j < H; ++j) v = fmaf(sW2[i * H + j], e2[j], v);
-    dz1[(size_t)b * H + i] = h1[(size_t)b * H + i] > 0.f ? v : 0.f;
+#pragma unroll 16
+    for (int i = 0; i < H; ++i) v = fmaf(sW2[j][i], sz[q][i], v);
+    dz1[(size_t)b * H + j] = a1 > 0.f ? v : 0.f;
   }
 }
 
 // One thread per parameter: dW[i][j] = sum_b a[b][i] * delta[b][j] and
-// db[j] = sum_b delta[b][j], summed in sample order.
+// db[j] = sum_b delta[b][j], summed in sample order; then, when M is given,
+// the parameter's Adam update.
 __global__ void k_cm_wgrad(const float* __restrict__ xn, const float* __restrict__ h1,
                            const float* __restrict__ h2, const float* __restrict__ dz1,
                            const float* __restrict__ dz2, const float* __restrict__ d, uint32_t n,
-                           float* __restrict__ G) {
+                           float* __restrict__ G, float* __restrict__ P, float* __restrict__ M,
+                           float* __restrict__ V, float lr, float b1, float b2, float eps, float c1, float c2) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= NPARAM) return;
   const float* a = nullptr;  // activation column (nullptr: bias)
@@ -175,19 +161,15 @@ __global__ void k_cm_wgrad(const float* __restrict__ xn, const float* __restrict
   }
   float s = 0.f;
   if (a) {
+#pragma unroll 16
     for (uint32_t b = 0; b < n; ++b) s = fmaf(a[(size_t)b * as + i], e[(size_t)b * es + j], s);
   } else {
+#pragma unroll 16
     for (uint32_t b = 0; b < n; ++b) s += e[(size_t)b * es + j];
   }
   G[p] = s;
-}
-
-__global__ void k_cm_adam(float* __restrict__ P, const float* __restrict__ G, float* __restrict__ M,
-                          float* __restrict__ V, float lr, float b1, float b2, float eps, float c1,
-                          float c2) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= NPARAM) return;
-  const float g = G[p];
+  if (!M) return;
+  const float g = s;
   const float m = b1 * M[p] + (1.f - b1) * g;
   const float v = b2 * V[p] + (1.f - b2) * g * g;
   M[p] = m;
@@ -282,11 +264,14 @@ struct chsga_cost_model {
     dz2.alloc((size_t)n * H);
   }
   // forward + backward of the batch idx (or all n) into G
+  void sample(const uint32_t* didx, uint32_t n) {
+    k_cm_sample<<<(n + kCmSamples - 1) / kCmSamples, kCmSamples * H, 0, st>>>(
+        P.p, N.p, X.p, Y.p, didx, n, xn.p, h1.p, h2.p, o.p, d.p, dz1.p, dz2.p);
+  }
   void grad(const uint32_t* didx, uint32_t n) {
-    const unsigned g = (n + 127) / 128;
-    k_cm_forward<<<g, 128, 0, st>>>(P.p, N.p, X.p, Y.p, didx, n, xn.p, h1.p, h2.p, o.p, d.p);
-    k_cm_backward<<<g, 128, 0, st>>>(P.p, h1.p, h2.p, d.p, n, dz1.p, dz2.p);
-    k_cm_wgrad<<<(NPARAM + 127) / 128, 128, 0, st>>>(xn.p, h1.p, h2.p, dz1.p, dz2.p, d.p, n, G.p);
+    sample(didx, n);
+    k_cm_wgrad<<<(NPARAM + 127) / 128, 128, 0, st>>>(xn.p, h1.p, h2.p, dz1.p, dz2.p, d.p, n, G.p, P.p, nullptr,
+                                                     nullptr, 0.f, 0.f, 0.f, 0.f, 1.f, 1.f);
     CKM(cudaGetLastError());
   }
 };
@@ -445,7 +430,12 @@ chsga_status chsga_cm_train(chsga_cost_model* m, const float* x, const float* y,
     m->upload();
     m->stage(x, y, n);
     m->batch_bufs(B);
-    m->idx.alloc(n);
+    // the sample orders of up to kCmOrders / n epochs go to the device at once,
+    // so the host waits for it only when they are used up
+    constexpr size_t kCmOrders = 1u << 20;
+    const uint32_t span = (uint32_t)std::min<size_t>(o.epochs, std::max<size_t>(1, kCmOrders / n));
+    m->idx.alloc((size_t)span * n);
+    std::vector<uint32_t> orders((size_t)span * n);
     CKM(cudaMemsetAsync(m->M.p, 0, NPARAM * 4, m->st));
     CKM(cudaMemsetAsync(m->V.p, 0, NPARAM * 4, m->st));
     std::vector<uint32_t> perm(n);
@@ -453,19 +443,26 @@ chsga_status chsga_cm_train(chsga_cost_model* m, const float* x, const float* y,
     uint64_t s = o.seed ^ 0x7EA1Bull;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     uint64_t t = 0;
-    for (uint32_t ep = 0; ep < o.epochs; ++ep) {
-      for (uint32_t i = n; i > 1; --i) std::swap(perm[i - 1], perm[splitmix(s) % i]);
-      CKM(cudaMemcpyAsync(m->idx.p, perm.data(), (size_t)n * 4, cudaMemcpyHostToDevice, m->st));
-      for (uint32_t off = 0; off + B <= n; off += B) {  // full batches only
-        m->grad(m->idx.p + off, B);
-        ++t;
-        const float c1 = 1.f - std::pow(b1, (float)t), c2 = 1.f - std::pow(b2, (float)t);
-        k_cm_adam<<<(NPARAM + 127) / 128, 128, 0, m->st>>>(m->P.p, m->G.p, m->M.p, m->V.p, o.lr, b1,
-                                                           b2, eps, c1, c2);
-        CKM(cudaGetLastError());
+    for (uint32_t ep0 = 0; ep0 < o.epochs; ep0 += span) {
+      const uint32_t eps_here = std::min(span, o.epochs - ep0);
+      for (uint32_t ep = 0; ep < eps_here; ++ep) {
+        for (uint32_t i = n; i > 1; --i) std::swap(perm[i - 1], perm[splitmix(s) % i]);
+        std::copy(perm.begin(), perm.end(), orders.begin() + (size_t)ep * n);
       }
-      // the permutation buffer is rewritten next epoch: wait for its readers
+      // the earlier epochs still read the orders
       CKM(cudaStreamSynchronize(m->st));
+      CKM(cudaMemcpyAsync(m->idx.p, orders.data(), (size_t)eps_here * n * 4, cudaMemcpyHostToDevice, m->st));
+      for (uint32_t ep = 0; ep < eps_here; ++ep)
+        for (uint32_t off = 0; off + B <= n; off += B) {  // full batches only
+          m->sample(m->idx.p + (size_t)ep * n + off, B);
+          ++t;
+          const float c1 = 1.f - std::pow(b1, (float)t), c2 = 1.f - std::pow(b2, (float)t);
+          k_cm_wgrad<<<(NPARAM + 127) / 128, 128, 0, m->st>>>(m->xn.p, m->h1.p, m->h2.p, m->dz1.p, m->dz2.p, m->d.p,
+                                                              B, m->G.p, m->P.p, m->M.p, m->V.p, o.lr, b1, b2, eps, c1,
+                                                              c2);
+          CKM(cudaGetLastError());
+        }
+      CKM(cudaStreamSynchronize(m->st));  // `orders` is rewritten
     }
     m->download();
     m->trained = true;
@@ -487,8 +484,8 @@ chsga_status chsga_cm_predict(chsga_cost_model* m, const float* x, uint32_t n, f
     check_data(x, nullptr, n);
     m->stage(x, nullptr, n);
     m->o.alloc((size_t)n * O);
-    k_cm_forward<<<(n + 127) / 128, 128, 0, m->st>>>(m->P.p, m->N.p, m->X.p, nullptr, nullptr, n,
-                                                     nullptr, nullptr, nullptr, m->o.p, nullptr);
+    k_cm_sample<<<(n + kCmSamples - 1) / kCmSamples, kCmSamples * H, 0, m->st>>>(
+        m->P.p, m->N.p, m->X.p, nullptr, nullptr, n, nullptr, nullptr, nullptr, m->o.p, nullptr, nullptr, nullptr);
     CKM(cudaGetLastError());
     std::vector<float> z((size_t)n * O);
     CKM(cudaMemcpyAsync(z.data(), m->o.p, z.size() * 4, cudaMemcpyDeviceToHost, m->st));

@@ -745,10 +745,13 @@ bool bits_apply(const chsga_ctx& c) {
 
 // 32 to 128 slots of 16-bit scores slice the bits over the slots; fewer slots,
 // 32-bit scores and vertices too long for one thread's serial chain keep a
-// read's bits in words.
+// read's bits in words. So do graphs of at most 400,000 (vertex, slot) pairs:
+// there a row-step is one thread's chain of loads, which is shorter with
+// words (64 slots on 5,500 vertices: 13.9 us against 14.5, 32 slots 11.4
+// against 14.6; on 22,000 vertices 28.7 against 22.0 and 19.0 against 18.4).
 template <int R, typename ST>
 bool bits_sliced(const chsga_ctx& c) {
-  return R >= 32 && std::is_same_v<ST, uint16_t> && c.g->L.max_len <= 512;
+  return R >= 32 && std::is_same_v<ST, uint16_t> && c.g->L.max_len <= 512 && (uint64_t)c.g->L.S * R > 400'000;
 }
 
 template <int R, typename ST>
