@@ -245,14 +245,19 @@ HostClosure build_closure(const HostLayout& L) {
     return q < hg ? std::min(32 * q, c.heavy) : std::min<uint32_t>(S, c.heavy + 32 * (q - hg));
   };
   std::vector<uint64_t> g_words((size_t)groups + 1, 0), g_ent((size_t)groups + 1, 0);
-  for (uint32_t q = 0; q < groups; ++q) {
+#pragma omp parallel for schedule(static)
+  for (int64_t q = 0; q < (int64_t)groups; ++q) {
     uint64_t w = 0, n = 0;
-    for (uint32_t i = g_lo(q); i < g_lo(q + 1); ++i) {
+    for (uint32_t i = g_lo((uint32_t)q); i < g_lo((uint32_t)q + 1); ++i) {
       w += (len_of(at[i]) - 1 + 31) / 32;
       n = i < c.heavy ? n + count(at[i]) : std::max<uint64_t>(n, 32ull * count(at[i]));
     }
-    g_words[q + 1] = g_words[q] + w;
-    g_ent[q + 1] = g_ent[q] + n;
+    g_words[q + 1] = w;
+    g_ent[q + 1] = n;
+  }
+  for (uint32_t q = 0; q < groups; ++q) {
+    g_words[q + 1] += g_words[q];
+    g_ent[q + 1] += g_ent[q];
   }
   if (g_words[groups] >= (1ull << 31) || g_ent[groups] >= (1ull << 31)) return HostClosure{};
   c.words = g_words[groups];

@@ -94,45 +94,33 @@ HostLayout build_layout(const chsga_graph_host& g) {
   require(max_len < (1u << 29), CHSGA_ERR_UNSUPPORTED, "string vertex labels must be shorter than 2^29 chars");
   L.max_len = max_len;
   const chsga_csr& cg = g.char_graph;
-  // in-CSR with sources in ascending order, as build_in_csr (align.hpp:220-242):
-  // counted and placed in parallel, then each target's sources sorted
-  std::vector<uint64_t> ioff(N + 1, 0);
-  uint64_t bad_t = 0;
-#pragma omp parallel for reduction(+ : bad_t) schedule(dynamic, 1 << 14)
-  for (int64_t u = 0; u < (int64_t)N; ++u)
+  // The in-edges of build_in_csr (align.hpp:220-242). A char after the first
+  // of its string must have the single in-edge c-1 -> c, which the char before
+  // it shows; only first chars (a tenth of the chars) need an in-CSR, its
+  // sources in ascending order.
+  uint64_t bad_t = 0, bad_chain = kNone;
+  L.vin_off.assign(S + 1, 0);
+#pragma omp parallel for reduction(+ : bad_t) reduction(min : bad_chain) schedule(dynamic, 1 << 14)
+  for (int64_t u = 0; u < (int64_t)N; ++u) {
+    uint32_t next = 0;  // edges to the char after u
     for (uint64_t e = cg.offset[u]; e < cg.offset[u + 1]; ++e) {
-      if (cg.target[e] >= N) {
+      const uint32_t t = cg.target[e];
+      if (t >= N) {
         ++bad_t;
         continue;
       }
-      __atomic_fetch_add(&ioff[cg.target[e] + 1], 1ull, __ATOMIC_RELAXED);
+      const uint32_t v = vertex_of[t];
+      if (L.sv_off[v] == t)
+        __atomic_fetch_add(&L.vin_off[v + 1], 1u, __ATOMIC_RELAXED);
+      else if (t == (uint32_t)u + 1)
+        ++next;
+      else
+        bad_chain = std::min(bad_chain, (uint64_t)t);
     }
+    if ((uint64_t)u + 1 < L.sv_off[vertex_of[u] + 1] && next != 1) bad_chain = std::min(bad_chain, (uint64_t)u + 1);
+  }
   require(bad_t == 0, CHSGA_ERR_FORMAT, "char edge target out of range");
-  for (uint32_t v = 0; v < N; ++v) ioff[v + 1] += ioff[v];
-  std::vector<uint32_t> isrc(ioff[N]);
-  {
-    std::vector<uint64_t> cur(ioff.begin(), ioff.end() - 1);
-#pragma omp parallel for schedule(dynamic, 1 << 14)
-    for (int64_t u = 0; u < (int64_t)N; ++u)
-      for (uint64_t e = cg.offset[u]; e < cg.offset[u + 1]; ++e)
-        isrc[__atomic_fetch_add(&cur[cg.target[e]], 1ull, __ATOMIC_RELAXED)] = (uint32_t)u;
-#pragma omp parallel for schedule(dynamic, 1 << 14)
-    for (int64_t v = 0; v < (int64_t)N; ++v)
-      if (ioff[v + 1] - ioff[v] > 1) std::sort(isrc.begin() + ioff[v], isrc.begin() + ioff[v + 1]);
-  }
-  L.char_in_edges = ioff[N];
-  L.vin_off.assign(S + 1, 0);
-  uint64_t bad_chain = kNone;
-#pragma omp parallel for reduction(min : bad_chain) schedule(static)
-  for (int64_t s = 0; s < (int64_t)S; ++s) {
-    const uint32_t f = L.sv_off[s], e = L.sv_off[s + 1];
-    for (uint32_t c = f + 1; c < e; ++c)
-      if (!(ioff[c + 1] - ioff[c] == 1 && isrc[ioff[c]] == c - 1)) {
-        bad_chain = std::min(bad_chain, (uint64_t)c);
-        break;
-      }
-    L.vin_off[s + 1] = (uint32_t)(ioff[f + 1] - ioff[f]);
-  }
+  L.char_in_edges = cg.offset[N];
   if (bad_chain != kNone)
     fail(CHSGA_ERR_UNSUPPORTED,
          "char " + std::to_string(bad_chain) + " is not the chain successor of char " +
@@ -142,13 +130,18 @@ HostLayout build_layout(const chsga_graph_host& g) {
   for (uint32_t s = 0; s < S; ++s) L.vin_off[s + 1] += L.vin_off[s];
   L.vin_src.resize(L.vin_off[S]);
   L.vin_srcv.resize(L.vin_off[S]);
-#pragma omp parallel for schedule(static)
-  for (int64_t s = 0; s < (int64_t)S; ++s) {
-    const uint32_t f = L.sv_off[s];
-    for (uint64_t k = 0; k < ioff[f + 1] - ioff[f]; ++k) {
-      uint32_t u = isrc[ioff[f] + k];
-      L.vin_src[L.vin_off[s] + k] = u;
-      L.vin_srcv[L.vin_off[s] + k] = vertex_of[u];
+  {
+    std::vector<uint32_t> cur(L.vin_off.begin(), L.vin_off.end() - 1);
+#pragma omp parallel for schedule(dynamic, 1 << 14)
+    for (int64_t u = 0; u < (int64_t)N; ++u)
+      for (uint64_t e = cg.offset[u]; e < cg.offset[u + 1]; ++e) {
+        const uint32_t t = cg.target[e], v = vertex_of[t];
+        if (L.sv_off[v] == t) L.vin_src[__atomic_fetch_add(&cur[v], 1u, __ATOMIC_RELAXED)] = (uint32_t)u;
+      }
+#pragma omp parallel for schedule(dynamic, 1 << 14)
+    for (int64_t s = 0; s < (int64_t)S; ++s) {
+      std::sort(L.vin_src.begin() + L.vin_off[s], L.vin_src.begin() + L.vin_off[s + 1]);
+      for (uint32_t k = L.vin_off[s]; k < L.vin_off[s + 1]; ++k) L.vin_srcv[k] = vertex_of[L.vin_src[k]];
     }
   }
 
