@@ -191,6 +191,17 @@ def algorithmic_delta_row_bytes(st, slots, multi):
             + 3 * N / 8 + 12 * S + 4 * e_first)
 
 
+def algorithmic_bit_row_bytes(st, slots, score_bytes=2):
+    """Bytes one bit-row step must move: two difference bits per char and
+    slot read and written (N R / 2), the raw first and last score of every
+    vertex read and written (4 w S R), labels (3N/8), 16 bytes per vertex
+    record and 8 per hierarchy edge and first-char in-edge (the closure
+    lists hold a few more entries)."""
+    N, S = st["num_chars"], st["num_strings"]
+    edges = st["pch_up_edges"] + st["pch_down_edges"] + st["num_char_edges"] - (N - S)
+    return N * slots / 2 + 4 * score_bytes * S * slots + 3 * N / 8 + 16 * S + 8 * edges
+
+
 def algorithmic_sweep_bytes(st, lay, slots, score_bytes, fl_first=True):
     """Bytes per row-step of the grid-wide sweep kernels below the top
     region (16-byte pull-list heads and vertex words, w bytes per score):
@@ -611,8 +622,8 @@ def run_top_compare(args):
 
 
 def run_launch_compare(args):
-    """Device time of the same reads through the CUDA-graph chain of
-    row-step kernels (with and without programmatic dependent launch between
+    """Device time of the same reads through the bit-row steps, through the
+    CUDA-graph chain of level-sweep kernels (with and without programmatic dependent launch between
     its kernels) and through the persistent row-step kernel, at 1, 8 and
     128 slots, on the config-2-mix graph; the one-slot chain also with the
     one-thread-per-vertex row kernel (the plain path's row kernel before the
@@ -640,21 +651,22 @@ def run_launch_compare(args):
               ((1, 4, 31_000, 1000), (8, 32, 31_001, 2000), (128, 256, 31_002, 2000)) if R in want]
     for R, reads in shapes:
         cells = sum(len(r) for r in reads) * N
-        runs = [("graphs", dict(use_graphs=cb.LAUNCH_GRAPHS, steps_per_graph=16)),
-                ("graphs_no_pdl", dict(use_graphs=cb.LAUNCH_GRAPHS, steps_per_graph=16, ctx=ctx_nopdl)),
+        sweeps = dict(use_graphs=cb.LAUNCH_GRAPHS, steps_per_graph=16, top_vertices=8000)
+        runs = [("bit_rows", dict(use_graphs=cb.LAUNCH_GRAPHS, steps_per_graph=16)),
+                ("bit_rows_no_pdl", dict(use_graphs=cb.LAUNCH_GRAPHS, steps_per_graph=16, ctx=ctx_nopdl)),
+                ("graphs", sweeps),
+                ("graphs_no_pdl", dict(sweeps, ctx=ctx_nopdl)),
                 ("persistent", dict(use_graphs=cb.LAUNCH_PERSISTENT, steps_per_graph=16)),
                 ("persistent_64", dict(use_graphs=cb.LAUNCH_PERSISTENT, steps_per_graph=64))]
         if R == 1:
             runs.append(("graphs_direct_row", dict(use_graphs=cb.LAUNCH_GRAPHS, steps_per_graph=16,
                                                    row_kernel=cb.ROW_DIRECT)))
         if R >= 8:
-            runs.append(("graphs_pull_unbounded", dict(use_graphs=cb.LAUNCH_GRAPHS, steps_per_graph=16,
-                                                       ctx=ctx_gen)))
+            runs.append(("graphs_pull_unbounded", dict(sweeps, ctx=ctx_gen)))
         if R >= 64:
-            runs.append(("graphs_pull_coop", dict(use_graphs=cb.LAUNCH_GRAPHS, steps_per_graph=16,
-                                                  ctx=ctx_coop)))
+            runs.append(("graphs_pull_coop", dict(sweeps, ctx=ctx_coop)))
         if R == 128:
-            # AUTO runs delta rows here; the 16-bit stream rows for comparison
+            # the chain runs delta rows here; the 16-bit stream rows for comparison
             runs.append(("graphs_stream_rows", dict(use_graphs=cb.LAUNCH_GRAPHS, steps_per_graph=16,
                                                     row_kernel=cb.ROW_STREAM)))
         rec = {"slots": R, "reads": len(reads), "bases": sum(len(r) for r in reads)}
@@ -678,7 +690,7 @@ def run_launch_compare(args):
     pctx = cb.Context(0, flags=cb.FLAG_PROFILE).load(g)
     one = make_reads(g, 4, 31_000, len_max=1000)
     for name, rk in (("tile_row", cb.ROW_AUTO), ("direct_row", cb.ROW_DIRECT)):
-        pctx.align_scores_batched(one[:2], slots=1, row_kernel=rk)
+        pctx.align_scores_batched(one[:2], slots=1, row_kernel=rk, top_vertices=8000)
         pr = pctx.profile()
         st = max(1, pr["row_launches"])
         out["plain_profile_" + name] = {k.replace("_ms", "_us"): 1e3 * pr[k] / st for k in
@@ -688,7 +700,7 @@ def run_launch_compare(args):
     if 128 in want:
         reads128 = make_reads(g, 128, 31_003, len_max=1000)
         for name, cx in (("pull16", pctx), ("pull16_unbounded", pctx_gen), ("pull16c", pctx_coop)):
-            cx.align_scores_batched(reads128, slots=128)
+            cx.align_scores_batched(reads128, slots=128, top_vertices=8000)
             pr = cx.profile()
             st = max(1, pr["row_launches"])
             out["batched_profile_" + name] = {k.replace("_ms", "_us"): 1e3 * pr[k] / st for k in
@@ -906,20 +918,26 @@ def profiled_roofline(cb, g, st, multi, device, R, opts, peak, src, row_bits, cl
     pctx.close()
     w = pr["row_bits"] // 8
     row_avg_s = pr["row_ms"] / max(1, pr["row_launches"]) / 1e3
-    # AUTO: delta rows for score-only steps at 128 slots (this pass is score-only)
+    # AUTO without a level grouping: the bit-row kernels, unless the graph has no closure
+    # lists (then delta rows for score-only steps at 128 slots)
+    bits = pr["launches"] < 3 * pr["row_launches"] + 64  # one kernel a row-step
     auto16 = "k_row_delta" if R == 128 else ("k_row_stream" if R >= 64 else ("k_row_dpx" if R >= 2 else "k_row_t1"))
     kname = {cb.ROW_DIRECT: "k_row_direct", cb.ROW_TILED: "k_row_tiled", cb.ROW_DPX: "k_row_dpx",
              cb.ROW_STREAM: "k_row_stream", cb.ROW_DELTA: "k_row_delta"}.get(
         opts["row_kernel"] if R > 1 else 0, auto16 if pr["row_bits"] == 16 else "k_row_direct")
     if pr["row_bits"] == 32 and kname in ("k_row_stream", "k_row_dpx", "k_row_delta"):
         kname = "k_row_direct"  # the 16-bit kernels do not run 32-bit rows
-    ab = algorithmic_delta_row_bytes(st, R, multi) if kname == "k_row_delta" else \
+    if bits:
+        kname = "k_row_sliced" if R >= 32 and w == 2 and st["num_strings"] * R > 400_000 else "k_row_words"
+    ab = algorithmic_bit_row_bytes(st, R, w) if bits else \
+        algorithmic_delta_row_bytes(st, R, multi) if kname == "k_row_delta" else \
         algorithmic_row_bytes(st, R, multi, w)
     tr = ncu_traffic(kname)
     total = pr["row_ms"] + pr["sweep_up_ms"] + pr["top_ms"] + pr["sweep_down_ms"] + pr["other_ms"]
     # working set of one row-step: two score rows, BV and FL, graph arrays
     S = st["num_strings"]
-    work = 2 * w * st["num_chars"] * R + 2 * 2 * w * S * R + 3 * st["num_chars"] / 8 + 40 * S
+    work = (ab - st["num_chars"] * R / 4) if bits else \
+        2 * w * st["num_chars"] * R + 2 * 2 * w * S * R + 3 * st["num_chars"] / 8 + 40 * S
     out = {
         "bound": "hbm", "kernel": f"{kname}<{R}>", "row_bits": int(pr["row_bits"]),
         "achieved": ab / row_avg_s / 1e9, "peak": peak, "unit": "GB/s",
@@ -965,6 +983,9 @@ def profiled_roofline(cb, g, st, multi, device, R, opts, peak, src, row_bits, cl
                               "frac": s_ab / s_avg / 1e9 / peak,
                               "row_step_ms": sum(qs[k] for k in ("row_ms", "sweep_up_ms", "top_ms", "sweep_down_ms",
                                                                  "other_ms")) / max(1, qs["row_launches"])}
+    if bits:
+        out["limiter"] = "load latency and instruction issue (one pass; no sweeps)"
+        return out
     # sweep kernels below the top region (the top region the run used)
     lay = g.check_layout(R, pr["row_bits"], opts["top_vertices"] if R > 1 else 0)
     up_b, down_b = algorithmic_sweep_bytes(st, lay, R, w, fl_first=kname != "k_row_delta")
@@ -1096,10 +1117,13 @@ def main():
         "metric": METRIC, "value": value, "unit": "GCUPS", "n_gpus": ws, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": dev_s * 1e3 / args.steps, "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None, "dtype": "int32", "data": "synthetic",
-        "row_storage": (("2-bit delta rows (per char and slot, T[c] - T[c-1] + 1 in 0..2 within a "
+        "row_storage": (("bit rows: two difference bits per char and slot and the raw first and last score "
+                        "of every vertex in 16 bits (graphs without closure lists: 2-bit delta rows)"
+                        if opts["row_kernel"] == 0 and opts["top_vertices"] == 0 else
+                        ("2-bit delta rows (per char and slot, T[c] - T[c-1] + 1 in 0..2 within a "
                          "vertex) plus the raw first score of every vertex in 16 bits, u16x2 DPX "
                          "arithmetic" if opts["slots"] == 128 and opts["row_kernel"] in (0, 5) else
-                         "uint16 rows with u16x2 DPX arithmetic")
+                         "uint16 rows with u16x2 DPX arithmetic"))
                         + ": int32 results exactly, since every row-i value is at most i + 1 (reads "
                           "of at most 65000 bases; longer reads run int32 rows)"),
         "config": {"workload": WORKLOAD, "num_chars": N, "num_strings": st["num_strings"],

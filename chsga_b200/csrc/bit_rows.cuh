@@ -225,6 +225,14 @@ __host__ __device__ constexpr size_t bits_row_bytes(uint64_t words, uint32_t S) 
 }
 
 // ---------------------------------------------------------------------------
+// What bounds it: at one slot the chain of dependent loads of a vertex (state
+// of the launch before, record and entries, gathers, stores) on a small graph
+// (5.4 us a row-step at 100 kbp, of which about 3 us are launch and state), and
+// the number of loads in flight on a large one (17.5 us at 5 Mbp; the level
+// sweeps and their row kernel took 24.6 and 85 us in 12 and 18 launches). The
+// longest lists set the chain: four dependent rounds less for lists of up to
+// 60 entries took the 5 Mbp graph from 21.8 to 17.5 us.
+//
 // k_row_words: one thread per (string vertex, slot), a vertex's chain in
 // words of 32 chars. Slots are interleaved (RF[s * R + r], word w of slot r at
 // w * R + r), so the gathers of neighbouring slots share sectors; with MAT
@@ -505,11 +513,29 @@ struct BitRowView {
   }
 };
 
-__global__ void __launch_bounds__(32) k_walk_bits(GraphPtrs g, BitGraph bg, const unsigned char* __restrict__ M,
-                                                  size_t pitch, long long row_lo, long long row_hi, uint32_t start,
-                                                  const unsigned char* __restrict__ read, WalkOp* __restrict__ ops,
-                                                  uint32_t max_ops, WalkOut* __restrict__ out, int match_n) {
+// One walk: rows [row_lo, row_hi] of the matrix at M, from char `start`.
+struct WalkJob {
+  const unsigned char* M;
+  const unsigned char* read;
+  long long row_lo, row_hi;
+  uint32_t start, pad;
+};
+
+// Block j takes jobs[j] (null: the one job given by value) and writes out[j]
+// and at most max_ops ops from ops + j * max_ops on. A walk is a chain of
+// round trips, so the reads that finish together walk together.
+__global__ void __launch_bounds__(32) k_walk_bits(GraphPtrs g, BitGraph bg, size_t pitch,
+                                                  const WalkJob* __restrict__ jobs, WalkJob one,
+                                                  WalkOp* __restrict__ ops, uint32_t max_ops,
+                                                  WalkOut* __restrict__ out, int match_n) {
   constexpr unsigned FULL = 0xFFFFFFFFu;
+  const WalkJob job = jobs ? jobs[blockIdx.x] : one;
+  const unsigned char* const M = job.M;
+  const unsigned char* const read = job.read;
+  const long long row_lo = job.row_lo, row_hi = job.row_hi;
+  const uint32_t start = job.start;
+  ops += (size_t)blockIdx.x * max_ops;
+  out += blockIdx.x;
   const int lane = threadIdx.x;
   const BitRowView v{M, pitch, bits_row_rf(bg.words), bits_row_f(bg.words, bg.S)};
   uint32_t lo = 0, hi = g.S;
@@ -646,6 +672,14 @@ __global__ void __launch_bounds__(32) k_walk_bits(GraphPtrs g, BitGraph bg, cons
 // word pair {P, N} g of char c (slots 32g .. 32g+31) at c * R/32 + g. Each
 // char of 32 slots is a handful of logic operations, where the packed 16-bit
 // update spends tens of instructions.
+//
+// What bounds it: 5 Mbp graph, 128 slots, 305 us a row-step (the sweeps'
+// chain: 771): 0.94 GB from and to HBM is 145 us at the copy peak and 144 M
+// warp-instructions are 125 us of issue; the rest is load latency at 32 warps
+// an SM (8.7 of 14 stall cycles an instruction). Without the gathers it takes
+// 100 us less, without the chain 150. Blocks of 128 threads with barriers
+// between the passes took 353, five or six gathers in flight 316-357 (spills
+// past 64 registers), prefetches to L2 or shared memory 374-440.
 //
 // A warp takes a group of vertices in three passes:
 //   1  lane = (vertex, 8 slots): closure and first char in 16-bit pairs; the

@@ -149,6 +149,16 @@ struct RowTileDev {
   bool ok = false;
 };
 
+// chsga_align_scores without a launch mode of its own (CHSGA_PLAIN_LAUNCH):
+// level sweeps and long calls replay a CUDA graph of 16 row-steps, bit rows of
+// fewer than kPlainStreamRows rows are launched one by one. A bit row-step is
+// one launch of about 2.5 us on the host and 5 on the device, so the host
+// stays ahead and the graph's capture and instantiation (0.2 ms a call) is
+// all it would add: 3 reads of 100 bp on 100 kbp 1.89 ms with it, 1.68
+// without; 5 of 150 bp on 5 Mbp 13.4 and 13.3.
+constexpr uint32_t kPlainAuto = ~0u;
+constexpr uint64_t kPlainStreamRows = 4096;
+
 constexpr uint32_t kRow16Max = 65000;  // longest read whose rows fit uint16  // 2 x int32 per vertex in shared memory
 constexpr int kTopThreads = 1024;
 
@@ -185,11 +195,12 @@ struct chsga_ctx {
   // top regions other than the graph's default, by their vertex limit
   std::map<uint32_t, std::unique_ptr<chsga::TopDev>> tops;
   const chsga::TopDev* top_sel = nullptr;  // this call's top region (nullptr: the default)
+  bool sweeps = false;                     // this call chose a level grouping: level sweeps
   int num_sms = 148;
   chsga::RowKernel row_kernel = chsga::RowKernel::Auto;
-  // launch mode of the one-read path (chsga_align_scores): CHSGA_LAUNCH_*;
-  // CUDA graphs, measured faster than the persistent kernel at one slot
-  uint32_t plain_mode = CHSGA_LAUNCH_GRAPHS;
+  // launch mode of the one-read path (chsga_align_scores): CHSGA_LAUNCH_*, or
+  // kPlainAuto (see there)
+  uint32_t plain_mode = chsga::kPlainAuto;
   // programmatic dependent launch between the kernels of a row-step
   // (CHSGA_PDL=0 turns it off; measured 1-4 % faster per row-step)
   bool pdl = true;
@@ -198,6 +209,7 @@ struct chsga_ctx {
   // upward levels in the form bounded by the level's largest edge list
   // (CHSGA_PULL_LEAN=0 runs the unbounded form everywhere)
   bool pull_lean = true;
+  std::map<const void*, uint32_t> resident;  // resident blocks of the bit-row kernels
   // resident blocks of k_row_delta on this device (0 until the first 128-slot buffers)
   uint32_t delta_grid = 0;
   chsga::DevArr<unsigned char> reads;
@@ -740,7 +752,7 @@ void launch_persist(chsga_ctx& c, SlotBufs& b, uint32_t grid, uint32_t steps, cu
 // closure lists exist and the caller chose neither a row kernel nor a level
 // grouping (those select the level-sweep kernels).
 bool bits_apply(const chsga_ctx& c) {
-  return c.g->bits && c.row_kernel == RowKernel::Auto && c.top_sel == nullptr;
+  return c.g->bits && c.row_kernel == RowKernel::Auto && !c.sweeps;
 }
 
 // 32 to 128 slots of 16-bit scores slice the bits over the slots; fewer slots,
@@ -796,11 +808,16 @@ dev::BitArgs bit_args(const chsga_ctx& c, BitBufs& b, int par) {
   return a;
 }
 
-// Blocks of `threads` threads of kernel k that fit the device at once.
-uint32_t resident_blocks(const chsga_ctx& c, const void* k, int threads) {
-  int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, 0));
-  return (uint32_t)std::max(per_sm, 1) * (uint32_t)c.num_sms;
+// Blocks of `threads` threads of kernel k that fit the device at once (asked
+// once per context and kernel: a row-step is launched every few microseconds).
+uint32_t resident_blocks(chsga_ctx& c, const void* k, int threads) {
+  uint32_t& n = c.resident[k];
+  if (!n) {
+    int per_sm = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, 0));
+    n = (uint32_t)std::max(per_sm, 1) * (uint32_t)c.num_sms;
+  }
+  return n;
 }
 
 template <int R, typename ST>
@@ -1520,8 +1537,8 @@ void walk_bits(chsga_ctx& c, const unsigned char* M, int64_t lo, int64_t hi, uin
   c.h_walk.alloc(bytes);
   auto* out = reinterpret_cast<dev::WalkOut*>(c.tb_walk.p);
   auto* ops = reinterpret_cast<dev::WalkOp*>(c.tb_walk.p + head);
-  dev::k_walk_bits<<<1, 32, 0, c.st>>>(c.g->gp, c.g->bg, M, bit_row_bytes(c), lo, hi, start, c.reads.p, ops, max_ops,
-                                       out, match_n(c));
+  dev::k_walk_bits<<<1, 32, 0, c.st>>>(c.g->gp, c.g->bg, bit_row_bytes(c), nullptr,
+                                       dev::WalkJob{M, c.reads.p, lo, hi, start, 0}, ops, max_ops, out, match_n(c));
   check_launch();
   // a path has about one op a row: copy that many with the result
   const uint32_t guess = (uint32_t)std::min<uint64_t>(max_ops, (uint64_t)(hi - lo) + (uint64_t)(hi - lo) / 8 + 16);
@@ -1851,6 +1868,12 @@ void traceback_batched(chsga_ctx& parent, const char* const* reads, const uint32
   wout.alloc(wcap);
   std::vector<dev::WalkOut> hout(wcap);
   std::vector<dev::WalkOp> hops(max_ops);
+  DevArr<dev::WalkJob> djobs;
+  PinnedArr<dev::WalkJob> hjobs;
+  if (bits) {
+    djobs.alloc(wcap);
+    hjobs.alloc(wcap);
+  }
   // matrices held at once: what is free once the engine's buffers exist;
   // the stream-ordered pool keeps freed matrices for the next reads instead
   // of unmapping them at every synchronisation
@@ -1877,16 +1900,19 @@ void traceback_batched(chsga_ctx& parent, const char* const* reads, const uint32
       for (uint32_t i = i0; i < i1; ++i) {
         const dev::CompletionRec& r = hring.p[(size_t)k * nf + i];
         const uint32_t id = (uint32_t)r.id, len = rl[id], j = i - i0;
-        if (len > 1 && bits)
-          dev::k_walk_bits<<<1, 32, 0, c.side>>>(c.g->gp, c.g->bg, reinterpret_cast<unsigned char*>(hm[id]),
-                                                  row_bytes, 0, (long long)len - 1, r.vertex, c.reads.p + roff[id],
-                                                  ops_buf.p + (size_t)j * max_ops, (uint32_t)max_ops, wout.p + j,
-                                                  match_n(c));
+        if (bits)  // a one-base read's job is an empty walk
+          hjobs.p[j] = dev::WalkJob{reinterpret_cast<const unsigned char*>(hm[id]), c.reads.p + roff[id], 0,
+                                    (long long)len - 1, r.vertex, 0};
         else if (len > 1)
           dev::k_walk<uint16_t><<<1, 1, 0, c.side>>>(c.g->gp, hm[id], pitch, 0, (long long)len - 1,
                                                       r.vertex, c.reads.p + roff[id],
                                                       ops_buf.p + (size_t)j * max_ops, (uint32_t)max_ops,
                                                       wout.p + j, match_n(c));
+      }
+      if (bits) {
+        CK(cudaMemcpyAsync(djobs.p, hjobs.p, (i1 - i0) * sizeof(dev::WalkJob), cudaMemcpyHostToDevice, c.side));
+        dev::k_walk_bits<<<i1 - i0, 32, 0, c.side>>>(c.g->gp, c.g->bg, row_bytes, djobs.p, dev::WalkJob{}, ops_buf.p,
+                                                     (uint32_t)max_ops, wout.p, match_n(c));
       }
       check_launch();
       CK(cudaMemcpyAsync(hout.data(), wout.p, (i1 - i0) * sizeof(dev::WalkOut), cudaMemcpyDeviceToHost,
@@ -2238,8 +2264,9 @@ struct CallKnobs {
   chsga_ctx& c;
   RowKernel rk;
   const TopDev* ts;
+  bool sw;
   CallKnobs(chsga_ctx& cx, uint32_t row_kernel, uint32_t top_vertices)
-      : c(cx), rk(cx.row_kernel), ts(cx.top_sel) {
+      : c(cx), rk(cx.row_kernel), ts(cx.top_sel), sw(cx.sweeps) {
     require(row_kernel <= CHSGA_ROW_DELTA, CHSGA_ERR_INVALID_ARG, "row_kernel must be CHSGA_ROW_*");
     if (row_kernel == CHSGA_ROW_DIRECT) c.row_kernel = RowKernel::Direct;
     if (row_kernel == CHSGA_ROW_TILED) c.row_kernel = RowKernel::Tiled;
@@ -2247,10 +2274,12 @@ struct CallKnobs {
     if (row_kernel == CHSGA_ROW_STREAM) c.row_kernel = RowKernel::Stream;
     if (row_kernel == CHSGA_ROW_DELTA) c.row_kernel = RowKernel::Delta;
     c.top_sel = top_for(c, top_vertices);
+    c.sweeps = top_vertices != 0;
   }
   ~CallKnobs() {
     c.row_kernel = rk;
     c.top_sel = ts;
+    c.sweeps = sw;
   }
 };
 
@@ -2754,7 +2783,13 @@ chsga_status chsga_align_scores(chsga_ctx* c, const char* const* reads, const ui
   return guarded_ctx(c, [&] {
     require(c && (n == 0 || (reads && lens && scores_out)), CHSGA_ERR_INVALID_ARG, "null argument");
     require(c->loaded, CHSGA_ERR_INVALID_ARG, "no graph loaded");
-    scores_with<1>(*c, reads, lens, n, scores_out, c->plain_mode, 16,
+    uint32_t mode = c->plain_mode;
+    if (mode == kPlainAuto) {
+      uint64_t rows = 0;
+      for (uint32_t i = 0; i < n; ++i) rows += lens[i];
+      mode = bits_apply(*c) && rows < kPlainStreamRows ? CHSGA_LAUNCH_STREAM : CHSGA_LAUNCH_GRAPHS;
+    }
+    scores_with<1>(*c, reads, lens, n, scores_out, mode, 16,
                    (uint32_t)std::strtoul(std::getenv("CHSGA_ROW_BITS") ? std::getenv("CHSGA_ROW_BITS") : "0",
                                           nullptr, 10));
   });

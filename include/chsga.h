@@ -271,10 +271,17 @@ typedef struct {
   uint32_t row_kernel;    /* CHSGA_ROW_*: which row kernel runs; 0 = AUTO */
   uint32_t top_vertices;  /* level grouping: hierarchy vertices (highest levels first) swept
                              by the one-CTA-per-slot top kernel, the levels below one grid
-                             launch each; 0 = 8000; at most 23000 (the most shared memory
-                             holds) */
+                             launch each; at most 23000 (the most shared memory holds).
+                             0 = no level sweeps where the graph's closure lists exist (see
+                             CHSGA_ROW_AUTO below), else 8000 */
 } chsga_batch_opts;
-/* Row kernels. With 16-bit rows, slots >= 2 and no string vertex label over
+/* Row kernels. AUTO runs the bit-row kernels, one launch a row-step: the
+ * hierarchy closure is one minimum per vertex over lists made when the graph
+ * is loaded, and a row is the first and last score of every vertex and two
+ * difference bits per char. They need the lists, which graphs made mostly of
+ * one-char vertices do not get, and top_vertices = 0. The other kernels run
+ * with the level-by-level sweeps. Where AUTO cannot use bit rows: with 16-bit
+ * rows, slots >= 2 and no string vertex label over
  * 512 chars, AUTO runs DELTA for score-only steps at 128 slots, STREAM for
  * other steps at 64 slots and up, DPX below, else DIRECT; one slot runs the
  * tile kernel (one warp per tile of whole vertices, one lane per 8 chars).
@@ -410,7 +417,8 @@ uint64_t chsga_ops_to_cigar(const chsga_op* ops, uint64_t n, char* buf, uint64_t
  * CHSGA_FLAG_PROFILE (CUDA graphs off, one sync per row-step) the five kernel
  * groups of every row-step are timed with CUDA events: row_ms (k_row),
  * sweep_up_ms (upward level kernels), top_ms (top region), sweep_down_ms
- * (downward levels with the final propagation), other_ms (slot advance). */
+ * (downward levels with the final propagation), other_ms (slot advance). A
+ * bit-row step is one kernel: row_ms, the others hold only the events' own time. */
 typedef struct {
   double row_ms, sweep_up_ms, top_ms, sweep_down_ms, other_ms, total_ms;
   uint64_t row_bits;      /* 16 or 32: storage width of the score rows */
