@@ -820,6 +820,29 @@ uint32_t resident_blocks(chsga_ctx& c, const void* k, int threads) {
   return n;
 }
 
+// The word kernel's row-step.
+template <int R, typename ST>
+void launch_words(chsga_ctx& c, const dev::BitArgs& a, cudaStream_t s) {
+  const uint32_t S = c.g->L.S;
+  auto launch = [&](auto kern, uint32_t threads, uint32_t P) {
+    const uint32_t VB = threads / R, items = S + c.g->bg.heavy * (P - 1);
+    chain_launch(c, kern, std::min((items + VB - 1) / VB + 1, resident_blocks(c, (const void*)kern, (int)threads)),
+                 threads, 0, s, a);
+  };
+  // Fewer threads a block where blocks of 256 would leave SMs idle. Lanes that
+  // share long lists shorten the longest chain of loads, which is a row-step's
+  // time on a small graph (8 slots, 100 kbp: 10.3 us without, 7.4 with four
+  // lanes), but cost idle lanes once the device is full (5 Mbp: 87 and 101 us).
+  constexpr int P = R <= 8 ? 4 : R <= 16 ? 2 : 1;
+  if constexpr (R <= 64) {
+    if ((uint64_t)S * R < 256ull * 2 * c.num_sms) return launch(dev::k_row_words<R, ST, 0, 64, P>, 64, P);
+  }
+  if constexpr (R >= 8 && P > 1) {
+    if ((uint64_t)S * R > 2'000'000) return launch(dev::k_row_words<R, ST, 0, 256, 1>, 256, 1);
+  }
+  launch(dev::k_row_words<R, ST, 0, 256, P>, 256, P);
+}
+
 template <int R, typename ST>
 void bit_step(chsga_ctx& c, BitBufs& b, int par, cudaStream_t s) {
   dev::BitArgs a = bit_args(c, b, par);
@@ -842,23 +865,7 @@ void bit_step(chsga_ctx& c, BitBufs& b, int par, cudaStream_t s) {
       return;
     }
   }
-  auto launch = [&](auto kern, uint32_t threads, uint32_t P) {
-    const uint32_t VB = threads / R, items = S + c.g->bg.heavy * (P - 1);
-    chain_launch(c, kern, std::min((items + VB - 1) / VB + 1, resident_blocks(c, (const void*)kern, (int)threads)),
-                 threads, 0, s, a);
-  };
-  // Fewer threads a block where blocks of 256 would leave SMs idle. Lanes that
-  // share long lists shorten the longest chain of loads, which is a row-step's
-  // time on a small graph (8 slots, 100 kbp: 10.3 us without, 7.4 with four
-  // lanes), but cost idle lanes once the device is full (5 Mbp: 87 and 101 us).
-  constexpr int P = R <= 8 ? 4 : R <= 16 ? 2 : 1;
-  if constexpr (R <= 64) {
-    if ((uint64_t)S * R < 256ull * 2 * c.num_sms) return launch(dev::k_row_words<R, ST, 0, 64, P>, 64, P);
-  }
-  if constexpr (R >= 8 && P > 1) {
-    if ((uint64_t)S * R > 2'000'000) return launch(dev::k_row_words<R, ST, 0, 256, 1>, 256, 1);
-  }
-  launch(dev::k_row_words<R, ST, 0, 256, P>, 256, P);
+  launch_words<R, ST>(c, a, s);
 }
 
 // Buffers of H slots whose rows go to their reads' matrices (traceback): the
@@ -1503,6 +1510,7 @@ struct TbMatrix {
         t_peak_bytes = std::max(t_peak_bytes, t_live_bytes);
       }
     } else {
+      c.tb_mat.release();  // a large matrix may need the room
       own.alloc(bytes);
       p = own.p;
     }
@@ -2007,7 +2015,11 @@ struct NoallocLayout {
       res_vertex, res_t0, res_t1, out, end;
 };
 
-NoallocLayout noalloc_layout(uint64_t N, uint64_t S, uint64_t read_bytes, uint64_t n) {
+// words != ~0: the bit-row engine's buffers (score rows = raw first scores, bv
+// = the words, fl = raw last scores, slots = the two states, best = its four
+// minima) instead of the level sweeps'.
+NoallocLayout noalloc_layout(uint64_t N, uint64_t S, uint64_t read_bytes, uint64_t n, uint64_t words = ~0ull) {
+  const bool bits = words != ~0ull;
   NoallocLayout l{};
   uint64_t at = 0;
   auto take = [&](uint64_t bytes) {
@@ -2016,13 +2028,13 @@ NoallocLayout noalloc_layout(uint64_t N, uint64_t S, uint64_t read_bytes, uint64
     return o;
   };
   // the same sizes as the context's own buffers for one slot of 16-bit rows
-  l.rows[0] = take((N + 32) * sizeof(uint16_t));
-  l.rows[1] = take((N + 32) * sizeof(uint16_t));
-  l.bv = take(2 * S * sizeof(uint16_t));
+  l.rows[0] = take((bits ? S : N + 32) * sizeof(uint16_t));
+  l.rows[1] = take((bits ? S : N + 32) * sizeof(uint16_t));
+  l.bv = take(bits ? words * 8 : 2 * S * sizeof(uint16_t));
   l.fl = take(2 * (S + 16) * sizeof(uint16_t));
-  l.slots = take(sizeof(dev::SlotState));
+  l.slots = take(bits ? 2 * sizeof(dev::BitState) : sizeof(dev::SlotState));
   l.word = take(sizeof(uint32_t));
-  l.best = take(sizeof(unsigned long long));
+  l.best = take(4 * sizeof(unsigned long long));
   l.ctl = take(sizeof(dev::StepCtl));
   l.reads = take(read_bytes);
   l.lens = take(n * sizeof(uint32_t));
@@ -2038,6 +2050,7 @@ NoallocLayout noalloc_layout(uint64_t N, uint64_t S, uint64_t read_bytes, uint64
 }
 
 struct NoallocBufs {
+  bool bits;
   uint16_t* rows[2];
   uint16_t* BV;
   uint16_t* FL;
@@ -2163,6 +2176,33 @@ void noalloc_row_step(chsga_ctx& c, const NoallocBufs& b, const uint16_t* D, uin
   check_launch();
 }
 
+// One bit-row step of one slot on the buffers of the fixed array.
+void noalloc_bit_step(chsga_ctx& c, const NoallocBufs& b, int par) {
+  auto* states = reinterpret_cast<dev::BitState*>(b.slots);
+  const uint32_t S = c.g->L.S;
+  dev::BitArgs a{};
+  a.g = c.g->bg;
+  a.RFin = b.rows[par];
+  a.RFout = b.rows[par ^ 1];
+  a.RLin = b.FL + (size_t)par * S;
+  a.RLout = b.FL + (size_t)(par ^ 1) * S;
+  a.bits = b.BV;
+  a.st_in = states + par;
+  a.st_out = states + (par ^ 1);
+  a.best = b.best;
+  a.ctl = b.ctl;
+  a.queue = b.queue;
+  a.reads = b.reads;
+  a.res_score = b.res_score;
+  a.res_vertex = b.res_vertex;
+  a.res_t0 = b.res_t0;
+  a.res_t1 = b.res_t1;
+  a.qmask = 0xFFFFFFFFu;
+  a.special = c.g->L.special;
+  a.match_n = match_n(c);
+  launch_words<1, uint16_t>(c, a, c.st);
+}
+
 void scores_noalloc_enqueue(chsga_ctx& c, const NoallocBufs& b, const char* const* reads,
                             const uint32_t* lens, uint32_t n, uint64_t total, uint32_t m,
                             int32_t* out);
@@ -2190,14 +2230,20 @@ void scores_noalloc(chsga_ctx& c, const char* const* reads, const uint32_t* lens
   }
   require(max_len <= kRow16Max, CHSGA_ERR_UNSUPPORTED,
           "chsga_align_scores_noalloc keeps 16-bit rows: reads of at most 65000 bases");
-  const NoallocLayout l = noalloc_layout(c.g->L.N, c.g->L.S, total, n);
+  NoallocLayout l = noalloc_layout(c.g->L.N, c.g->L.S, total, n);
   require(l.end <= CHSGA_NOALLOC_SCRATCH_BYTES, CHSGA_ERR_OOM,
           "chsga_align_scores_noalloc needs " + std::to_string(l.end) +
               " bytes of its fixed device array for this graph and these reads; the array holds " +
               std::to_string((uint64_t)CHSGA_NOALLOC_SCRATCH_BYTES) + " (CHSGA_NOALLOC_SCRATCH_BYTES)");
   if (n == 0) return;
+  // bit rows where their buffers fit too (8 bytes a word of up to 32 chain
+  // chars instead of 4 a char, so nearly always)
+  const NoallocLayout lb = noalloc_layout(c.g->L.N, c.g->L.S, total, n, c.g->bits ? c.g->bg.words : 0);
+  const bool bits = bits_apply(c) && lb.end <= CHSGA_NOALLOC_SCRATCH_BYTES;
+  if (bits) l = lb;
   unsigned char* base = d.base;
   NoallocBufs b{};
+  b.bits = bits;
   b.rows[0] = reinterpret_cast<uint16_t*>(base + l.rows[0]);
   b.rows[1] = reinterpret_cast<uint16_t*>(base + l.rows[1]);
   b.BV = reinterpret_cast<uint16_t*>(base + l.bv);
@@ -2237,9 +2283,16 @@ void scores_noalloc_enqueue(chsga_ctx& c, const NoallocBufs& b, const char* cons
     if (lens[i]) CK(cudaMemcpyAsync(b.reads + off, reads[i], lens[i], cudaMemcpyHostToDevice, s));
     off += lens[i];
   }
+  if (b.bits) {  // the first state idle (k_noalloc_prepare sets its slot), the minima unset
+    CK(cudaMemsetAsync(b.slots, 0, 2 * sizeof(dev::BitState), s));
+    CK(cudaMemsetAsync(b.best, 0xFF, 4 * sizeof(unsigned long long), s));
+  }
   k_noalloc_prepare<<<1, 1024, 0, s>>>(b.lens, n, b.queue, b.slot_of, b.slots, b.ctl, b.best);
   check_launch();
-  if (m) {
+  if (m && b.bits) {
+    // the rows, the last read's closure, its hand-in
+    for (uint64_t k = 0; k < total + 2; ++k) noalloc_bit_step(c, b, (int)(k & 1));
+  } else if (m) {
     // admit the first read, then one row per step: `total` steps finish every read
     dev::k_advance<1><<<1, 128, 0, s>>>(b.slots, b.queue, b.reads, b.best, b.res_score,
                                         b.res_vertex, b.res_t0, b.res_t1, b.word, b.ctl,
