@@ -1493,29 +1493,52 @@ void traceback_rows(chsga_ctx& c, const char* read, uint32_t len, const chsga_tb
 // read's row-steps). Larger ones live for one call.
 constexpr uint64_t kKeepMatrix = 1ull << 30;
 
-// A device buffer of one traceback: the context's kept one where it fits,
-// counted by the request meter as if it were allocated for the call.
+// Leaves the request meter as it was: what a context keeps between calls is
+// counted by the calls that use it, for as long as they do.
+struct MeterPause {
+  const int64_t live = t_live_bytes, peak = t_peak_bytes;
+  ~MeterPause() {
+    t_live_bytes = live;
+    t_peak_bytes = peak;
+  }
+};
+
+// Bytes of kept memory the request meter counts while this lives.
+struct MeterHold {
+  const int64_t bytes;
+  explicit MeterHold(uint64_t n) : bytes((int64_t)n) {
+    t_live_bytes += bytes;
+    t_peak_bytes = std::max(t_peak_bytes, t_live_bytes);
+  }
+  ~MeterHold() { t_live_bytes -= bytes; }
+  MeterHold(const MeterHold&) = delete;
+  MeterHold& operator=(const MeterHold&) = delete;
+};
+
+// A device buffer of one traceback: the context's kept one where it fits. The
+// request meter counts it while it lives, whichever it is.
 struct TbMatrix {
   DevArr<unsigned char> own;
   unsigned char* p = nullptr;
-  int64_t counted = 0;
+  std::unique_ptr<MeterHold> hold;
   TbMatrix(chsga_ctx& c, uint64_t bytes) {
-    if (bytes <= kKeepMatrix) {
-      const bool fresh = !c.tb_mat.p || c.tb_mat.n < bytes;
-      c.tb_mat.alloc(bytes);
-      p = c.tb_mat.p;
-      if (!fresh) {
-        counted = (int64_t)bytes;
-        t_live_bytes += counted;
-        t_peak_bytes = std::max(t_peak_bytes, t_live_bytes);
+    {
+      MeterPause pause;
+      if (bytes <= kKeepMatrix) {
+        c.tb_mat.alloc(bytes);
+        p = c.tb_mat.p;
+      } else {
+        c.tb_mat.release();  // a large matrix may need the room
+        own.alloc(bytes);
+        p = own.p;
       }
-    } else {
-      c.tb_mat.release();  // a large matrix may need the room
-      own.alloc(bytes);
-      p = own.p;
     }
+    hold = std::make_unique<MeterHold>(bytes);
   }
-  ~TbMatrix() { t_live_bytes -= counted; }
+  ~TbMatrix() {
+    MeterPause pause;
+    own.release();
+  }
   TbMatrix(const TbMatrix&) = delete;
   TbMatrix& operator=(const TbMatrix&) = delete;
 };
@@ -1541,7 +1564,11 @@ void walk_bits(chsga_ctx& c, const unsigned char* M, int64_t lo, int64_t hi, uin
                std::vector<dev::WalkOp>& path, uint32_t* landing) {
   const uint32_t max_ops = (uint32_t)(2 * (hi - lo) + 2 * (uint64_t)len + 16);
   const size_t head = 32, bytes = head + max_ops * sizeof(dev::WalkOp);
-  c.tb_walk.alloc(bytes);
+  {
+    MeterPause pause;
+    c.tb_walk.alloc(bytes);
+  }
+  const MeterHold hold(bytes);
   c.h_walk.alloc(bytes);
   auto* out = reinterpret_cast<dev::WalkOut*>(c.tb_walk.p);
   auto* ops = reinterpret_cast<dev::WalkOp*>(c.tb_walk.p + head);
