@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "common.hpp"
+#include "device_memory.hpp"
 
 namespace chsga {
 extern thread_local std::string g_last_error;
@@ -208,7 +209,7 @@ struct Buf {
     if (p) cudaFree(p);
     p = nullptr;
     n = 0;
-    CKM(cudaMalloc((void**)&p, std::max<size_t>(count, 1) * sizeof(T)));
+    CKM(device_malloc((void**)&p, std::max<size_t>(count, 1) * sizeof(T)));
     n = count;
   }
 };

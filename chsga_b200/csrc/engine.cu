@@ -17,6 +17,7 @@
 #include "bit_rows.cuh"
 #include "closure.hpp"
 #include "device_graph.hpp"
+#include "device_memory.hpp"
 #include "engine_api.hpp"
 #include "host_graph.hpp"
 #include "kernels.cuh"
@@ -60,7 +61,7 @@ struct DevArr {
     if (count <= n && p) return;
     release();
     if (count == 0) count = 1;
-    CK(cudaMalloc((void**)&p, count * sizeof(T)));
+    CK(device_malloc((void**)&p, count * sizeof(T)));
     n = count;
     t_live_bytes += (int64_t)(count * sizeof(T));
     t_peak_bytes = std::max(t_peak_bytes, t_live_bytes);
@@ -226,7 +227,8 @@ struct chsga_ctx {
   // traceback on bit rows: checkpoint states, a matrix of up to kKeepMatrix
   // bytes kept between calls, the matrix pointer and the walk's output
   chsga::PinnedArr<unsigned char> h_ckbits, h_walk;
-  chsga::DevArr<unsigned char> tb_mat, tb_walk;
+  chsga::KeptBuffer tb_mat;
+  chsga::DevArr<unsigned char> tb_walk;
   chsga::DevArr<unsigned char*> tb_ptr;
   chsga_profile prof{};
 };
@@ -1166,6 +1168,7 @@ void upload_graph(chsga_ctx& c, const chsga_graph_host& g) {
   c.bit_bufs.clear();
   c.row_tiles.clear();
   c.tops.clear();
+  c.tb_mat.drop();
   c.top_sel = nullptr;
   c.loaded = true;
 }
@@ -1490,7 +1493,9 @@ void traceback_rows(chsga_ctx& c, const char* read, uint32_t len, const chsga_tb
 
 // Largest matrix a context keeps between tracebacks (a 150 bp read's on the
 // 5 Mbp graph is 0.8 GB; mapping and unmapping it costs as much as the
-// read's row-steps). Larger ones live for one call.
+// read's row-steps). Larger ones live for one call. A kept matrix is freed
+// when another allocation needs the room (device_memory.hpp), when the context
+// loads another graph and when it closes.
 constexpr uint64_t kKeepMatrix = 1ull << 30;
 
 // Leaves the request meter as it was: what a context keeps between calls is
@@ -1518,26 +1523,22 @@ struct MeterHold {
 // A device buffer of one traceback: the context's kept one where it fits. The
 // request meter counts it while it lives, whichever it is.
 struct TbMatrix {
+  KeptBuffer* kept = nullptr;
   DevArr<unsigned char> own;
   unsigned char* p = nullptr;
   std::unique_ptr<MeterHold> hold;
   TbMatrix(chsga_ctx& c, uint64_t bytes) {
-    {
-      MeterPause pause;
-      if (bytes <= kKeepMatrix) {
-        c.tb_mat.alloc(bytes);
-        p = c.tb_mat.p;
-      } else {
-        c.tb_mat.release();  // a large matrix may need the room
-        own.alloc(bytes);
-        p = own.p;
-      }
+    if (bytes <= kKeepMatrix) {
+      hold = std::make_unique<MeterHold>(bytes);
+      CK(c.tb_mat.take(bytes, &p));
+      kept = &c.tb_mat;
+    } else {
+      own.alloc(bytes);
+      p = own.p;
     }
-    hold = std::make_unique<MeterHold>(bytes);
   }
   ~TbMatrix() {
-    MeterPause pause;
-    own.release();
+    if (kept) kept->put();
   }
   TbMatrix(const TbMatrix&) = delete;
   TbMatrix& operator=(const TbMatrix&) = delete;
@@ -1987,7 +1988,12 @@ void traceback_batched(chsga_ctx& parent, const char* const* reads, const uint32
         // always admit when nothing else holds a matrix, so the loop progresses
         if (used + need > budget && used > 0) break;
         void* p = nullptr;
-        CK(cudaMallocAsync(&p, need, c.st));
+        cudaError_t e = cudaMallocAsync(&p, need, c.st);
+        if (e == cudaErrorMemoryAllocation && free_kept_buffers()) {
+          cudaGetLastError();  // the failed attempt's
+          e = cudaMallocAsync(&p, need, c.st);
+        }
+        CK(e);
         hm[next] = static_cast<uint16_t*>(p);
         dev::k_set_ptr<<<1, 1, 0, c.st>>>(mats.p, next, hm[next]);
         used += need;
@@ -2768,7 +2774,7 @@ uint64_t device_free_bytes(const chsga_ctx& c) {
   CK(cudaSetDevice(c.device));
   size_t f = 0, t = 0;
   CK(cudaMemGetInfo(&f, &t));
-  return f;
+  return f + kept_bytes(c.device);  // those give way
 }
 
 std::unique_ptr<ScoreLane> make_score_lane(chsga_ctx& parent, uint32_t slots, uint32_t per_graph,
@@ -2823,6 +2829,7 @@ chsga_status chsga_open(const chsga_opts* opts, chsga_ctx** out) {
     CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
     size_t free_b = 0, total_b = 0;
     CK(cudaMemGetInfo(&free_b, &total_b));
+    free_b += kept_bytes(c->device);  // those give way
     c->cap = (opts && opts->hbm_cap_bytes) ? opts->hbm_cap_bytes : (uint64_t)(free_b * 0.85);
     *out = c.release();
   });

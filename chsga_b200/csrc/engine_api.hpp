@@ -28,7 +28,8 @@ uint64_t graph_string_vertices(const chsga_ctx& c);
 int32_t empty_read_score(const chsga_ctx& c);
 // Makes the context's device current on the calling thread.
 void bind_device(const chsga_ctx& c);
-// Free device memory now (cudaMemGetInfo) on the context's device.
+// Device memory an allocation on the context's device can get now: free
+// (cudaMemGetInfo) or held by idle kept buffers.
 uint64_t device_free_bytes(const chsga_ctx& c);
 // Device bytes the library allocated on this thread: meter_reset starts a
 // window (returns its base), meter_peak_since(base) is the window's peak

@@ -17,6 +17,7 @@
 #include <string>
 
 #include "common.hpp"
+#include "device_memory.hpp"
 #include "pch_gpu.hpp"
 
 namespace chsga {
@@ -158,7 +159,7 @@ struct Buf {
     if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
-    CKP(cudaMalloc((void**)&p, std::max<size_t>(n, 1) * sizeof(T)));
+    CKP(device_malloc((void**)&p, std::max<size_t>(n, 1) * sizeof(T)));
     cap = std::max<size_t>(n, 1);
   }
   void put(const std::vector<T>& v, cudaStream_t s) {

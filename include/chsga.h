@@ -364,7 +364,10 @@ chsga_status chsga_align_scores_noalloc(chsga_ctx* ctx, const char* const* reads
  * If len x N x 4 bytes fit under the byte cap the full score matrix stays in
  * HBM and the path is walked by score equality (src/traceback.hpp:483-586);
  * otherwise rows 0, k, 2k, ... are copied to pinned host memory and segments
- * are recomputed on the device before the walk. */
+ * are recomputed on the device before the walk.
+ * Between calls the context keeps a matrix of up to 1 GiB for the next one.
+ * It is freed when any allocation of the library on that device would fail
+ * without its room, when the context loads another graph and when it closes. */
 typedef struct {
   int64_t k;              /* checkpoint interval, default 500 (-k) */
   const char* dir;        /* if non-NULL, checkpoint rows are also written as

@@ -33,3 +33,55 @@ def test_peak_bytes_counts_the_whole_matrix(tmp_path):
         # the context's own buffers grow with the longest read so far
         if i:
             assert abs(p - repeated[n]) <= 1 << 20, (i, n, p, repeated[n])
+
+
+def _fill(leave):
+    """Takes the device's free memory but `leave` bytes."""
+    import torch
+    held = []
+    step = 1 << 36
+    while step >= 1 << 25:
+        while torch.cuda.mem_get_info(0)[0] >= leave + step:
+            held.append(torch.empty(step, dtype=torch.uint8, device="cuda"))
+        step >>= 1
+    return held
+
+
+@pytest.mark.parametrize("who", ["same context", "another context", "cost model"])
+def test_kept_matrix_gives_way_to_other_allocations(tmp_path, who):
+    """On a device that is full but for the matrix a context keeps after a
+    traceback, whatever else allocates gets that memory."""
+    import torch
+    g, _ = gen_graph(tmp_path, "g", backbone_len=100_000, seed=2)
+    read = g.gen_reads(1, 3, 9000).to_list()[0]
+    short = g.gen_reads(3, 4, 100).to_list()
+    want = cb.Context(0).load(g).align_scores(short)
+    ctx, other = cb.Context(0).load(g), cb.Context(0).load(g)
+    model = cb.CostModel(0, seed=1)
+    # kernels of the calls below are loaded before the device is full
+    for c in (ctx, other):
+        c.align_scores_batched(short, slots=32, row_bits=32, row_kernel=cb.ROW_DIRECT)
+        c.align_traceback(short[0])
+    model.predict([[1.0] * 8])
+    part = read[:7000]
+    part_score = ctx.align_scores([part])[0]
+    _, score, ck = ctx.align_traceback(read)  # about 0.8 GB
+    assert not ck
+    held = _fill(64 << 20)
+    try:
+        assert torch.cuda.mem_get_info(0)[0] < 100 << 20
+        if who == "same context":  # about 140 MB of score rows
+            got = ctx.align_scores_batched(short, slots=128, row_bits=32, row_kernel=cb.ROW_DIRECT)
+            assert list(got) == list(want)
+        elif who == "another context":  # a matrix of about 0.6 GB
+            assert other.align_traceback(part)[1] == part_score
+        else:  # about 400 MB of samples
+            assert model.predict([[1.0] * 8] * (10 << 20)).shape == (10 << 20, 2)
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    # and the context goes on
+    assert ctx.align_traceback(read)[1] == score
+    for c in (ctx, other):
+        c.close()
+    model.close()
