@@ -2747,6 +2747,9 @@ int32_t empty_read_score(const chsga_ctx& c) { return empty_score(c); }
 
 void bind_device(const chsga_ctx& c) { CK(cudaSetDevice(c.device)); }
 
+uint64_t kept_matrix_bytes(const chsga_ctx& c) { return c.tb_mat.idle_bytes(); }
+void drop_kept_matrix(chsga_ctx& c) { c.tb_mat.drop(); }
+
 int64_t meter_reset() {
   t_peak_bytes = t_live_bytes;
   return t_live_bytes;

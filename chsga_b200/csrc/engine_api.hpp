@@ -31,6 +31,10 @@ void bind_device(const chsga_ctx& c);
 // Device memory an allocation on the context's device can get now: free
 // (cudaMemGetInfo) or held by idle kept buffers.
 uint64_t device_free_bytes(const chsga_ctx& c);
+// Bytes of the matrix a context that runs no call keeps for its next
+// traceback, and giving it back. Any thread may ask.
+uint64_t kept_matrix_bytes(const chsga_ctx& c);
+void drop_kept_matrix(chsga_ctx& c);
 // Device bytes the library allocated on this thread: meter_reset starts a
 // window (returns its base), meter_peak_since(base) is the window's peak
 // above the base.

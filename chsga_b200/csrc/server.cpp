@@ -14,6 +14,8 @@
 // the graph, take requests in arrival order; the request at the head runs
 // once its projected device footprint fits what the running ones leave of
 // the budget (head-of-line: a large request is never overtaken forever).
+// Workers keep a matrix between requests; the ones of idle workers count
+// towards the budget and are freed where an admitted request needs the room.
 #include <algorithm>
 #include <chrono>
 #include <atomic>
@@ -145,6 +147,7 @@ struct chsga_server {
   uint64_t submitted = 0, finished = 0, failed = 0;
   uint64_t lane_running = 0;  // published to the lane, not yet harvested
   uint64_t tb_running = 0, tb_used = 0, tb_peak = 0;
+  std::vector<uint8_t> tb_busy;  // by worker: runs a request
   uint64_t cells = 0;
   int64_t first_submit = 0, last_done = 0;
   std::vector<int64_t> lat_score, lat_tb;
@@ -314,11 +317,33 @@ struct chsga_server {
     }
   }
 
+  // The idle workers whose kept matrices have to go so that they and the
+  // running requests' footprints fit the budget (under mu). A worker never
+  // keeps more than the footprint of the request it runs (tb_loop).
+  std::vector<chsga_ctx*> kept_to_drop() {
+    std::vector<std::pair<uint64_t, chsga_ctx*>> idle;
+    uint64_t held = tb_used;
+    for (size_t v = 0; v < tb_ctx.size(); ++v)
+      if (!tb_busy[v]) {
+        idle.push_back({kept_matrix_bytes(*tb_ctx[v]), tb_ctx[v]});
+        held += idle.back().first;
+      }
+    std::sort(idle.begin(), idle.end());
+    std::vector<chsga_ctx*> drop;
+    while (held > o.hbm_budget_bytes && !idle.empty()) {
+      held -= idle.back().first;
+      drop.push_back(idle.back().second);
+      idle.pop_back();
+    }
+    return drop;
+  }
+
   void tb_loop(size_t w) {
     chsga_ctx* c = tb_ctx[w];
     const uint64_t budget = o.hbm_budget_bytes;
     while (true) {
       Request q;
+      std::vector<chsga_ctx*> drop;
       {
         std::unique_lock<std::mutex> lk(mu);
         cv_tb.wait(lk, [&] {
@@ -333,7 +358,13 @@ struct chsga_server {
         tb_used += q.footprint;
         tb_peak = std::max(tb_peak, tb_used);
         ++tb_running;
+        tb_busy[w] = 1;
+        drop = kept_to_drop();
       }
+      // freed before this request allocates (a worker that started since then
+      // has its own matrix in use, within its request's footprint)
+      for (chsga_ctx* d : drop) drop_kept_matrix(*d);
+      if (kept_matrix_bytes(*c) > q.footprint) drop_kept_matrix(*c);
       chsga_server_result r{};
       r.ticket = q.ticket;
       r.read_len = (uint32_t)q.read.size();
@@ -348,10 +379,12 @@ struct chsga_server {
       r.peak_bytes = meter_peak_since(base);
       r.score = r.tb.score;
       r.done_ns = now_ns();
+      if (kept_matrix_bytes(*c) > q.footprint) drop_kept_matrix(*c);  // a footprint predicted too small
       std::lock_guard<std::mutex> lk(mu);
       if (r.status != CHSGA_OK && err.empty()) err = chsga_last_error(c);
       tb_used -= q.footprint;
       --tb_running;
+      tb_busy[w] = 0;
       finish(std::move(r));
       cv_tb.notify_all();
     }
@@ -432,6 +465,7 @@ chsga_status chsga_server_open(chsga_ctx* ctx, const chsga_server_opts* opts, ch
       for (auto* c : s->tb_ctx) chsga_close(c);
       throw;
     }
+    s->tb_busy.assign(o.tb_workers, 0);
     chsga_server* p = s.get();
     p->engine = std::thread([p] { p->engine_loop(); });
     for (uint32_t w = 0; w < o.tb_workers; ++w) p->workers.emplace_back([p, w] { p->tb_loop(w); });

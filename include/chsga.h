@@ -504,7 +504,8 @@ typedef struct {
   uint32_t queue_capacity;   /* score reads queued or running on the device (power of 2); 0 = 4096 */
   uint32_t tb_workers;       /* traceback requests running at once; 0 = 2 */
   uint64_t arena_bytes;      /* device bytes for the bases of queued score reads; 0 = 64 MiB */
-  uint64_t hbm_budget_bytes; /* device bytes running traceback requests may hold; 0 = 50% of free */
+  uint64_t hbm_budget_bytes; /* device bytes running traceback requests may hold, the matrices
+                                idle workers keep included; 0 = 50% of free */
   int64_t tb_k;              /* checkpoint interval of traceback requests; 0 = 500 */
   uint64_t tb_cap_bytes;     /* full-matrix byte cap of a traceback request; 0 = the context's */
   uint32_t row_bits;         /* score rows: 16 (reads <= 65000 bases) or 32; 0 = 16 */

@@ -85,3 +85,29 @@ def test_kept_matrix_gives_way_to_other_allocations(tmp_path, who):
     for c in (ctx, other):
         c.close()
     model.close()
+
+
+def test_workers_keep_no_more_than_the_budget(tmp_path):
+    """hbm_budget_bytes bounds what the traceback workers hold between and
+    during requests, whichever worker each request falls to: here it has room
+    for one request and there are four workers."""
+    import torch
+    g, _ = gen_graph(tmp_path, "g", backbone_len=100_000, seed=2)
+    read = g.gen_reads(1, 3, 9000).to_list()[0]
+    ctx = cb.Context(0).load(g)
+    need = 2 * g.stats()["num_chars"] * 9100
+    srv = cb.Server(ctx, tb_workers=4, slots=16, hbm_budget_bytes=need)
+    for _ in range(4):
+        srv.submit(read[:50], cb.REQ_TRACEBACK)
+    srv.collect()
+    before = torch.cuda.mem_get_info(0)[0]
+    scores = set()
+    for _ in range(24):
+        t = srv.submit(read, cb.REQ_TRACEBACK)
+        r = srv.collect()[t]
+        assert r["status"] == cb.OK and not r["checkpointed"] and r["projected_bytes"] <= need
+        scores.add(r["score"])
+        assert before - torch.cuda.mem_get_info(0)[0] <= need + (200 << 20)
+    assert len(scores) == 1
+    srv.close()
+    ctx.close()
