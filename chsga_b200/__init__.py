@@ -225,6 +225,7 @@ _sig("chsga_align_traceback_batched", C.c_int32, vp, C.POINTER(C.c_char_p), u32p
      C.POINTER(TbOpts), C.c_uint32, C.POINTER(TbResult))
 _sig("chsga_ops_to_cigar", C.c_uint64, C.POINTER(OpT), C.c_uint64, C.c_char_p, C.c_uint64)
 _sig("chsga_get_profile", C.c_int32, vp, C.POINTER(ProfileT))
+_sig("chsga_last_row_kernel", C.c_char_p, vp)
 _sig("chsga_get_read_times", C.c_int32, vp, u64p, u64p, C.c_uint32)
 _sig("chsga_selftest_wait", C.c_int32, vp, C.c_uint32)
 _sig("chsga_selftest_grid_wait", C.c_int32, vp, C.c_uint32)
@@ -544,6 +545,10 @@ class Context:
         """Runs a bounded device wait that cannot succeed (chsga_selftest_wait):
         raises ChsgaError with ERR_TIMEOUT."""
         self._ck(_lib.chsga_selftest_wait(self._h, polls))
+
+    def last_row_kernel(self) -> str:
+        """Row kernel of the row-step launched last (chsga_last_row_kernel)."""
+        return _lib.chsga_last_row_kernel(self._h).decode()
 
     def profile(self) -> dict:
         p = ProfileT()

@@ -143,6 +143,11 @@ struct BitBufs {
 // tiled, for comparisons).
 enum class RowKernel { Auto, Direct, Tiled, Dpx, Stream, Delta };
 
+// Form of the bit-row kernels at 32 to 128 slots of 16-bit scores (CHSGA_BIT_ROWS
+// = words | sliced | sliced4, for comparisons and tests; Auto: bits_sliced and
+// bit_step).
+enum class BitForm { Auto, Words, Sliced, Sliced4 };
+
 struct RowTileDev {
   DevArr<int4> rec;
   DevArr<uint32_t> desc;
@@ -199,6 +204,8 @@ struct chsga_ctx {
   bool sweeps = false;                     // this call chose a level grouping: level sweeps
   int num_sms = 148;
   chsga::RowKernel row_kernel = chsga::RowKernel::Auto;
+  chsga::BitForm bit_form = chsga::BitForm::Auto;
+  const char* row_name = "";  // row kernel of the row-step launched last
   // launch mode of the one-read path (chsga_align_scores): CHSGA_LAUNCH_*, or
   // kPlainAuto (see there)
   uint32_t plain_mode = chsga::kPlainAuto;
@@ -549,6 +556,7 @@ void row_step(chsga_ctx& c, SlotBufs& b, const ST* D, ST* T, cudaStream_t s,
     if (c.g->t1.ntiles && c.row_kernel == RowKernel::Auto) {
       chain_launch(c, dev::k_row_t1<DEFER>, (c.g->t1.ntiles + dev::kT1Warps - 1) / dev::kT1Warps,
                    dev::kT1Warps * 32, 0, s, c.g->gp, c.g->t1, D, T, BVc, FL, b.word.p, b.best.p, b.ctl.p);
+      c.row_name = "k_row_t1";
       done = true;
     }
   }
@@ -564,6 +572,7 @@ void row_step(chsga_ctx& c, SlotBufs& b, const ST* D, ST* T, cudaStream_t s,
       const uint32_t grid = c.delta_grid ? std::min(all, c.delta_grid) : all;
       chain_launch(c, dev::k_row_delta, grid, tpb, dev::delta_smem_bytes(), s, c.g->gp, D, T, BVc, FL, b.word.p,
                    b.best.p, b.ctl.p, (const uint32_t*)c.g->gd.delta_order.p, runs);
+      c.row_name = "k_row_delta";
       done = true;
       delta_rows = true;
     }
@@ -577,12 +586,14 @@ void row_step(chsga_ctx& c, SlotBufs& b, const ST* D, ST* T, cudaStream_t s,
           constexpr unsigned tpb = dev::kStreamWarps * 32;
           chain_launch(c, dev::k_row_stream<R, DEFER>, nblocks(runs * 32, tpb), tpb, dev::stream_smem_bytes(R), s,
                        c.g->gp, D, T, BVc, FL, b.word.p, b.best.p, b.ctl.p);
+          c.row_name = "k_row_stream";
           done = true;
         }
       }
       if (!done) {
         chain_launch(c, dev::k_row_dpx<R, DEFER>, nblocks((uint64_t)L.S * dev::Pairs<R>::G), 256, 0, s,
                      c.g->gp, D, T, BVc, FL, b.word.p, b.best.p, b.ctl.p);
+        c.row_name = "k_row_dpx";
         done = true;
       }
     }
@@ -593,13 +604,16 @@ void row_step(chsga_ctx& c, SlotBufs& b, const ST* D, ST* T, cudaStream_t s,
         chain_launch(c, dev::k_row_tiled<R, DEFER, ST>, c.num_sms, dev::kRowThreads,
                      dev::row_smem_bytes(dev::row_slot_bytes(*rt), rt->nslots, R), s, c.g->gp, *rt, D, T, BVc,
                      FL, b.word.p, b.best.p, b.ctl.p);
+        c.row_name = "k_row_tiled";
         done = true;
       }
     }
   }
-  if (!done)
+  if (!done) {
     chain_launch(c, dev::k_row_direct<R, DEFER, ST>, nblocks((uint64_t)L.S * G), 256, 0, s, c.g->gp, D, T,
                  BVc, FL, b.word.p, b.best.p, b.ctl.p);
+    c.row_name = "k_row_direct";
+  }
   if (ev) CK(cudaEventRecord(ev->e[1], s));
   const uint32_t fl = top.h.first_level;
   for (uint32_t l = 0; l < fl; ++l) {
@@ -746,6 +760,7 @@ void launch_persist(chsga_ctx& c, SlotBufs& b, uint32_t grid, uint32_t steps, cu
   cfg.attrs = at;
   cfg.numAttrs = 1;
   CK(cudaLaunchKernelEx(&cfg, dev::k_persist<R>, a));
+  c.row_name = "k_persist";
 }
 
 // ---- bit-row engine (bit_rows.cuh) --------------------------------------------
@@ -765,7 +780,9 @@ bool bits_apply(const chsga_ctx& c) {
 // against 14.6; on 22,000 vertices 28.7 against 22.0 and 19.0 against 18.4).
 template <int R, typename ST>
 bool bits_sliced(const chsga_ctx& c) {
-  return R >= 32 && std::is_same_v<ST, uint16_t> && c.g->L.max_len <= 512 && (uint64_t)c.g->L.S * R > 400'000;
+  if (R < 32 || !std::is_same_v<ST, uint16_t> || c.g->L.max_len > 512) return false;
+  if (c.bit_form != BitForm::Auto) return c.bit_form != BitForm::Words;
+  return (uint64_t)c.g->L.S * R > 400'000;
 }
 
 template <int R, typename ST>
@@ -826,6 +843,7 @@ uint32_t resident_blocks(chsga_ctx& c, const void* k, int threads) {
 template <int R, typename ST>
 void launch_words(chsga_ctx& c, const dev::BitArgs& a, cudaStream_t s) {
   const uint32_t S = c.g->L.S;
+  c.row_name = std::is_same_v<ST, uint16_t> ? "k_row_words" : "k_row_words<int>";
   auto launch = [&](auto kern, uint32_t threads, uint32_t P) {
     const uint32_t VB = threads / R, items = S + c.g->bg.heavy * (P - 1);
     chain_launch(c, kern, std::min((items + VB - 1) / VB + 1, resident_blocks(c, (const void*)kern, (int)threads)),
@@ -860,10 +878,15 @@ void bit_step(chsga_ctx& c, BitBufs& b, int par, cudaStream_t s) {
       using S1 = dev::SlicedShared<R, 1>;
       // four items a lane where that gives every warp of the device work
       a.g.by_len = c.g->gd.cl_by_len[R == 128 ? 0 : R == 64 ? 1 : 2].p;
-      if (S >= (uint32_t)S4::VB * 16u * (uint32_t)c.num_sms)
+      const bool four = c.bit_form == BitForm::Auto ? S >= (uint32_t)S4::VB * 16u * (uint32_t)c.num_sms
+                                                    : c.bit_form == BitForm::Sliced4;
+      if (four)
         launch(dev::k_row_sliced<R, 4>, S4::VB * S4::NW);
       else
         launch(dev::k_row_sliced<R, 1>, S1::VB * S1::NW);
+      c.row_name = R == 32 ? (four ? "k_row_sliced<32,4>" : "k_row_sliced<32,1>")
+                   : R == 64 ? (four ? "k_row_sliced<64,4>" : "k_row_sliced<64,1>")
+                             : (four ? "k_row_sliced<128,4>" : "k_row_sliced<128,1>");
       return;
     }
   }
@@ -891,6 +914,7 @@ void mat_step(chsga_ctx& c, BitBufs& b, unsigned char* const* mats, int par, cud
   dev::BitArgs a = bit_args(c, b, par);
   a.mats = mats;
   a.pitch = bit_row_bytes(c);
+  c.row_name = "k_row_words";
   const uint32_t S = c.g->L.S;
   auto launch = [&](auto kern, uint32_t threads) {
     const uint32_t res = std::max(1u, resident_blocks(c, (const void*)kern, (int)threads) / H);
@@ -2178,6 +2202,7 @@ void noalloc_row_step(chsga_ctx& c, const NoallocBufs& b, const uint16_t* D, uin
   constexpr int G = Lanes<1>::G;
   dev::k_row_direct<1, true, uint16_t><<<nblocks((uint64_t)L.S * G), 256, 0, s>>>(
       c.g->gp, D, T, b.BV, b.FL, b.word, b.best, b.ctl);
+  c.row_name = "k_row_direct";
   const uint32_t fl = top.h.first_level;
   for (uint32_t l = 0; l < fl; ++l) {
     if (L.lvl_up_edges[l] == 0) continue;
@@ -2706,6 +2731,7 @@ chsga_ctx* fork_context(chsga_ctx& p) {
   c->cap = p.cap;
   c->num_sms = p.num_sms;
   c->row_kernel = p.row_kernel;
+  c->bit_form = p.bit_form;
   c->plain_mode = p.plain_mode;
   c->pdl = p.pdl;
   c->pull_coop = p.pull_coop;
@@ -2824,6 +2850,11 @@ chsga_status chsga_open(const chsga_opts* opts, chsga_ctx** out) {
       if (std::string(pl) == "stream") c->plain_mode = CHSGA_LAUNCH_STREAM;
       if (std::string(pl) == "graphs") c->plain_mode = CHSGA_LAUNCH_GRAPHS;
       if (std::string(pl) == "persistent") c->plain_mode = CHSGA_LAUNCH_PERSISTENT;
+    }
+    if (const char* bf = std::getenv("CHSGA_BIT_ROWS")) {
+      if (std::string(bf) == "words") c->bit_form = BitForm::Words;
+      if (std::string(bf) == "sliced") c->bit_form = BitForm::Sliced;
+      if (std::string(bf) == "sliced4") c->bit_form = BitForm::Sliced4;
     }
     if (const char* pd = std::getenv("CHSGA_PDL")) c->pdl = std::string(pd) != "0";
     if (const char* pc = std::getenv("CHSGA_PULL_COOP")) c->pull_coop = std::string(pc) == "1";
@@ -3105,6 +3136,8 @@ chsga_status chsga_selftest_grid_wait(chsga_ctx* c, uint32_t limit_us) {
             "the grid barrier wait did not give up (abort word " + std::to_string(gb.abort) + ")");
   });
 }
+
+const char* chsga_last_row_kernel(chsga_ctx* c) { return c ? c->row_name : ""; }
 
 chsga_status chsga_get_profile(chsga_ctx* c, chsga_profile* out) {
   return guarded_ctx(c, [&] {

@@ -432,6 +432,11 @@ typedef struct {
   uint64_t launch_mode;   /* how the row-steps ran: CHSGA_LAUNCH_* */
 } chsga_profile;
 chsga_status chsga_get_profile(chsga_ctx* ctx, chsga_profile* out);
+/* Row kernel of the row-step the context launched last: k_row_sliced<slots,items
+ * a lane>, k_row_words or k_row_words<int> (bit rows), else k_row_t1, k_row_delta,
+ * k_row_stream, k_row_dpx, k_row_tiled, k_row_direct or k_persist; empty before
+ * the first. A server's row-steps run on contexts of its own. */
+const char* chsga_last_row_kernel(chsga_ctx* ctx);
 
 /* Per-read admission and completion times of the last score call (device
  * global timer, ns), in the order of the non-empty reads passed in. No
