@@ -2418,9 +2418,10 @@ void scores_batched(chsga_ctx& c, const char* const* reads, const uint32_t* lens
 
 // Coordinate search over the batched engine's knobs on a read sample:
 // slots, then steps per graph, then the row kernel, then the level
-// grouping, each stage keeping the fastest by device time. With a cost
-// model, the slot stage only runs the candidates of highest predicted
-// throughput. Every run must return the first run's scores.
+// grouping (of the fastest row kernel with level sweeps), each stage keeping
+// the fastest by device time. With a cost model, the slot stage only runs the
+// candidates of highest predicted throughput. Every run must return the first
+// run's scores.
 chsga_batch_opts autotune(chsga_ctx& c, const char* const* reads, const uint32_t* lens, uint32_t n,
                           const chsga_tune_opts* o, std::vector<chsga_tune_trial>& trials) {
   const uint32_t repeats = o && o->repeats ? o->repeats : 2;
@@ -2488,22 +2489,31 @@ chsga_batch_opts autotune(chsga_ctx& c, const char* const* reads, const uint32_t
     const double g = run(b, 0);
     if (g > best_g) best_g = g, best = b;
   }
-  // row kernel
+  // row kernel: the ones AUTO does not run at these slots (bit rows where the
+  // graph has closure lists; else DELTA at 128 slots, STREAM at 64, DPX below)
   cur = best;
-  for (uint32_t rk : {(uint32_t)CHSGA_ROW_STREAM, (uint32_t)CHSGA_ROW_DPX, (uint32_t)CHSGA_ROW_DIRECT,
-                      (uint32_t)CHSGA_ROW_TILED}) {
+  const bool bits = bits_apply(c);
+  const uint32_t auto_rk = bits               ? (uint32_t)CHSGA_ROW_AUTO
+                           : cur.slots == 128 ? (uint32_t)CHSGA_ROW_DELTA
+                           : cur.slots == 64  ? (uint32_t)CHSGA_ROW_STREAM
+                                              : (uint32_t)CHSGA_ROW_DPX;
+  chsga_batch_opts sweeps = best;  // the fastest that runs the level sweeps
+  double sweeps_g = bits ? -1 : best_g;
+  for (uint32_t rk : {(uint32_t)CHSGA_ROW_DELTA, (uint32_t)CHSGA_ROW_STREAM, (uint32_t)CHSGA_ROW_DPX,
+                      (uint32_t)CHSGA_ROW_DIRECT, (uint32_t)CHSGA_ROW_TILED}) {
+    if (rk == auto_rk) continue;
     if (rk == CHSGA_ROW_TILED && cur.slots < 32) continue;
-    if (rk == CHSGA_ROW_DPX && cur.slots < 64) continue;        // AUTO already is DPX there
-    if (rk == CHSGA_ROW_STREAM && cur.slots != 128) continue;   // AUTO is STREAM at 64, DELTA at 128
+    if (rk == CHSGA_ROW_STREAM && cur.slots < 64) continue;
+    if (rk == CHSGA_ROW_DELTA && cur.slots != 128) continue;
     chsga_batch_opts b = cur;
     b.row_kernel = rk;
     const double g = run(b, 0);
+    if (g > sweeps_g) sweeps_g = g, sweeps = b;
     if (g > best_g) best_g = g, best = b;
   }
-  // level grouping
-  cur = best;
+  // level grouping, which only the sweeps have
   for (uint32_t K : {kTopMaxVertices, 3000u}) {
-    chsga_batch_opts b = cur;
+    chsga_batch_opts b = sweeps;
     b.top_vertices = K;
     const double g = run(b, 0);
     if (g > best_g) best_g = g, best = b;
