@@ -87,6 +87,77 @@ struct BitArgs {
   size_t pitch;
 };
 
+// ---------------------------------------------------------------------------
+// k_closure_arrays, k_by_len: the arrays of the bit-row kernels from the lists
+// of build_closure, once a graph is loaded (they took a third of the list
+// build's time on the host and twice the bytes to upload).
+//   ent    in {source, weight}; out for 16-bit rows: {source, weight for M |
+//          weight for F << 16}, 0xFFFF = no such entry (or a weight no 16-bit
+//          score can win with)
+//   wrec   in HostClosure::order; out {first bit word, length | key << 29,
+//          first entry, entries}
+//   wsv    {string vertex, first char} by position; pos the position by vertex
+//   went   {source | class << 30 (0 both, 1 M only, 2 F only), weight}
+//   lab    per bit word the label planes of its 32 chain chars (bit k of word j
+//          = char first + 1 + 32 j + k): {code bit 0, code bit 1, special, 0}
+// Eight lanes a position.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) k_closure_arrays(uint32_t S, uint32_t heavy, const uint4* __restrict__ rec,
+                                                        uint2* ent, uint4* wrec, uint2* wsv, uint32_t* pos,
+                                                        uint2* went, uint4* lab, const uint32_t* __restrict__ lab4) {
+  const uint32_t t = blockIdx.x * 256 + threadIdx.x, i = t / 8, l = t % 8;
+  const bool live = i < S;
+  const uint4 in = live ? wrec[i] : make_uint4(0, 0, 0, 0);
+  __syncwarp();  // all lanes of a position have read its record
+  if (!live) return;
+  const uint4 r = rec[in.y];
+  const uint32_t nb = r.w & 255u, nm = (r.w >> 8) & 255u, n = nb + nm + (r.w >> 16), len = r.y & 0x1FFFFFFFu;
+  if (l == 0) {
+    wrec[i] = make_uint4(in.x, r.y, in.z, n);
+    wsv[i] = make_uint2(in.y, r.x);
+    pos[in.y] = i;
+  }
+  for (uint32_t k = l; k < n; k += 8) {
+    const uint2 e = ent[r.z + k];
+    const uint32_t cls = k < nb ? 0u : k < nb + nm ? 1u : 2u, w = min(e.y, 0xFFFEu);
+    went[in.z + (size_t)(i < heavy ? 1 : 32) * k] = make_uint2(e.x | cls << 30, e.y);
+    ent[r.z + k] = make_uint2(e.x, (cls == 2 ? 0xFFFFu : w) | (cls == 0 ? w + 1 : cls == 2 ? w : 0xFFFFu) << 16);
+  }
+  for (uint32_t j = l; j < (len + 30) / 32; j += 8) {
+    const uint32_t c0 = r.x + 1 + 32 * j, m = min(32u, len - 1 - 32 * j);
+    uint4 p = make_uint4(0, 0, 0, 0);
+    for (uint32_t k = 0; k < m; ++k) {
+      const uint32_t key = lab4[(c0 + k) >> 3] >> ((c0 + k) & 7u) * 4u;
+      p.x |= (key & 1u) << k;
+      p.y |= ((key >> 1) & 1u) << k;
+      p.z |= ((key >> 2) & 1u) << k;
+    }
+    lab[in.x + j] = p;
+  }
+}
+
+// Order of the vertices inside every window of 32, 64 and 128 by falling label
+// length (local indexes), ties in their order: a thread counts the vertices
+// before its own. Blocks of 128 threads.
+__global__ void __launch_bounds__(128) k_by_len(uint32_t S, const uint32_t* __restrict__ sv_off, uint8_t* by32,
+                                                uint8_t* by64, uint8_t* by128) {
+  __shared__ uint32_t s_len[128];
+  const uint32_t t = threadIdx.x, base = blockIdx.x * 128, s = base + t;
+  const uint32_t len = s < S ? sv_off[s + 1] - sv_off[s] : 0;  // none has length 0: past the end goes last
+  s_len[t] = len;
+  __syncthreads();
+  if (s >= S) return;
+  auto place = [&](uint32_t W, uint8_t* out) {
+    const uint32_t w0 = t / W * W;
+    uint32_t r = 0;
+    for (uint32_t u = w0; u < w0 + W; ++u) r += s_len[u] > len || (s_len[u] == len && u < t) ? 1u : 0u;
+    out[base + w0 + r] = (uint8_t)(t - w0);
+  };
+  place(32, by32);
+  place(64, by64);
+  place(128, by128);
+}
+
 // What a row-step has to do, the same in every block.
 struct HeadFlags {
   bool work, end, drain, init, wide;

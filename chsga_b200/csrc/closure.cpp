@@ -3,7 +3,7 @@
 
 #include <algorithm>
 #include <atomic>
-#include <numeric>
+#include <vector>
 
 namespace chsga {
 
@@ -11,289 +11,291 @@ namespace {
 
 constexpr int64_t kMaxWeight = 1 << 30;  // sums stay below int32 with any score
 
-using List = std::vector<EdgeW>;  // {source vertex, weight}
+// An entry as one number (source vertex above, weight below), so that lists
+// sort by source, then weight.
+using Entry = uint64_t;
+using List = std::vector<Entry>;
+
+Entry entry(uint32_t src, int32_t w) { return (Entry)src << 32 | (uint32_t)w; }
+uint32_t src_of(Entry e) { return (uint32_t)(e >> 32); }
+int32_t w_of(Entry e) { return (int32_t)(uint32_t)e; }
+Entry heavier(Entry e, int32_t by) {
+  return entry(src_of(e), (int32_t)std::min<int64_t>((int64_t)w_of(e) + by, kMaxWeight));
+}
 
 // One entry per source, the smallest weight; `self` (a one-char vertex's own
 // score, which a positive weight cannot lower) is dropped.
-void tidy(List& l, int32_t self) {
-  std::sort(l.begin(), l.end(), [](const EdgeW& a, const EdgeW& b) {
-    return a.src != b.src ? a.src < b.src : a.w < b.w;
-  });
+void tidy(List& l, int64_t self) {
+  std::sort(l.begin(), l.end());
   size_t k = 0;
-  for (const EdgeW& e : l) {
-    if (e.src == self || (k && l[k - 1].src == e.src)) continue;
+  for (const Entry e : l) {
+    if (src_of(e) == self || (k && src_of(l[k - 1]) == src_of(e))) continue;
     l[k++] = e;
   }
   l.resize(k);
 }
 
-int32_t add_w(int32_t a, int32_t b) { return (int32_t)std::min<int64_t>((int64_t)a + b, kMaxWeight); }
+// out = the union of two tidy lists, b's weights raised by `by`.
+void merge(const List& a, const Entry* b, const Entry* b_end, int32_t by, List& out) {
+  out.clear();
+  auto i = a.begin();
+  while (i != a.end() || b != b_end) {
+    if (b == b_end || (i != a.end() && src_of(*i) < src_of(*b))) {
+      out.push_back(*i++);
+    } else if (i == a.end() || src_of(*b) < src_of(*i)) {
+      out.push_back(heavier(*b++, by));
+    } else {
+      out.push_back(std::min(*i++, heavier(*b, by)));
+      ++b;
+    }
+  }
+}
+
+// f(i) for i in [0, n), on all threads when there are many.
+template <typename F>
+void parallel(int64_t n, bool many, F&& f) {
+#pragma omp parallel for schedule(dynamic) if (many)
+  for (int64_t i = 0; i < n; ++i) f(i);
+}
 
 }  // namespace
 
 HostClosure build_closure(const HostLayout& L) {
   HostClosure c;
   const uint32_t S = L.S;
-  std::atomic<bool> too_long{false};
+  const bool many = S > 2048;
+  std::atomic<bool> refused{false};
+  auto single = [&](uint32_t d) { return L.dv_len[d] == 1; };
   // expanded lists of one-char vertices that are sources, by hierarchy
   // position: after the upward sweep (what upward edges read) and final
-  // (what downward edges read)
+  // (what downward edges read). An even source index of an edge names the
+  // only score of a one-char vertex.
   std::vector<uint8_t> up_src(S, 0), dn_src(S, 0);
-  for (const EdgeW& e : L.up_in)
-    if (!(e.src & 1)) up_src[e.src >> 1] = 1;
-  for (const EdgeW& e : L.dn_in)
-    if (!(e.src & 1)) dn_src[e.src >> 1] = 1;
-  for (uint32_t d = 0; d < S; ++d)  // an even index names the only score of a one-char vertex
-    if (L.dv_len[d] != 1) up_src[d] = dn_src[d] = 0;
+  auto mark = [&](const std::vector<EdgeW>& in, std::vector<uint8_t>& src) {
+#pragma omp parallel for schedule(static) if (many)
+    for (int64_t k = 0; k < (int64_t)in.size(); ++k)
+      if (!(in[k].src & 1) && single(in[k].src >> 1)) __atomic_store_n(&src[in[k].src >> 1], 1, __ATOMIC_RELAXED);
+  };
+  mark(L.up_in, up_src);
+  mark(L.dn_in, dn_src);
   std::vector<uint32_t> slot(S, 0);
   std::vector<List> ups(1), fins(1);
-  auto single = [&](uint32_t d) { return L.dv_len[d] == 1; };
+  // the source of an edge and, through a one-char source, that one's sources
+  auto take = [&](const EdgeW& e, bool through, const std::vector<List>& lists,
+                  const std::vector<uint32_t>& at, List& l) {
+    const uint32_t x = (uint32_t)e.src >> 1;
+    l.push_back(entry(L.dv_s[x], e.w));
+    if (through)
+      for (const Entry y : lists[at[x]]) l.push_back(heavier(y, e.w));
+  };
   auto expand_up = [&](uint32_t d, List& l) {
-    for (uint32_t k = L.up_off[d]; k < L.up_off[d + 1]; ++k) {
+    for (uint32_t k = L.up_off[d]; k < L.up_off[d + 1] && !refused; ++k) {
       const uint32_t x = (uint32_t)L.up_in[k].src >> 1;
-      l.push_back({(int32_t)L.dv_s[x], L.up_in[k].w});
-      if (single(x) && L.up_off[x + 1] > L.up_off[x])
-        for (const EdgeW& e : ups[slot[x]]) l.push_back({e.src, add_w(e.w, L.up_in[k].w)});
+      take(L.up_in[k], single(x) && L.up_off[x + 1] > L.up_off[x], ups, slot, l);
     }
   };
   auto finish = [&](uint32_t d, List& l) {
-    tidy(l, single(d) ? (int32_t)L.dv_s[d] : -1);
-    if (l.size() > kClosureMaxList) too_long = true;
+    tidy(l, single(d) ? (int64_t)L.dv_s[d] : -1);
+    if (l.size() > kClosureMaxList) refused = true;
   };
-  // one-char vertices with upward in-edges, by rising level
-  for (uint32_t l = 0; l < L.levels && !too_long; ++l) {
-    const uint32_t lo = L.lvl_off[l], hi = L.lvl_off[l + 1];
-    const size_t first = ups.size();
+  // the one-char vertices of a level that `want` picks, in pieces of 64
+  auto by_level = [&](uint32_t level, std::vector<List>& lists, std::vector<uint32_t>& at, auto&& want, auto&& make) {
+    const size_t first = lists.size();
     std::vector<uint32_t> todo;
-    for (uint32_t d = lo; d < hi; ++d)
-      if (single(d) && (up_src[d] || dn_src[d]) && L.up_off[d + 1] > L.up_off[d]) {
-        slot[d] = (uint32_t)(first + todo.size());
+    for (uint32_t d = L.lvl_off[level]; d < L.lvl_off[level + 1]; ++d)
+      if (want(d)) {
+        at[d] = (uint32_t)(first + todo.size());
         todo.push_back(d);
       }
-    ups.resize(first + todo.size());
-#pragma omp parallel for schedule(dynamic, 64) if (todo.size() > 256)
-    for (int64_t i = 0; i < (int64_t)todo.size(); ++i) {
-      if (too_long) continue;
-      expand_up(todo[i], ups[first + i]);
-      finish(todo[i], ups[first + i]);
-    }
-  }
-  if (too_long) return HostClosure{};
+    lists.resize(first + todo.size());
+    parallel(((int64_t)todo.size() + 63) / 64, todo.size() > 256, [&](int64_t q) {
+      for (size_t i = 64 * (size_t)q; i < std::min(todo.size(), 64 * (size_t)q + 64) && !refused; ++i) {
+        make(todo[i], lists[first + i]);
+        finish(todo[i], lists[first + i]);
+      }
+    });
+  };
+  // one-char vertices with upward in-edges, by rising level
+  for (uint32_t l = 0; l < L.levels && !refused; ++l)
+    by_level(l, ups, slot,
+             [&](uint32_t d) { return single(d) && (up_src[d] || dn_src[d]) && L.up_off[d + 1] > L.up_off[d]; },
+             expand_up);
+  if (refused) return HostClosure{};
   // final lists of one-char sources of downward edges, by falling level
   std::vector<uint32_t> fslot(S, 0);
   auto expand_final = [&](uint32_t d, List& l) {
     expand_up(d, l);
-    for (uint32_t k = L.dn_off[d]; k < L.dn_off[d + 1]; ++k) {
-      const uint32_t x = (uint32_t)L.dn_in[k].src >> 1;
-      l.push_back({(int32_t)L.dv_s[x], L.dn_in[k].w});
-      if (single(x))
-        for (const EdgeW& e : fins[fslot[x]]) l.push_back({e.src, add_w(e.w, L.dn_in[k].w)});
-    }
-    finish(d, l);
+    for (uint32_t k = L.dn_off[d]; k < L.dn_off[d + 1] && !refused; ++k)
+      take(L.dn_in[k], single((uint32_t)L.dn_in[k].src >> 1), fins, fslot, l);
   };
-  for (uint32_t l = L.levels; l-- > 0 && !too_long;) {
-    const size_t first = fins.size();
-    std::vector<uint32_t> todo;
-    for (uint32_t d = L.lvl_off[l]; d < L.lvl_off[l + 1]; ++d)
-      if (dn_src[d]) {
-        fslot[d] = (uint32_t)(first + todo.size());
-        todo.push_back(d);
-      }
-    fins.resize(first + todo.size());
-#pragma omp parallel for schedule(dynamic, 64) if (todo.size() > 256)
-    for (int64_t i = 0; i < (int64_t)todo.size(); ++i)
-      if (!too_long) expand_final(todo[i], fins[first + i]);
-  }
-  if (too_long) return HostClosure{};
-  // A(v) of every vertex, by string vertex
-  constexpr int64_t kChunk = 4096;
-  const int64_t chunks = ((int64_t)S + kChunk - 1) / kChunk;
-  std::vector<uint32_t> a_off((size_t)S + 1, 0);
+  for (uint32_t l = L.levels; l-- > 0 && !refused;)
+    by_level(l, fins, fslot, [&](uint32_t d) { return dn_src[d] != 0; }, expand_final);
+  if (refused) return HostClosure{};
+  // A(v) of every vertex, in chunks of string vertices
+  // log2 of a chunk: some hundred chunks, whose lists stay below the size at
+  // which the allocator maps and unmaps memory for each
+  uint32_t shift = 6;
+  while (shift < 10 && (S >> shift) > 256) ++shift;
+  const int64_t chunks = ((int64_t)S + (1 << shift) - 1) >> shift;
+  auto chunk_end = [&](int64_t q) { return (uint32_t)std::min<int64_t>(S, (q + 1) << shift); };
+  RawArray<uint32_t> a_off, a_n;
+  a_off.alloc(S);
+  a_n.alloc(S);
   std::vector<List> a_chunk(chunks);
-  uint64_t total = 0;
+  std::atomic<uint64_t> total{0};
   const uint64_t limit = (uint64_t)kClosureMaxGrowth * (L.up_in.size() + L.dn_in.size()) + 1024;
-#pragma omp parallel for schedule(dynamic) reduction(+ : total)
-  for (int64_t q = 0; q < chunks; ++q) {
-    List l;
-    for (int64_t s = q * kChunk; s < std::min<int64_t>(S, (q + 1) * kChunk) && !too_long; ++s) {
+  parallel(chunks, many, [&](int64_t q) {
+    List l, out;  // local: neighbouring chunks' lists share cache lines
+    out.reserve((size_t)4 << shift);
+    for (uint32_t s = (uint32_t)(q << shift); s < chunk_end(q) && !refused; ++s) {
       l.clear();
       expand_final(L.sv_dev[s], l);
-      a_off[s + 1] = (uint32_t)l.size();
-      a_chunk[q].insert(a_chunk[q].end(), l.begin(), l.end());
-      total += l.size();
+      finish(L.sv_dev[s], l);
+      a_off[s] = (uint32_t)out.size();
+      a_n[s] = (uint32_t)l.size();
+      out.insert(out.end(), l.begin(), l.end());
     }
-  }
-  if (too_long || total > limit || total > (1u << 30)) return HostClosure{};
-  for (uint32_t s = 0; s < S; ++s) a_off[s + 1] += a_off[s];
-  List a(total);
-#pragma omp parallel for schedule(static)
-  for (int64_t q = 0; q < chunks; ++q)
-    std::copy(a_chunk[q].begin(), a_chunk[q].end(), a.begin() + a_off[q * kChunk]);
-  a_chunk = std::vector<List>();
+    total += out.size();
+    a_chunk[q] = std::move(out);
+  });
+  if (refused || total > limit || total > (1u << 30)) return HostClosure{};
+  auto a_list = [&](uint32_t s) { return a_chunk[s >> shift].data() + a_off[s]; };
   // merged entries: both, M only, F only
-  c.rec.assign((size_t)4 * S, 0);
-  std::vector<List> e_chunk(chunks);
-  std::vector<uint32_t> e_cnt((size_t)S + 1, 0);
-  total = 0;
-#pragma omp parallel for schedule(dynamic) reduction(+ : total)
-  for (int64_t q = 0; q < chunks; ++q) {
-    List b, both, m, f;
-    for (int64_t s = q * kChunk; s < std::min<int64_t>(S, (q + 1) * kChunk) && !too_long; ++s) {
-      b.clear();
-      both.clear();
-      m.clear();
-      f.clear();
-      for (uint32_t k = L.vin_off[s]; k < L.vin_off[s + 1]; ++k) {
-        const uint32_t u = L.vin_srcv[k], len = L.sv_off[u + 1] - L.sv_off[u];
-        b.push_back({(int32_t)u, 0});
-        for (uint32_t j = a_off[u]; j < a_off[u + 1]; ++j)
-          b.push_back({a[j].src, add_w(a[j].w, (int32_t)(len - 1))});
-      }
-      tidy(b, -1);
-      uint32_t j = a_off[s];
-      for (const EdgeW& e : b) {
-        for (; j < a_off[s + 1] && a[j].src < e.src; ++j) f.push_back(a[j]);
-        if (j < a_off[s + 1] && a[j].src == e.src) {
-          if (e.w == a[j].w - 1) {
-            both.push_back(e);
-          } else {
-            if (e.w <= a[j].w) m.push_back(e);
-            f.push_back(a[j]);
-          }
-          ++j;
-        } else {
-          m.push_back(e);
-        }
-      }
-      for (; j < a_off[s + 1]; ++j) f.push_back(a[j]);
-      const size_t n = both.size() + m.size() + f.size();
-      if (std::max({both.size(), m.size(), f.size()}) > 255) too_long = true;
-      // light entries first: the sources that win are near
-      for (List* l : {&both, &m, &f}) {
-        std::stable_sort(l->begin(), l->end(), [](const EdgeW& x, const EdgeW& y) { return x.w < y.w; });
-        e_chunk[q].insert(e_chunk[q].end(), l->begin(), l->end());
-      }
-      e_cnt[s + 1] = (uint32_t)n;
-      c.rec[4 * s + 3] = (uint32_t)(both.size() | m.size() << 8 | f.size() << 16);
-      total += n;
-    }
-  }
-  if (too_long || total > 3 * limit || total > (1u << 30)) return HostClosure{};
-  for (uint32_t s = 0; s < S; ++s) e_cnt[s + 1] += e_cnt[s];
-  c.ent.resize(total);
-#pragma omp parallel for schedule(static)
-  for (int64_t q = 0; q < chunks; ++q)
-    std::copy(e_chunk[q].begin(), e_chunk[q].end(), c.ent.begin() + e_cnt[q * kChunk]);
   auto key = [&](uint32_t ch) { return (L.lab4[ch >> 3] >> ((ch & 7) * 4)) & 0xFu; };
   auto len_of = [&](uint32_t s) { return L.sv_off[s + 1] - L.sv_off[s]; };
-  c.ent16.resize(2 * c.ent.size());
-#pragma omp parallel for schedule(static)
-  for (int64_t s = 0; s < (int64_t)S; ++s) {
-    uint32_t* r = &c.rec[4 * (size_t)s];
-    r[0] = L.sv_off[s];
-    r[1] = len_of((uint32_t)s) | key(L.sv_off[s]) << 29;
-    r[2] = e_cnt[s];
-    const uint32_t n = r[3], kb = e_cnt[s] + (n & 255), km = kb + ((n >> 8) & 255);
-    for (uint32_t k = e_cnt[s]; k < e_cnt[s + 1]; ++k) {
-      const uint32_t w = std::min<uint32_t>((uint32_t)c.ent[k].w, 0xFFFE), none = 0xFFFF;
-      const uint32_t wm = k < km ? w : none, wf = k < kb ? w + 1 : k >= km ? w : none;
-      c.ent16[2 * (size_t)k] = (uint32_t)c.ent[k].src;
-      c.ent16[2 * (size_t)k + 1] = wm | wf << 16;
+  c.rec.alloc((size_t)4 * S);
+  std::vector<std::vector<EdgeW>> e_chunk(chunks);
+  std::vector<uint32_t> h_chunk(chunks + 1, 0);  // long lists
+  total = 0;
+  parallel(chunks, many, [&](int64_t q) {
+    List b, t, cls[3];
+    std::vector<EdgeW> out;
+    uint32_t heavy = 0;
+    out.reserve((size_t)6 << shift);
+    for (uint32_t s = (uint32_t)(q << shift); s < chunk_end(q) && !refused; ++s) {
+      b.clear();
+      for (List& l : cls) l.clear();
+      for (uint32_t k = L.vin_off[s]; k < L.vin_off[s + 1]; ++k) {
+        const uint32_t u = L.vin_srcv[k];
+        merge(b, a_list(u), a_list(u) + a_n[u], (int32_t)(len_of(u) - 1), t);
+        const Entry last = entry(u, 0);
+        merge(t, &last, &last + 1, 0, b);
+      }
+      const Entry *a = a_list(s), *const a_end = a + a_n[s];
+      for (const Entry e : b) {
+        for (; a != a_end && src_of(*a) < src_of(e); ++a) cls[2].push_back(*a);
+        if (a != a_end && src_of(*a) == src_of(e)) {
+          if (w_of(e) == w_of(*a) - 1) {
+            cls[0].push_back(e);
+          } else {
+            if (w_of(e) <= w_of(*a)) cls[1].push_back(e);
+            cls[2].push_back(*a);
+          }
+          ++a;
+        } else {
+          cls[1].push_back(e);
+        }
+      }
+      cls[2].insert(cls[2].end(), a, a_end);
+      if (std::max({cls[0].size(), cls[1].size(), cls[2].size()}) > 255) refused = true;
+      const uint32_t at = (uint32_t)out.size();
+      // light entries first: the sources that win are near
+      for (List& l : cls) {
+        for (Entry& e : l) e = e << 32 | e >> 32;
+        std::sort(l.begin(), l.end());
+        for (const Entry e : l) out.push_back(EdgeW{(int32_t)(uint32_t)e, (int32_t)(e >> 32)});
+      }
+      uint32_t* r = &c.rec[4 * (size_t)s];
+      r[0] = L.sv_off[s];
+      r[1] = len_of(s) | key(L.sv_off[s]) << 29;
+      r[2] = at;
+      r[3] = (uint32_t)(cls[0].size() | cls[1].size() << 8 | cls[2].size() << 16);
+      heavy += out.size() - at > kWordLight;
     }
+    total += out.size();
+    e_chunk[q] = std::move(out);
+    h_chunk[q + 1] = heavy;
+  });
+  if (refused || total > 3 * limit || total > (1u << 30)) return HostClosure{};
+  std::vector<uint32_t> e_base(chunks + 1, 0);
+  for (int64_t q = 0; q < chunks; ++q) {
+    e_base[q + 1] = e_base[q] + (uint32_t)e_chunk[q].size();
+    h_chunk[q + 1] += h_chunk[q];
   }
-  for (int i = 0; i < 3; ++i) {
-    const uint32_t W = 32u << i;
-    std::vector<uint8_t>& out = c.by_len[i];
-    out.resize(S);
-#pragma omp parallel for schedule(static)
-    for (int64_t w0 = 0; w0 < (int64_t)S; w0 += W) {
-      const uint32_t n = std::min<uint32_t>(W, S - (uint32_t)w0);
-      uint8_t* o = &out[w0];
-      std::iota(o, o + n, (uint8_t)0);
-      std::stable_sort(o, o + n, [&](uint8_t x, uint8_t y) {
-        return len_of((uint32_t)w0 + x) > len_of((uint32_t)w0 + y);
-      });
-    }
-  }
-  // the word kernel's order and arrays
-  c.pos.resize(S);
-  std::vector<uint32_t> at(S);
-  auto count = [&](uint32_t s) { return e_cnt[s + 1] - e_cnt[s]; };
-  {
-    uint32_t h = 0;
-    for (uint32_t s = 0; s < S; ++s)
-      if (count(s) > kWordLight) at[h++] = s;
-    c.heavy = h;
-    for (uint32_t s = 0; s < S; ++s)
-      if (count(s) <= kWordLight) at[h++] = s;
-  }
-#pragma omp parallel for schedule(static)
-  for (int64_t w0 = c.heavy; w0 < (int64_t)S; w0 += kWordWindow) {
-    const auto b = at.begin() + w0, e = at.begin() + std::min<int64_t>(S, w0 + kWordWindow);
-    // by list length, then vertices without chain chars together
-    auto rank = [&](uint32_t s) { return 2 * count(s) + (len_of(s) > 1 ? 1u : 0u); };
-    std::stable_sort(b, e, [&](uint32_t x, uint32_t y) { return rank(x) > rank(y); });
-  }
-#pragma omp parallel for schedule(static)
-  for (int64_t i = 0; i < (int64_t)S; ++i) c.pos[at[i]] = (uint32_t)i;
-  c.wsv.resize((size_t)2 * S);
-  c.wrec.resize((size_t)4 * S);
-  // groups of 32 positions, counted from the first short list on
-  const uint32_t groups = c.heavy / 32 + 1 + (S - c.heavy + 31) / 32;
-  auto g_lo = [&](uint32_t q) {  // positions [g_lo(q), g_lo(q + 1))
-    const uint32_t hg = c.heavy / 32 + 1;
-    return q < hg ? std::min(32 * q, c.heavy) : std::min<uint32_t>(S, c.heavy + 32 * (q - hg));
+  c.heavy = h_chunk[chunks];
+  c.ent.alloc(e_base[chunks]);
+  RawArray<uint32_t> at;
+  at.alloc(S);
+  auto count = [&](uint32_t s) {
+    const uint32_t n = c.rec[4 * (size_t)s + 3];
+    return (n & 255) + ((n >> 8) & 255) + (n >> 16);
   };
-  std::vector<uint64_t> g_words((size_t)groups + 1, 0), g_ent((size_t)groups + 1, 0);
-#pragma omp parallel for schedule(static)
-  for (int64_t q = 0; q < (int64_t)groups; ++q) {
+  parallel(chunks, many, [&](int64_t q) {
+    std::copy(e_chunk[q].begin(), e_chunk[q].end(), c.ent.data() + e_base[q]);
+    const uint32_t s0 = (uint32_t)(q << shift);
+    uint32_t h = h_chunk[q], l = c.heavy + s0 - h;
+    for (uint32_t s = s0; s < chunk_end(q); ++s) {
+      c.rec[4 * (size_t)s + 2] += e_base[q];
+      at[count(s) > kWordLight ? h++ : l++] = s;
+    }
+  });
+  // the word kernel's order: segments of up to kWordWindow positions, those of
+  // the long lists first
+  const int64_t hs = ((int64_t)c.heavy + kWordWindow - 1) / kWordWindow,
+                segs = hs + ((int64_t)S - c.heavy + kWordWindow - 1) / kWordWindow;
+  auto seg = [&](int64_t q) {
+    const int64_t lo = q < hs ? q * kWordWindow : c.heavy + (q - hs) * kWordWindow,
+                  end = q < hs ? c.heavy : S;
+    return std::pair<uint32_t, uint32_t>((uint32_t)lo, (uint32_t)std::min<int64_t>(end, lo + kWordWindow));
+  };
+  std::vector<uint64_t> w_base(segs + 1, 0), n_base(segs + 1, 0);
+  parallel(segs, many, [&](int64_t q) {
+    const auto [lo, hi] = seg(q);
+    if (q >= hs) {
+      // by list length, then vertices without chain chars together, else in
+      // their order: a counting sort
+      uint32_t first[2 * kWordLight + 3] = {}, s_of[kWordWindow];
+      auto rank = [&](uint32_t s) { return 2 * (kWordLight - count(s)) + (len_of(s) > 1 ? 0 : 1); };
+      for (uint32_t i = lo; i < hi; ++i) ++first[rank(at[i]) + 1];
+      for (uint32_t r = 1; r < 2 * kWordLight + 2; ++r) first[r + 1] += first[r];
+      for (uint32_t i = lo; i < hi; ++i) s_of[first[rank(at[i])]++] = at[i];
+      std::copy(s_of, s_of + (hi - lo), at.data() + lo);
+    }
     uint64_t w = 0, n = 0;
-    for (uint32_t i = g_lo((uint32_t)q); i < g_lo((uint32_t)q + 1); ++i) {
+    for (uint32_t i = lo; i < hi; ++i) {
       w += (len_of(at[i]) - 1 + 31) / 32;
-      n = i < c.heavy ? n + count(at[i]) : std::max<uint64_t>(n, 32ull * count(at[i]));
+      // a group of short lists is as wide as its longest, which is its first
+      if (q < hs || (i - lo) % 32 == 0) n += (q < hs ? 1 : 32) * count(at[i]);
     }
-    g_words[q + 1] = w;
-    g_ent[q + 1] = n;
+    w_base[q + 1] = w;
+    n_base[q + 1] = n;
+  });
+  for (int64_t q = 0; q < segs; ++q) {
+    w_base[q + 1] += w_base[q];
+    n_base[q + 1] += n_base[q];
   }
-  for (uint32_t q = 0; q < groups; ++q) {
-    g_words[q + 1] += g_words[q];
-    g_ent[q + 1] += g_ent[q];
-  }
-  if (g_words[groups] >= (1ull << 31) || g_ent[groups] >= (1ull << 31)) return HostClosure{};
-  c.words = g_words[groups];
-  c.lab.assign(4 * (size_t)std::max<uint64_t>(c.words, 1), 0);
-  c.went.assign((size_t)g_ent[groups], EdgeW{0, 0});
-#pragma omp parallel for schedule(static)
-  for (int64_t q = 0; q < (int64_t)groups; ++q) {
-    uint64_t wo = g_words[q], eo = g_ent[q];
-    const uint32_t lo = g_lo((uint32_t)q);
-    for (uint32_t i = lo; i < g_lo((uint32_t)q + 1); ++i) {
-      const uint32_t s = at[i], f = L.sv_off[s], len = len_of(s), n = count(s);
-      const bool heavy = i < c.heavy;
-      uint32_t* r = &c.wrec[4 * (size_t)i];
-      c.wsv[2 * (size_t)i] = s;
-      c.wsv[2 * (size_t)i + 1] = f;
-      r[0] = (uint32_t)wo;
-      r[1] = len | key(f) << 29;
-      r[2] = (uint32_t)(heavy ? eo : eo + (i - lo));
-      r[3] = n;
-      const uint32_t nb = c.rec[4 * (size_t)s + 3] & 255, nm = (c.rec[4 * (size_t)s + 3] >> 8) & 255;
-      for (uint32_t k = 0; k < n; ++k) {
-        const EdgeW& e = c.ent[e_cnt[s] + k];
-        const uint32_t cls = k < nb ? 0u : k < nb + nm ? 1u : 2u;
-        c.went[r[2] + (heavy ? 1 : 32) * (size_t)k] = EdgeW{(int32_t)((uint32_t)e.src | cls << 30), e.w};
+  if (w_base[segs] >= (1ull << 31) || n_base[segs] >= (1ull << 31)) return HostClosure{};
+  c.words = w_base[segs];
+  c.n_went = n_base[segs];
+  c.order.alloc((size_t)4 * S);
+  parallel(segs, many, [&](int64_t q) {
+    const auto [lo, hi] = seg(q);
+    uint64_t w = w_base[q], n = n_base[q], wide = 0;
+    for (uint32_t i = lo; i < hi; ++i) {
+      const uint32_t k = (i - lo) % 32;
+      if (q >= hs && k == 0) {
+        n += wide;
+        wide = 32ull * count(at[i]);
       }
-      if (heavy) eo += n;
-      for (uint32_t k = 0; k + 1 < len; ++k) {
-        uint32_t* w = &c.lab[4 * (wo + k / 32)];
-        const uint32_t x = key(f + 1 + k), bit = 1u << (k & 31);
-        if (x & 1) w[0] |= bit;
-        if (x & 2) w[1] |= bit;
-        if (x & 4) w[2] |= bit;
-      }
-      wo += (len - 1 + 31) / 32;
+      uint32_t* r = &c.order[4 * (size_t)i];
+      r[0] = (uint32_t)w;
+      r[1] = at[i];
+      r[2] = (uint32_t)(q < hs ? n : n + k);
+      r[3] = 0;
+      w += (len_of(at[i]) - 1 + 31) / 32;
+      if (q < hs) n += count(at[i]);
     }
-  }
+  });
   c.ok = true;
   return c;
 }

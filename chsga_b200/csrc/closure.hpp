@@ -27,8 +27,9 @@
 // engine sweeps the levels instead.
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
-#include <vector>
+#include <memory>
 
 #include "device_graph.hpp"
 
@@ -40,43 +41,53 @@ constexpr uint32_t kClosureMaxList = 192;
 constexpr uint32_t kClosureMaxGrowth = 6;
 constexpr uint32_t kWordWindow = 512, kWordLight = 8;
 
+// An array that is not cleared first: it is filled by all threads, which then
+// share its page faults too (a quarter of the build's time where one thread
+// cleared it).
+template <typename T>
+class RawArray {
+ public:
+  void alloc(size_t n) {
+    p_.reset(new T[n]);
+    n_ = n;
+  }
+  T& operator[](size_t i) { return p_[i]; }
+  const T& operator[](size_t i) const { return p_[i]; }
+  T* data() { return p_.get(); }
+  const T* data() const { return p_.get(); }
+  size_t size() const { return n_; }
+
+ private:
+  std::unique_ptr<T[]> p_;
+  size_t n_ = 0;
+};
+
 struct HostClosure {
   bool ok = false;
   // 4 words per string vertex: first char; length | label key of the first
   // char << 29; first entry; entries of each class (both | M only << 8 | F
   // only << 16)
-  std::vector<uint32_t> rec;
+  RawArray<uint32_t> rec;
   // {source vertex, weight}, classes in that order; the weight counts for M
   // (a "both" entry has weight w + 1 for F), for F-only entries for F
-  std::vector<EdgeW> ent;
-  // the entries for 16-bit rows: {source vertex, weight for M | weight for F
-  // << 16}, 0xFFFF = no such entry (or a weight no 16-bit score can win with)
-  std::vector<uint32_t> ent16;
-  // order of the vertices inside every window of 32, 64 and 128 by label
-  // length (local indexes)
-  std::vector<uint8_t> by_len[3];
+  RawArray<EdgeW> ent;
 
   // The one-read-a-word kernel works in an order of its own. Vertices with
   // more than kWordLight entries come first (several lanes share such a
   // list); the others follow, by list length inside every window of
   // kWordWindow vertices, so that the 32 vertices of a warp end together and
-  // lie side by side in these arrays. Everything below is by position in that
-  // order (the scores stay by string vertex, where neighbours are near).
+  // lie side by side in the arrays of that order (the scores stay by string
+  // vertex, where neighbours are near).
   //   heavy     vertices of the first kind
-  //   pos       position of string vertex s
-  //   wsv       {string vertex, first char}
-  //   wrec      4 words: first bit word; length | key << 29; first entry; entries
-  //   went      {source vertex | class << 30 (0 both, 1 M only, 2 F only),
-  //             weight}; a long list is contiguous, entry k of a short one is at
-  //             wrec[2] + 32 k (a group of 32 vertices side by side)
-  //   lab       per bit word the label planes of its 32 chain chars (bit k of
-  //             word j = char first + 1 + 32 j + k): {code bit 0, code bit 1,
-  //             special, 0}
+  //   order     4 words per position: first bit word, string vertex, first of
+  //             its n_went entries, 0. A long list is contiguous, entry k of a
+  //             short one lies at first + 32 k (a group of 32 vertices side
+  //             by side)
+  //   words     bit words (32 chain chars each)
+  // The arrays themselves are made on the device (k_closure_arrays).
   uint32_t heavy = 0;
-  std::vector<uint32_t> pos, wsv, wrec;
-  std::vector<EdgeW> went;
-  std::vector<uint32_t> lab;
-  uint64_t words = 0;
+  RawArray<uint32_t> order;
+  uint64_t n_went = 0, words = 0;
 };
 
 HostClosure build_closure(const HostLayout& L);

@@ -101,11 +101,8 @@ struct GraphDev {
   DevArr<uint4> t1_desc, t1_vrec;  // tiles of the one-read row kernel (k_row_t1)
   DevArr<uint8_t> t1_heads;
   DevArr<uint32_t> delta_order;    // k_row_delta: runs of 32 string vertices by decreasing char count
-  // bit-row kernels (closure.hpp)
-  DevArr<uint4> cl_rec, cl_wrec, cl_lab;
-  DevArr<uint2> cl_ent16, cl_went, cl_wsv;
-  DevArr<uint8_t> cl_by_len[3];
-  DevArr<uint32_t> cl_pos;
+  DevArr<unsigned char> cl;        // every array of the bit-row kernels (closure.hpp)
+  const uint8_t* cl_by_len[3] = {};
 };
 
 struct TopDev {
@@ -877,7 +874,7 @@ void bit_step(chsga_ctx& c, BitBufs& b, int par, cudaStream_t s) {
       using S4 = dev::SlicedShared<R, 4>;
       using S1 = dev::SlicedShared<R, 1>;
       // four items a lane where that gives every warp of the device work
-      a.g.by_len = c.g->gd.cl_by_len[R == 128 ? 0 : R == 64 ? 1 : 2].p;
+      a.g.by_len = c.g->gd.cl_by_len[R == 128 ? 0 : R == 64 ? 1 : 2];
       const bool four = c.bit_form == BitForm::Auto ? S >= (uint32_t)S4::VB * 16u * (uint32_t)c.num_sms
                                                     : c.bit_form == BitForm::Sliced4;
       if (four)
@@ -1143,40 +1140,51 @@ void upload_graph(chsga_ctx& c, const chsga_graph_host& g) {
   {
     const HostClosure cl = build_closure(L);
     if (cl.ok) {
-      auto as4 = [&](DevArr<uint4>& to, const std::vector<uint32_t>& v) {
-        to.alloc(v.size() / 4);
-        CK(cudaMemcpyAsync(to.p, v.data(), v.size() * 4, cudaMemcpyHostToDevice, s));
+      // one allocation: {records, entries, order} as the host has them, then
+      // what the device makes from them
+      const size_t E = cl.ent.size(), W = std::max<uint64_t>(cl.words, 1);
+      size_t bytes = 0;
+      auto room = [&](size_t n) {
+        const size_t at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
       };
-      auto as2 = [&](DevArr<uint2>& to, const void* v, size_t n) {
-        to.alloc(n);
-        if (n) CK(cudaMemcpyAsync(to.p, v, n * sizeof(uint2), cudaMemcpyHostToDevice, s));
-      };
-      as4(d.cl_rec, cl.rec);
-      as4(d.cl_wrec, cl.wrec);
-      as4(d.cl_lab, cl.lab);
-      as2(d.cl_ent16, cl.ent16.data(), cl.ent16.size() / 2);
-      as2(d.cl_went, cl.went.data(), cl.went.size());
-      d.cl_pos.upload(cl.pos, s);
-      as2(d.cl_wsv, cl.wsv.data(), cl.wsv.size() / 2);
-      for (int i = 0; i < 3; ++i) d.cl_by_len[i].upload(cl.by_len[i], s);
-      CK(cudaStreamSynchronize(s));  // the host vectors die with this scope
-      lg->bits = true;
+      const size_t rec = room(16 * (size_t)L.S), ent = room(8 * E), wrec = room(16 * (size_t)L.S),
+                   wsv = room(8 * (size_t)L.S), pos = room(4 * (size_t)L.S), went = room(8 * cl.n_went),
+                   lab = room(16 * W), by32 = room(L.S), by64 = room(L.S), by128 = room(L.S);
+      d.cl.alloc(bytes);
+      unsigned char* const m = d.cl.p;
+      CK(cudaMemcpyAsync(m + rec, cl.rec.data(), 16 * (size_t)L.S, cudaMemcpyHostToDevice, s));
+      if (E) CK(cudaMemcpyAsync(m + ent, cl.ent.data(), 8 * E, cudaMemcpyHostToDevice, s));
+      CK(cudaMemcpyAsync(m + wrec, cl.order.data(), 16 * (size_t)L.S, cudaMemcpyHostToDevice, s));
       dev::BitGraph& b = lg->bg;
       b.S = L.S;
       b.N = L.N;
-      b.n_ent = (uint32_t)(cl.ent16.size() / 2);
-      b.n_went = (uint32_t)cl.went.size();
+      b.n_ent = (uint32_t)E;
+      b.n_went = (uint32_t)cl.n_went;
       b.heavy = cl.heavy;
       b.words = cl.words;
-      b.rec = d.cl_rec.p;
-      b.ent16 = d.cl_ent16.p;
+      b.rec = reinterpret_cast<const uint4*>(m + rec);
+      b.ent16 = reinterpret_cast<const uint2*>(m + ent);
       b.sv_off = d.sv_off.p;
       b.lab4 = d.lab4.p;
-      b.pos = d.cl_pos.p;
-      b.wsv = d.cl_wsv.p;
-      b.wrec = d.cl_wrec.p;
-      b.went = d.cl_went.p;
-      b.lab = d.cl_lab.p;
+      b.pos = reinterpret_cast<const uint32_t*>(m + pos);
+      b.wsv = reinterpret_cast<const uint2*>(m + wsv);
+      b.wrec = reinterpret_cast<const uint4*>(m + wrec);
+      b.went = reinterpret_cast<const uint2*>(m + went);
+      b.lab = reinterpret_cast<const uint4*>(m + lab);
+      dev::k_closure_arrays<<<nblocks((uint64_t)L.S * 8), 256, 0, s>>>(
+          L.S, cl.heavy, b.rec, reinterpret_cast<uint2*>(m + ent), reinterpret_cast<uint4*>(m + wrec),
+          reinterpret_cast<uint2*>(m + wsv), reinterpret_cast<uint32_t*>(m + pos),
+          reinterpret_cast<uint2*>(m + went), reinterpret_cast<uint4*>(m + lab), b.lab4);
+      check_launch();
+      dev::k_by_len<<<nblocks(L.S, 128), 128, 0, s>>>(L.S, b.sv_off, m + by32, m + by64, m + by128);
+      check_launch();
+      d.cl_by_len[0] = m + by32;
+      d.cl_by_len[1] = m + by64;
+      d.cl_by_len[2] = m + by128;
+      CK(cudaStreamSynchronize(s));  // the host arrays die with this scope
+      lg->bits = true;
     }
   }
   lg->nul_label = false;
