@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <exception>
 #include <vector>
 
 namespace chsga {
@@ -51,11 +52,22 @@ void merge(const List& a, const Entry* b, const Entry* b_end, int32_t by, List& 
   }
 }
 
-// f(i) for i in [0, n), on all threads when there are many.
+// f(i) for i in [0, n), on all threads when there are many; what one of them
+// throws is thrown here when all are done.
 template <typename F>
 void parallel(int64_t n, bool many, F&& f) {
+  std::exception_ptr err;
+  std::atomic<bool> failed{false};
 #pragma omp parallel for schedule(dynamic) if (many)
-  for (int64_t i = 0; i < n; ++i) f(i);
+  for (int64_t i = 0; i < n; ++i) {
+    if (failed.load(std::memory_order_relaxed)) continue;
+    try {
+      f(i);
+    } catch (...) {
+      if (!failed.exchange(true)) err = std::current_exception();
+    }
+  }
+  if (err) std::rethrow_exception(err);
 }
 
 }  // namespace
@@ -80,22 +92,27 @@ HostClosure build_closure(const HostLayout& L) {
   mark(L.dn_in, dn_src);
   std::vector<uint32_t> slot(S, 0);
   std::vector<List> ups(1), fins(1);
+  auto self_of = [&](uint32_t d) { return single(d) ? (int64_t)L.dv_s[d] : -1; };
   // the source of an edge and, through a one-char source, that one's sources
-  auto take = [&](const EdgeW& e, bool through, const std::vector<List>& lists,
+  auto take = [&](uint32_t d, const EdgeW& e, bool through, const std::vector<List>& lists,
                   const std::vector<uint32_t>& at, List& l) {
     const uint32_t x = (uint32_t)e.src >> 1;
     l.push_back(entry(L.dv_s[x], e.w));
-    if (through)
-      for (const Entry y : lists[at[x]]) l.push_back(heavier(y, e.w));
+    if (!through) return;
+    for (const Entry y : lists[at[x]]) l.push_back(heavier(y, e.w));
+    if (l.size() > kClosureTidy) {
+      tidy(l, self_of(d));
+      if (l.size() > kClosureMaxList) refused = true;
+    }
   };
   auto expand_up = [&](uint32_t d, List& l) {
     for (uint32_t k = L.up_off[d]; k < L.up_off[d + 1] && !refused; ++k) {
       const uint32_t x = (uint32_t)L.up_in[k].src >> 1;
-      take(L.up_in[k], single(x) && L.up_off[x + 1] > L.up_off[x], ups, slot, l);
+      take(d, L.up_in[k], single(x) && L.up_off[x + 1] > L.up_off[x], ups, slot, l);
     }
   };
   auto finish = [&](uint32_t d, List& l) {
-    tidy(l, single(d) ? (int64_t)L.dv_s[d] : -1);
+    tidy(l, self_of(d));
     if (l.size() > kClosureMaxList) refused = true;
   };
   // the one-char vertices of a level that `want` picks, in pieces of 64
@@ -126,7 +143,7 @@ HostClosure build_closure(const HostLayout& L) {
   auto expand_final = [&](uint32_t d, List& l) {
     expand_up(d, l);
     for (uint32_t k = L.dn_off[d]; k < L.dn_off[d + 1] && !refused; ++k)
-      take(L.dn_in[k], single((uint32_t)L.dn_in[k].src >> 1), fins, fslot, l);
+      take(d, L.dn_in[k], single((uint32_t)L.dn_in[k].src >> 1), fins, fslot, l);
   };
   for (uint32_t l = L.levels; l-- > 0 && !refused;)
     by_level(l, fins, fslot, [&](uint32_t d) { return dn_src[d] != 0; }, expand_final);
@@ -144,6 +161,10 @@ HostClosure build_closure(const HostLayout& L) {
   std::vector<List> a_chunk(chunks);
   std::atomic<uint64_t> total{0};
   const uint64_t limit = (uint64_t)kClosureMaxGrowth * (L.up_in.size() + L.dn_in.size()) + 1024;
+  auto grow = [&](uint64_t n, uint64_t most) {
+    const uint64_t now = total.fetch_add(n, std::memory_order_relaxed) + n;
+    if (now > most || now > (1u << 30)) refused = true;
+  };
   parallel(chunks, many, [&](int64_t q) {
     List l, out;  // local: neighbouring chunks' lists share cache lines
     out.reserve((size_t)4 << shift);
@@ -155,10 +176,10 @@ HostClosure build_closure(const HostLayout& L) {
       a_n[s] = (uint32_t)l.size();
       out.insert(out.end(), l.begin(), l.end());
     }
-    total += out.size();
+    grow(out.size(), limit);
     a_chunk[q] = std::move(out);
   });
-  if (refused || total > limit || total > (1u << 30)) return HostClosure{};
+  if (refused) return HostClosure{};
   auto a_list = [&](uint32_t s) { return a_chunk[s >> shift].data() + a_off[s]; };
   // merged entries: both, M only, F only
   auto key = [&](uint32_t ch) { return (L.lab4[ch >> 3] >> ((ch & 7) * 4)) & 0xFu; };
@@ -180,6 +201,9 @@ HostClosure build_closure(const HostLayout& L) {
         merge(b, a_list(u), a_list(u) + a_n[u], (int32_t)(len_of(u) - 1), t);
         const Entry last = entry(u, 0);
         merge(t, &last, &last + 1, 0, b);
+        // more than the three classes and the dropped ones can hold
+        if (b.size() > kClosureTidy) refused = true;
+        if (refused) return;
       }
       const Entry *a = a_list(s), *const a_end = a + a_n[s];
       for (const Entry e : b) {
@@ -212,11 +236,11 @@ HostClosure build_closure(const HostLayout& L) {
       r[3] = (uint32_t)(cls[0].size() | cls[1].size() << 8 | cls[2].size() << 16);
       heavy += out.size() - at > kWordLight;
     }
-    total += out.size();
+    grow(out.size(), 3 * limit);
     e_chunk[q] = std::move(out);
     h_chunk[q + 1] = heavy;
   });
-  if (refused || total > 3 * limit || total > (1u << 30)) return HostClosure{};
+  if (refused) return HostClosure{};
   std::vector<uint32_t> e_base(chunks + 1, 0);
   for (int64_t q = 0; q < chunks; ++q) {
     e_base[q + 1] = e_base[q] + (uint32_t)e_chunk[q].size();

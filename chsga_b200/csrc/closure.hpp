@@ -37,8 +37,13 @@ namespace chsga {
 
 // Longest list a vertex may have, and entries per hierarchy edge above which
 // the level sweeps are kept.
+// A list is cut down to one entry a source whenever it is longer than
+// kClosureTidy on the way, and the totals are watched while the lists grow, so
+// a graph that is refused costs little time and no more memory than one that
+// is not.
 constexpr uint32_t kClosureMaxList = 192;
 constexpr uint32_t kClosureMaxGrowth = 6;
+constexpr uint32_t kClosureTidy = 1024;
 constexpr uint32_t kWordWindow = 512, kWordLight = 8;
 
 // An array that is not cleared first: it is filled by all threads, which then
@@ -90,6 +95,7 @@ struct HostClosure {
   uint64_t n_went = 0, words = 0;
 };
 
+// Throws std::bad_alloc like a vector would, whichever thread ran out.
 HostClosure build_closure(const HostLayout& L);
 
 }  // namespace chsga
