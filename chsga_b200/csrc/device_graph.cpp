@@ -262,31 +262,6 @@ HostLayout build_layout(const chsga_graph_host& g) {
     for (uint64_t j = p.down_offset[u]; j < p.down_offset[u + 1]; ++j)
       L.dn_in[k++] = {(int32_t)bv_last(p.down_v[j]), (int32_t)p.down_w[j]};
   }
-  L.dn_head.assign((size_t)4 * S, 0);
-  // upward lists average about two edges: their head carries the first two
-  // (8 words: begin, end, src0, w0, src1, w1, 0, 0)
-  L.up_head.assign((size_t)8 * S, 0);
-  L.fin.assign((size_t)4 * S, 0);
-#pragma omp parallel for schedule(static)
-  for (int64_t d = 0; d < (int64_t)S; ++d) {
-    uint32_t* h = &L.dn_head[(size_t)4 * d];
-    h[0] = L.dn_off[d];
-    h[1] = L.dn_off[d + 1];
-    if (L.dn_off[d + 1] > L.dn_off[d]) {
-      h[2] = (uint32_t)L.dn_in[L.dn_off[d]].src;
-      h[3] = (uint32_t)L.dn_in[L.dn_off[d]].w;
-    }
-    uint32_t* u8 = &L.up_head[(size_t)8 * d];
-    u8[0] = L.up_off[d];
-    u8[1] = L.up_off[d + 1];
-    for (uint32_t j = 0; j < 2 && L.up_off[d] + j < L.up_off[d + 1]; ++j) {
-      u8[2 + 2 * j] = (uint32_t)L.up_in[L.up_off[d] + j].src;
-      u8[3 + 2 * j] = (uint32_t)L.up_in[L.up_off[d] + j].w;
-    }
-    L.fin[4 * d] = L.dv_first[d];
-    L.fin[4 * d + 1] = L.dv_len[d];
-    L.fin[4 * d + 2] = L.dv_s[d];
-  }
   // levels in hierarchy order
   L.lvl_off.push_back(0);
   for (uint32_t d = 1; d < S; ++d)
@@ -304,17 +279,27 @@ HostLayout build_layout(const chsga_graph_host& g) {
   // --- string-graph in-CSR for the traceback walk (traceback.hpp:716) -------
   const chsga_csr& sg = g.string_graph;
   L.istr_off.assign(S + 1, 0);
-  for (uint64_t u = 0; u < S; ++u)
+  uint64_t bad_st = 0;
+#pragma omp parallel for reduction(+ : bad_st) schedule(dynamic, 1 << 12)
+  for (int64_t u = 0; u < (int64_t)S; ++u)
     for (uint64_t e = sg.offset[u]; e < sg.offset[u + 1]; ++e) {
-      require(sg.target[e] < S, CHSGA_ERR_FORMAT, "string edge target out of range");
-      L.istr_off[sg.target[e] + 1]++;
+      if (sg.target[e] < S)
+        __atomic_fetch_add(&L.istr_off[sg.target[e] + 1], 1u, __ATOMIC_RELAXED);
+      else
+        ++bad_st;
     }
+  require(bad_st == 0, CHSGA_ERR_FORMAT, "string edge target out of range");
   for (uint32_t v = 0; v < S; ++v) L.istr_off[v + 1] += L.istr_off[v];
   L.istr_src.resize(L.istr_off[S]);
   {
     std::vector<uint32_t> cur(L.istr_off.begin(), L.istr_off.end() - 1);
-    for (uint64_t u = 0; u < S; ++u)
-      for (uint64_t e = sg.offset[u]; e < sg.offset[u + 1]; ++e) L.istr_src[cur[sg.target[e]]++] = (uint32_t)u;
+#pragma omp parallel for schedule(dynamic, 1 << 12)
+    for (int64_t u = 0; u < (int64_t)S; ++u)
+      for (uint64_t e = sg.offset[u]; e < sg.offset[u + 1]; ++e)
+        L.istr_src[__atomic_fetch_add(&cur[sg.target[e]], 1u, __ATOMIC_RELAXED)] = (uint32_t)u;
+#pragma omp parallel for schedule(dynamic, 1 << 12)
+    for (int64_t v = 0; v < (int64_t)S; ++v)
+      std::sort(L.istr_src.begin() + L.istr_off[v], L.istr_src.begin() + L.istr_off[v + 1]);
   }
   return L;
 }

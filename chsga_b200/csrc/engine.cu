@@ -1094,19 +1094,21 @@ void upload_graph(chsga_ctx& c, const chsga_graph_host& g) {
   d.istr_off.upload(L.istr_off, s);
   d.istr_src.upload(L.istr_src, s);
   d.dv_s.upload(L.dv_s, s);
-  std::vector<int2> up(L.up_in.size()), dn(L.dn_in.size());
-  for (size_t i = 0; i < up.size(); ++i) up[i] = make_int2(L.up_in[i].src, L.up_in[i].w);
-  for (size_t i = 0; i < dn.size(); ++i) dn[i] = make_int2(L.dn_in[i].src, L.dn_in[i].w);
-  d.up_in.upload(up, s);
-  d.dn_in.upload(dn, s);
-  auto to4 = [](const std::vector<uint32_t>& v) {
-    std::vector<uint4> o(v.size() / 4);
-    std::memcpy(o.data(), v.data(), o.size() * sizeof(uint4));
-    return o;
+  // a host array as the device's records of the same layout
+  auto as = [&](auto& to, const auto& v) {
+    const size_t each = sizeof(*to.p), n = v.size() * sizeof(v[0]) / each;
+    to.alloc(n);
+    if (n) CK(cudaMemcpyAsync(to.p, v.data(), n * each, cudaMemcpyHostToDevice, s));
   };
-  d.dn_head.upload(to4(L.dn_head), s);
-  d.up_head.upload(to4(L.up_head), s);
-  d.fin.upload(to4(L.fin), s);
+  static_assert(sizeof(EdgeW) == sizeof(int2), "host edges are the device's");
+  as(d.up_in, L.up_in);
+  as(d.dn_in, L.dn_in);
+  d.dn_head.alloc(L.S);
+  d.up_head.alloc(2 * (size_t)L.S);
+  d.fin.alloc(L.S);
+  dev::k_heads<<<nblocks(L.S), 256, 0, s>>>(L.S, d.up_off.p, d.up_in.p, d.dn_off.p, d.dn_in.p, d.dv_first.p,
+                                            d.dv_len.p, d.dv_s.p, d.dn_head.p, d.up_head.p, d.fin.p);
+  check_launch();
   {
     // runs of 32 consecutive string vertices, longest (in chars) first; ties by index
     const uint32_t nruns = (L.S + 31) / 32;
@@ -1124,8 +1126,8 @@ void upload_graph(chsga_ctx& c, const chsga_graph_host& g) {
   {
     HostT1 t1 = build_t1(L);
     if (t1.ok) {
-      d.t1_desc.upload(to4(t1.desc), s);
-      d.t1_vrec.upload(to4(t1.vrec), s);
+      as(d.t1_desc, t1.desc);
+      as(d.t1_vrec, t1.vrec);
       d.t1_heads.upload(t1.heads, s);
       lg->t1 = dev::T1Ptrs{d.t1_desc.p, d.t1_heads.p, d.t1_vrec.p, t1.ntiles()};
     }
@@ -1187,11 +1189,8 @@ void upload_graph(chsga_ctx& c, const chsga_graph_host& g) {
       lg->bits = true;
     }
   }
-  lg->nul_label = false;
-  for (uint32_t i = 0; i < g.num_chars; ++i) {
-    lg->nul_label |= g.labels[i] == '\0';
-    lg->n_label |= g.labels[i] == 'N';
-  }
+  lg->nul_label = std::memchr(g.labels, '\0', g.num_chars) != nullptr;
+  lg->n_label = std::memchr(g.labels, 'N', g.num_chars) != nullptr;
   lg->pitch = ((size_t)L.N + 15) / 16 * 16;
   lg->L = std::move(L);
   lg->top = std::move(top);

@@ -66,6 +66,28 @@ struct GraphPtrs {
   uint32_t n_vin, n_up, n_dn;  // entries of vin_srcv, up_in, dn_in (index checks)
 };
 
+// dn_head, up_head and fin from the lists, one thread per hierarchy position,
+// once a graph is loaded (64 bytes a position, which the host would spend
+// longer to write and to upload than the device to fill).
+__global__ void __launch_bounds__(256) k_heads(uint32_t S, const uint32_t* __restrict__ up_off,
+                                               const int2* __restrict__ up_in,
+                                               const uint32_t* __restrict__ dn_off,
+                                               const int2* __restrict__ dn_in,
+                                               const uint32_t* __restrict__ dv_first,
+                                               const uint32_t* __restrict__ dv_len,
+                                               const uint32_t* __restrict__ dv_s, uint4* dn_head, uint4* up_head,
+                                               uint4* fin) {
+  const uint32_t d = blockIdx.x * 256 + threadIdx.x;
+  if (d >= S) return;
+  auto at = [](const int2* in, uint32_t k, uint32_t end) { return k < end ? in[k] : make_int2(0, 0); };
+  const uint32_t u0 = up_off[d], u1 = up_off[d + 1], d0 = dn_off[d], d1 = dn_off[d + 1];
+  const int2 a = at(up_in, u0, u1), b = at(up_in, u0 + 1, u1), c = at(dn_in, d0, d1);
+  up_head[2 * (size_t)d] = make_uint4(u0, u1, (uint32_t)a.x, (uint32_t)a.y);
+  up_head[2 * (size_t)d + 1] = make_uint4((uint32_t)b.x, (uint32_t)b.y, 0, 0);
+  dn_head[d] = make_uint4(d0, d1, (uint32_t)c.x, (uint32_t)c.y);
+  fin[d] = make_uint4(dv_first[d], dv_len[d], dv_s[d], 0);
+}
+
 // ---------------------------------------------------------------------------
 // Index checks of the CHSGA_CHECKED build (make CHECKED=1): every index a
 // kernel reads from a graph array before using it as an address is checked
