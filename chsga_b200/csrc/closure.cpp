@@ -24,6 +24,13 @@ Entry heavier(Entry e, int32_t by) {
   return entry(src_of(e), (int32_t)std::min<int64_t>((int64_t)w_of(e) + by, kMaxWeight));
 }
 
+// Lists by index, many to an allocation.
+struct Lists {
+  std::vector<const Entry*> first{nullptr};  // list 0 is empty
+  std::vector<uint32_t> n{0};
+  std::vector<List> store;
+};
+
 // One entry per source, the smallest weight; `self` (a one-char vertex's own
 // score, which a positive weight cannot lower) is dropped.
 void tidy(List& l, int64_t self) {
@@ -91,15 +98,16 @@ HostClosure build_closure(const HostLayout& L) {
   mark(L.up_in, up_src);
   mark(L.dn_in, dn_src);
   std::vector<uint32_t> slot(S, 0);
-  std::vector<List> ups(1), fins(1);
+  Lists ups, fins;
   auto self_of = [&](uint32_t d) { return single(d) ? (int64_t)L.dv_s[d] : -1; };
   // the source of an edge and, through a one-char source, that one's sources
-  auto take = [&](uint32_t d, const EdgeW& e, bool through, const std::vector<List>& lists,
-                  const std::vector<uint32_t>& at, List& l) {
+  auto take = [&](uint32_t d, const EdgeW& e, bool through, const Lists& lists, const std::vector<uint32_t>& at,
+                  List& l) {
     const uint32_t x = (uint32_t)e.src >> 1;
     l.push_back(entry(L.dv_s[x], e.w));
     if (!through) return;
-    for (const Entry y : lists[at[x]]) l.push_back(heavier(y, e.w));
+    const Entry* y = lists.first[at[x]];
+    for (uint32_t k = 0; k < lists.n[at[x]]; ++k) l.push_back(heavier(y[k], e.w));
     if (l.size() > kClosureTidy) {
       tidy(l, self_of(d));
       if (l.size() > kClosureMaxList) refused = true;
@@ -116,20 +124,36 @@ HostClosure build_closure(const HostLayout& L) {
     if (l.size() > kClosureMaxList) refused = true;
   };
   // the one-char vertices of a level that `want` picks, in pieces of 64
-  auto by_level = [&](uint32_t level, std::vector<List>& lists, std::vector<uint32_t>& at, auto&& want, auto&& make) {
-    const size_t first = lists.size();
+  auto by_level = [&](uint32_t level, Lists& lists, std::vector<uint32_t>& at, auto&& want, auto&& make) {
+    const size_t first = lists.n.size(), piece = lists.store.size();
     std::vector<uint32_t> todo;
     for (uint32_t d = L.lvl_off[level]; d < L.lvl_off[level + 1]; ++d)
       if (want(d)) {
         at[d] = (uint32_t)(first + todo.size());
         todo.push_back(d);
       }
-    lists.resize(first + todo.size());
-    parallel(((int64_t)todo.size() + 63) / 64, todo.size() > 256, [&](int64_t q) {
-      for (size_t i = 64 * (size_t)q; i < std::min(todo.size(), 64 * (size_t)q + 64) && !refused; ++i) {
-        make(todo[i], lists[first + i]);
-        finish(todo[i], lists[first + i]);
+    const size_t pieces = (todo.size() + 63) / 64;
+    lists.first.resize(first + todo.size());
+    lists.n.resize(first + todo.size());
+    lists.store.resize(piece + pieces);
+    parallel((int64_t)pieces, todo.size() > 256, [&](int64_t q) {
+      const size_t lo = 64 * (size_t)q, hi = std::min(todo.size(), lo + 64);
+      List l, out;
+      uint32_t n[64];
+      for (size_t i = lo; i < hi && !refused; ++i) {
+        l.clear();
+        make(todo[i], l);
+        finish(todo[i], l);
+        n[i - lo] = (uint32_t)l.size();
+        out.insert(out.end(), l.begin(), l.end());
       }
+      if (refused) return;
+      const Entry* p = out.data();
+      for (size_t i = lo; i < hi; p += n[i - lo], ++i) {
+        lists.first[first + i] = p;
+        lists.n[first + i] = n[i - lo];
+      }
+      lists.store[piece + q] = std::move(out);  // its entries stay where they are
     });
   };
   // one-char vertices with upward in-edges, by rising level
