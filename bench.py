@@ -915,20 +915,12 @@ def profiled_roofline(cb, g, st, multi, device, R, opts, peak, src, row_bits, cl
         sample = make_reads(g, R, 77_777, len_max=1000)
         pctx.align_scores_batched(sample, **dict(opts, slots=R), row_bits=row_bits)
     pr = pctx.profile()
+    ran = pctx.last_row_kernel()
     pctx.close()
     w = pr["row_bits"] // 8
     row_avg_s = pr["row_ms"] / max(1, pr["row_launches"]) / 1e3
-    # AUTO without a level grouping: the bit-row kernels, unless the graph has no closure
-    # lists (then delta rows for score-only steps at 128 slots)
-    bits = pr["launches"] < 3 * pr["row_launches"] + 64  # one kernel a row-step
-    auto16 = "k_row_delta" if R == 128 else ("k_row_stream" if R >= 64 else ("k_row_dpx" if R >= 2 else "k_row_t1"))
-    kname = {cb.ROW_DIRECT: "k_row_direct", cb.ROW_TILED: "k_row_tiled", cb.ROW_DPX: "k_row_dpx",
-             cb.ROW_STREAM: "k_row_stream", cb.ROW_DELTA: "k_row_delta"}.get(
-        opts["row_kernel"] if R > 1 else 0, auto16 if pr["row_bits"] == 16 else "k_row_direct")
-    if pr["row_bits"] == 32 and kname in ("k_row_stream", "k_row_dpx", "k_row_delta"):
-        kname = "k_row_direct"  # the 16-bit kernels do not run 32-bit rows
-    if bits:
-        kname = "k_row_sliced" if R >= 32 and w == 2 and st["num_strings"] * R > 400_000 else "k_row_words"
+    kname = ran.split("<")[0]
+    bits = kname in ("k_row_words", "k_row_sliced")  # one kernel a row-step
     ab = algorithmic_bit_row_bytes(st, R, w) if bits else \
         algorithmic_delta_row_bytes(st, R, multi) if kname == "k_row_delta" else \
         algorithmic_row_bytes(st, R, multi, w)
