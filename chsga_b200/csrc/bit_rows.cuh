@@ -105,7 +105,8 @@ struct BitArgs {
 __global__ void __launch_bounds__(256) k_closure_arrays(uint32_t S, uint32_t heavy, const uint4* __restrict__ rec,
                                                         uint2* ent, uint4* wrec, uint2* wsv, uint32_t* pos,
                                                         uint2* went, uint4* lab, const uint32_t* __restrict__ lab4) {
-  const uint32_t t = blockIdx.x * 256 + threadIdx.x, i = t / 8, l = t % 8;
+  const uint64_t t = (uint64_t)blockIdx.x * 256 + threadIdx.x;
+  const uint32_t i = (uint32_t)(t / 8), l = (uint32_t)(t % 8);
   const bool live = i < S;
   const uint4 in = live ? wrec[i] : make_uint4(0, 0, 0, 0);
   __syncwarp();  // all lanes of a position have read its record

@@ -1109,10 +1109,14 @@ void upload_graph(chsga_ctx& c, const chsga_graph_host& g) {
   dev::k_heads<<<nblocks(L.S), 256, 0, s>>>(L.S, d.up_off.p, d.up_in.p, d.dn_off.p, d.dn_in.p, d.dv_first.p,
                                             d.dv_len.p, d.dv_s.p, d.dn_head.p, d.up_head.p, d.fin.p);
   check_launch();
+  // host arrays of copies in flight: they live until the one wait at the end
+  std::vector<uint32_t> order;
+  HostClosure cl;
+  HostT1 t1;
   {
     // runs of 32 consecutive string vertices, longest (in chars) first; ties by index
     const uint32_t nruns = (L.S + 31) / 32;
-    std::vector<uint32_t> order(nruns);
+    order.resize(nruns);
     std::vector<uint32_t> len(nruns);
     for (uint32_t r = 0; r < nruns; ++r) {
       order[r] = r;
@@ -1120,18 +1124,14 @@ void upload_graph(chsga_ctx& c, const chsga_graph_host& g) {
     }
     std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return len[a] > len[b]; });
     d.delta_order.upload(order, s);
-    CK(cudaStreamSynchronize(s));  // the host vectors die with this scope
   }
   auto top = make_top(L, d, kTopDefaultVertices, s);
-  {
-    HostT1 t1 = build_t1(L);
-    if (t1.ok) {
-      as(d.t1_desc, t1.desc);
-      as(d.t1_vrec, t1.vrec);
-      d.t1_heads.upload(t1.heads, s);
-      lg->t1 = dev::T1Ptrs{d.t1_desc.p, d.t1_heads.p, d.t1_vrec.p, t1.ntiles()};
-    }
-    CK(cudaStreamSynchronize(s));  // the host vectors die with this scope
+  t1 = build_t1(L);
+  if (t1.ok) {
+    as(d.t1_desc, t1.desc);
+    as(d.t1_vrec, t1.vrec);
+    d.t1_heads.upload(t1.heads, s);
+    lg->t1 = dev::T1Ptrs{d.t1_desc.p, d.t1_heads.p, d.t1_vrec.p, t1.ntiles()};
   }
   lg->gp = dev::GraphPtrs{L.N,          L.S,          L.special,    d.lab2.p,     d.lab_sp.p,
                           d.lab4.p,     d.sv_off.p,   d.sv_dev.p,   d.vin_off.p,  d.vin_src.p,
@@ -1140,7 +1140,7 @@ void upload_graph(chsga_ctx& c, const chsga_graph_host& g) {
                           d.dn_head.p,  d.up_head.p,  d.fin.p,
                           (uint32_t)L.vin_srcv.size(), (uint32_t)L.up_in.size(), (uint32_t)L.dn_in.size()};
   {
-    const HostClosure cl = build_closure(L);
+    cl = build_closure(L);
     if (cl.ok) {
       // one allocation: {records, entries, order} as the host has them, then
       // what the device makes from them
@@ -1185,10 +1185,10 @@ void upload_graph(chsga_ctx& c, const chsga_graph_host& g) {
       d.cl_by_len[0] = m + by32;
       d.cl_by_len[1] = m + by64;
       d.cl_by_len[2] = m + by128;
-      CK(cudaStreamSynchronize(s));  // the host arrays die with this scope
       lg->bits = true;
     }
   }
+  CK(cudaStreamSynchronize(s));
   lg->nul_label = std::memchr(g.labels, '\0', g.num_chars) != nullptr;
   lg->n_label = std::memchr(g.labels, 'N', g.num_chars) != nullptr;
   lg->pitch = ((size_t)L.N + 15) / 16 * 16;
