@@ -45,17 +45,19 @@ template <typename T>
 struct DevArr {
   T* p = nullptr;
   size_t n = 0;
+  bool view = false;  // part of another array (DevSlab), which frees it
   DevArr() = default;
   DevArr(const DevArr&) = delete;
   DevArr& operator=(const DevArr&) = delete;
   ~DevArr() { release(); }
   void release() {
-    if (p) {
+    if (p && !view) {
       cudaFree(p);
       t_live_bytes -= (int64_t)(n * sizeof(T));
     }
     p = nullptr;
     n = 0;
+    view = false;
   }
   void alloc(size_t count) {
     if (count <= n && p) return;
@@ -92,7 +94,78 @@ struct PinnedArr {
   }
 };
 
+// Arrays that are allocated and filled together: one allocation, and one copy
+// for a small set (each costs about 20 us: the 20-odd arrays of a 20 kbp graph
+// took half of its load).
+class DevSlab {
+ public:
+  // `to` gets room for n elements.
+  template <typename T>
+  void add(DevArr<T>& to, size_t n) {
+    add(to, n, nullptr, 0);
+  }
+  // `to` gets the elements of `v`, which stays until fill() has been waited for.
+  template <typename T, typename V>
+  void put(DevArr<T>& to, const V& v) {
+    const size_t bytes = v.size() * sizeof(v[0]);
+    add(to, bytes / sizeof(T), v.data(), bytes);
+  }
+  void fill(cudaStream_t s) {
+    size_t copied = 0, all = 0;
+    // the copied parts first, side by side
+    for (bool src : {true, false})
+      for (Part& q : parts_)
+        if ((q.src != nullptr) == src) {
+          q.at = all;
+          all += (q.room + 255) / 256 * 256;
+          if (src) copied = all;
+        }
+    mem_.alloc(all);
+    if (copied <= kOneCopy) {
+      stage_.resize(copied);
+      for (const Part& q : parts_)
+        if (q.src) std::memcpy(stage_.data() + q.at, q.src, q.bytes);
+      if (copied) CK(cudaMemcpyAsync(mem_.p, stage_.data(), copied, cudaMemcpyHostToDevice, s));
+    } else {
+      for (const Part& q : parts_)
+        if (q.src) CK(cudaMemcpyAsync(mem_.p + q.at, q.src, q.bytes, cudaMemcpyHostToDevice, s));
+    }
+    for (const Part& q : parts_) q.set(q.to, mem_.p + q.at, q.n);
+  }
+  // After the copies are done.
+  void done() {
+    parts_ = std::vector<Part>();
+    stage_ = std::vector<unsigned char>();
+  }
+
+ private:
+  static constexpr size_t kOneCopy = 4u << 20;
+  struct Part {
+    void* to;
+    void (*set)(void* to, unsigned char* p, size_t n);
+    size_t n, room, bytes;
+    const void* src;
+    size_t at;
+  };
+  template <typename T>
+  void add(DevArr<T>& to, size_t n, const void* src, size_t bytes) {
+    to.release();
+    parts_.push_back(Part{&to,
+                          [](void* t, unsigned char* p, size_t k) {
+                            auto& a = *static_cast<DevArr<T>*>(t);
+                            a.p = reinterpret_cast<T*>(p);
+                            a.n = k;
+                            a.view = true;
+                          },
+                          n, std::max<size_t>(n, 1) * sizeof(T), bytes, bytes ? src : nullptr, 0});
+  }
+  DevArr<unsigned char> mem_;
+  std::vector<Part> parts_;
+  std::vector<unsigned char> stage_;
+};
+
 struct GraphDev {
+  DevSlab slab;  // holds the arrays below
   DevArr<uint32_t> lab2, lab_sp, lab4, sv_off, sv_dev, vin_off, vin_src, vin_srcv, dv_first, dv_len;
   DevArr<uint32_t> up_off, dn_off, istr_off, istr_src;
   DevArr<uint32_t> dv_s;
@@ -101,8 +174,11 @@ struct GraphDev {
   DevArr<uint4> t1_desc, t1_vrec;  // tiles of the one-read row kernel (k_row_t1)
   DevArr<uint8_t> t1_heads;
   DevArr<uint32_t> delta_order;    // k_row_delta: runs of 32 string vertices by decreasing char count
-  DevArr<unsigned char> cl;        // every array of the bit-row kernels (closure.hpp)
-  const uint8_t* cl_by_len[3] = {};
+  // bit-row kernels (closure.hpp)
+  DevArr<uint4> cl_rec, cl_wrec, cl_lab;
+  DevArr<uint2> cl_ent16, cl_went, cl_wsv;
+  DevArr<uint8_t> cl_by_len[3];
+  DevArr<uint32_t> cl_pos;
 };
 
 struct TopDev {
@@ -874,7 +950,7 @@ void bit_step(chsga_ctx& c, BitBufs& b, int par, cudaStream_t s) {
       using S4 = dev::SlicedShared<R, 4>;
       using S1 = dev::SlicedShared<R, 1>;
       // four items a lane where that gives every warp of the device work
-      a.g.by_len = c.g->gd.cl_by_len[R == 128 ? 0 : R == 64 ? 1 : 2];
+      a.g.by_len = c.g->gd.cl_by_len[R == 128 ? 0 : R == 64 ? 1 : 2].p;
       const bool four = c.bit_form == BitForm::Auto ? S >= (uint32_t)S4::VB * 16u * (uint32_t)c.num_sms
                                                     : c.bit_form == BitForm::Sliced4;
       if (four)
@@ -1075,120 +1151,103 @@ void run_queue(chsga_ctx& c, uint32_t n, uint64_t total_rows, uint32_t mode, uin
 
 void upload_graph(chsga_ctx& c, const chsga_graph_host& g) {
   HostLayout L = build_layout(g);
-  // the previous graph (if any) stays alive while another context shares it
-  auto lg = std::make_shared<LoadedGraph>();
-  GraphDev& d = lg->gd;
-  cudaStream_t s = c.st;
-  d.lab2.upload(L.lab2, s);
-  d.lab_sp.upload(L.lab_sp, s);
-  d.lab4.upload(L.lab4, s);
-  d.sv_off.upload(L.sv_off, s);
-  d.sv_dev.upload(L.sv_dev, s);
-  d.vin_off.upload(L.vin_off, s);
-  d.vin_src.upload(L.vin_src, s);
-  d.vin_srcv.upload(L.vin_srcv, s);
-  d.dv_first.upload(L.dv_first, s);
-  d.dv_len.upload(L.dv_len, s);
-  d.up_off.upload(L.up_off, s);
-  d.dn_off.upload(L.dn_off, s);
-  d.istr_off.upload(L.istr_off, s);
-  d.istr_src.upload(L.istr_src, s);
-  d.dv_s.upload(L.dv_s, s);
-  // a host array as the device's records of the same layout
-  auto as = [&](auto& to, const auto& v) {
-    const size_t each = sizeof(*to.p), n = v.size() * sizeof(v[0]) / each;
-    to.alloc(n);
-    if (n) CK(cudaMemcpyAsync(to.p, v.data(), n * each, cudaMemcpyHostToDevice, s));
-  };
-  static_assert(sizeof(EdgeW) == sizeof(int2), "host edges are the device's");
-  as(d.up_in, L.up_in);
-  as(d.dn_in, L.dn_in);
-  d.dn_head.alloc(L.S);
-  d.up_head.alloc(2 * (size_t)L.S);
-  d.fin.alloc(L.S);
-  dev::k_heads<<<nblocks(L.S), 256, 0, s>>>(L.S, d.up_off.p, d.up_in.p, d.dn_off.p, d.dn_in.p, d.dv_first.p,
-                                            d.dv_len.p, d.dv_s.p, d.dn_head.p, d.up_head.p, d.fin.p);
-  check_launch();
-  // host arrays of copies in flight: they live until the one wait at the end
-  std::vector<uint32_t> order;
-  HostClosure cl;
-  HostT1 t1;
+  const HostT1 t1 = build_t1(L);
+  const HostClosure cl = build_closure(L);
+  // runs of 32 consecutive string vertices, longest (in chars) first; ties by index
+  const uint32_t nruns = (L.S + 31) / 32;
+  std::vector<uint32_t> order(nruns);
   {
-    // runs of 32 consecutive string vertices, longest (in chars) first; ties by index
-    const uint32_t nruns = (L.S + 31) / 32;
-    order.resize(nruns);
     std::vector<uint32_t> len(nruns);
     for (uint32_t r = 0; r < nruns; ++r) {
       order[r] = r;
       len[r] = L.sv_off[std::min<uint64_t>((uint64_t)32 * r + 32, L.S)] - L.sv_off[(uint64_t)32 * r];
     }
     std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return len[a] > len[b]; });
-    d.delta_order.upload(order, s);
+  }
+  // the previous graph (if any) stays alive while another context shares it
+  auto lg = std::make_shared<LoadedGraph>();
+  GraphDev& d = lg->gd;
+  cudaStream_t s = c.st;
+  DevSlab& m = d.slab;
+  static_assert(sizeof(EdgeW) == sizeof(int2), "host edges are the device's");
+  m.put(d.lab2, L.lab2);
+  m.put(d.lab_sp, L.lab_sp);
+  m.put(d.lab4, L.lab4);
+  m.put(d.sv_off, L.sv_off);
+  m.put(d.sv_dev, L.sv_dev);
+  m.put(d.vin_off, L.vin_off);
+  m.put(d.vin_src, L.vin_src);
+  m.put(d.vin_srcv, L.vin_srcv);
+  m.put(d.dv_first, L.dv_first);
+  m.put(d.dv_len, L.dv_len);
+  m.put(d.up_off, L.up_off);
+  m.put(d.dn_off, L.dn_off);
+  m.put(d.istr_off, L.istr_off);
+  m.put(d.istr_src, L.istr_src);
+  m.put(d.dv_s, L.dv_s);
+  m.put(d.up_in, L.up_in);
+  m.put(d.dn_in, L.dn_in);
+  m.put(d.delta_order, order);
+  m.add(d.dn_head, L.S);
+  m.add(d.up_head, 2 * (size_t)L.S);
+  m.add(d.fin, L.S);
+  if (t1.ok) {
+    m.put(d.t1_desc, t1.desc);
+    m.put(d.t1_vrec, t1.vrec);
+    m.put(d.t1_heads, t1.heads);
+  }
+  if (cl.ok) {
+    // {records, entries, order} as the host has them; k_closure_arrays and
+    // k_by_len make the rest of them
+    m.put(d.cl_rec, cl.rec);
+    m.put(d.cl_ent16, cl.ent);
+    m.put(d.cl_wrec, cl.order);
+    m.add(d.cl_wsv, L.S);
+    m.add(d.cl_pos, L.S);
+    m.add(d.cl_went, cl.n_went);
+    m.add(d.cl_lab, cl.words);
+    for (auto& x : d.cl_by_len) m.add(x, L.S);
+  }
+  m.fill(s);
+  dev::k_heads<<<nblocks(L.S), 256, 0, s>>>(L.S, d.up_off.p, d.up_in.p, d.dn_off.p, d.dn_in.p, d.dv_first.p,
+                                            d.dv_len.p, d.dv_s.p, d.dn_head.p, d.up_head.p, d.fin.p);
+  check_launch();
+  if (cl.ok) {
+    dev::k_closure_arrays<<<nblocks((uint64_t)L.S * 8), 256, 0, s>>>(L.S, cl.heavy, d.cl_rec.p, d.cl_ent16.p,
+                                                                     d.cl_wrec.p, d.cl_wsv.p, d.cl_pos.p,
+                                                                     d.cl_went.p, d.cl_lab.p, d.lab4.p);
+    check_launch();
+    dev::k_by_len<<<nblocks(L.S, 128), 128, 0, s>>>(L.S, d.sv_off.p, d.cl_by_len[0].p, d.cl_by_len[1].p,
+                                                    d.cl_by_len[2].p);
+    check_launch();
+    lg->bits = true;
+    dev::BitGraph& b = lg->bg;
+    b.S = L.S;
+    b.N = L.N;
+    b.n_ent = (uint32_t)cl.ent.size();
+    b.n_went = (uint32_t)cl.n_went;
+    b.heavy = cl.heavy;
+    b.words = cl.words;
+    b.rec = d.cl_rec.p;
+    b.ent16 = d.cl_ent16.p;
+    b.sv_off = d.sv_off.p;
+    b.lab4 = d.lab4.p;
+    b.pos = d.cl_pos.p;
+    b.wsv = d.cl_wsv.p;
+    b.wrec = d.cl_wrec.p;
+    b.went = d.cl_went.p;
+    b.lab = d.cl_lab.p;
   }
   auto top = make_top(L, d, kTopDefaultVertices, s);
-  t1 = build_t1(L);
-  if (t1.ok) {
-    as(d.t1_desc, t1.desc);
-    as(d.t1_vrec, t1.vrec);
-    d.t1_heads.upload(t1.heads, s);
-    lg->t1 = dev::T1Ptrs{d.t1_desc.p, d.t1_heads.p, d.t1_vrec.p, t1.ntiles()};
-  }
+  if (t1.ok) lg->t1 = dev::T1Ptrs{d.t1_desc.p, d.t1_heads.p, d.t1_vrec.p, t1.ntiles()};
   lg->gp = dev::GraphPtrs{L.N,          L.S,          L.special,    d.lab2.p,     d.lab_sp.p,
                           d.lab4.p,     d.sv_off.p,   d.sv_dev.p,   d.vin_off.p,  d.vin_src.p,
                           d.vin_srcv.p, d.dv_first.p, d.dv_len.p,   d.dv_s.p,     d.up_off.p,
                           d.up_in.p,    d.dn_off.p,   d.dn_in.p,    d.istr_off.p, d.istr_src.p,
                           d.dn_head.p,  d.up_head.p,  d.fin.p,
                           (uint32_t)L.vin_srcv.size(), (uint32_t)L.up_in.size(), (uint32_t)L.dn_in.size()};
-  {
-    cl = build_closure(L);
-    if (cl.ok) {
-      // one allocation: {records, entries, order} as the host has them, then
-      // what the device makes from them
-      const size_t E = cl.ent.size(), W = std::max<uint64_t>(cl.words, 1);
-      size_t bytes = 0;
-      auto room = [&](size_t n) {
-        const size_t at = bytes;
-        bytes += (n + 255) / 256 * 256;
-        return at;
-      };
-      const size_t rec = room(16 * (size_t)L.S), ent = room(8 * E), wrec = room(16 * (size_t)L.S),
-                   wsv = room(8 * (size_t)L.S), pos = room(4 * (size_t)L.S), went = room(8 * cl.n_went),
-                   lab = room(16 * W), by32 = room(L.S), by64 = room(L.S), by128 = room(L.S);
-      d.cl.alloc(bytes);
-      unsigned char* const m = d.cl.p;
-      CK(cudaMemcpyAsync(m + rec, cl.rec.data(), 16 * (size_t)L.S, cudaMemcpyHostToDevice, s));
-      if (E) CK(cudaMemcpyAsync(m + ent, cl.ent.data(), 8 * E, cudaMemcpyHostToDevice, s));
-      CK(cudaMemcpyAsync(m + wrec, cl.order.data(), 16 * (size_t)L.S, cudaMemcpyHostToDevice, s));
-      dev::BitGraph& b = lg->bg;
-      b.S = L.S;
-      b.N = L.N;
-      b.n_ent = (uint32_t)E;
-      b.n_went = (uint32_t)cl.n_went;
-      b.heavy = cl.heavy;
-      b.words = cl.words;
-      b.rec = reinterpret_cast<const uint4*>(m + rec);
-      b.ent16 = reinterpret_cast<const uint2*>(m + ent);
-      b.sv_off = d.sv_off.p;
-      b.lab4 = d.lab4.p;
-      b.pos = reinterpret_cast<const uint32_t*>(m + pos);
-      b.wsv = reinterpret_cast<const uint2*>(m + wsv);
-      b.wrec = reinterpret_cast<const uint4*>(m + wrec);
-      b.went = reinterpret_cast<const uint2*>(m + went);
-      b.lab = reinterpret_cast<const uint4*>(m + lab);
-      dev::k_closure_arrays<<<nblocks((uint64_t)L.S * 8), 256, 0, s>>>(
-          L.S, cl.heavy, b.rec, reinterpret_cast<uint2*>(m + ent), reinterpret_cast<uint4*>(m + wrec),
-          reinterpret_cast<uint2*>(m + wsv), reinterpret_cast<uint32_t*>(m + pos),
-          reinterpret_cast<uint2*>(m + went), reinterpret_cast<uint4*>(m + lab), b.lab4);
-      check_launch();
-      dev::k_by_len<<<nblocks(L.S, 128), 128, 0, s>>>(L.S, b.sv_off, m + by32, m + by64, m + by128);
-      check_launch();
-      d.cl_by_len[0] = m + by32;
-      d.cl_by_len[1] = m + by64;
-      d.cl_by_len[2] = m + by128;
-      lg->bits = true;
-    }
-  }
-  CK(cudaStreamSynchronize(s));
+  CK(cudaStreamSynchronize(s));  // the host arrays die with this scope
+  m.done();
   lg->nul_label = std::memchr(g.labels, '\0', g.num_chars) != nullptr;
   lg->n_label = std::memchr(g.labels, 'N', g.num_chars) != nullptr;
   lg->pitch = ((size_t)L.N + 15) / 16 * 16;
