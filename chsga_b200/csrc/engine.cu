@@ -117,7 +117,7 @@ class DevSlab {
       for (Part& q : parts_)
         if ((q.src != nullptr) == src) {
           q.at = all;
-          all += (q.room + 255) / 256 * 256;
+          all += (q.room + kAlign - 1) / kAlign * kAlign;
           if (src) copied = all;
         }
     mem_.alloc(all);
@@ -140,6 +140,10 @@ class DevSlab {
 
  private:
   static constexpr size_t kOneCopy = 4u << 20;
+  // A row-step of a small graph varies by up to 5 % with where its arrays fall.
+  // Mean over 32 placements, 64 slots on 100 kbp: 14.6 us with 4 KiB, as with an
+  // allocation for each array, 14.7 with 256 bytes.
+  static constexpr size_t kAlign = 4096;
   struct Part {
     void* to;
     void (*set)(void* to, unsigned char* p, size_t n);
