@@ -232,10 +232,12 @@ def measured_peak():
 
 
 def ncu_traffic(kname="k_row_stream"):
-    """The ncu DRAM bytes of one row-kernel launch, scaled to the bench graph
-    (profiles/k_row_traffic.json for k_row_stream, k_row_delta_traffic.json
-    for k_row_delta)."""
-    name = {"k_row_stream": "k_row_traffic.json", "k_row_delta": "k_row_delta_traffic.json"}.get(kname)
+    """The ncu DRAM bytes of one row-kernel launch at 128 slots, scaled to the
+    bench graph (profiles/k_row_sliced_traffic.json for k_row_sliced,
+    k_row_delta_traffic.json for k_row_delta, k_row_traffic.json for
+    k_row_stream)."""
+    name = {"k_row_stream": "k_row_traffic.json", "k_row_delta": "k_row_delta_traffic.json",
+            "k_row_sliced": "k_row_sliced_traffic.json"}.get(kname)
     if name is None:
         return None
     p = os.path.join(ROOT, "profiles", name)
@@ -924,7 +926,7 @@ def profiled_roofline(cb, g, st, multi, device, R, opts, peak, src, row_bits, cl
     ab = algorithmic_bit_row_bytes(st, R, w) if bits else \
         algorithmic_delta_row_bytes(st, R, multi) if kname == "k_row_delta" else \
         algorithmic_row_bytes(st, R, multi, w)
-    tr = ncu_traffic(kname)
+    tr = ncu_traffic(kname) if R == 128 else None
     total = pr["row_ms"] + pr["sweep_up_ms"] + pr["top_ms"] + pr["sweep_down_ms"] + pr["other_ms"]
     # working set of one row-step: two score rows, BV and FL, graph arrays
     S = st["num_strings"]

@@ -35,7 +35,7 @@ constexpr uint32_t SW_DRAIN = 1u << 13;     // the slot's previous read takes it
 constexpr uint32_t SW_PAR_SHIFT = 14;       // bits 14..15: which of the slot's four minima its read uses
 constexpr uint32_t kBitsNarrowMax = 32767;  // longest read whose sums need no saturation
 
-struct BitGraph {  // closure.hpp
+struct BitGraph {  // closure.hpp, k_closure_arrays
   uint32_t S, N, n_ent, n_went, heavy;
   uint64_t words;
   const uint4* rec;
@@ -499,6 +499,7 @@ __global__ void __launch_bounds__(NT, CHSGA_WORDS_THREADS / NT) k_row_words(BitA
       RLout[(size_t)sv.x * R] = (ST)last;
       // the raw row's minimum and its first char; a chain falls by at most
       // one a char, so most vertices cannot reach the block's best so far
+      // (which other warps lower meanwhile: an old value only prunes less)
       if ((w & SW_ENDING) &&
           max(T - (int)(len - 1), 0) <= (int)min(s_min[par * R + r] >> 32, 0x7FFFFFFFull)) {
         const uint32_t f = sv.y;
@@ -745,11 +746,12 @@ __global__ void __launch_bounds__(32) k_walk_bits(GraphPtrs g, BitGraph bg, size
 // char of 32 slots is a handful of logic operations, where the packed 16-bit
 // update spends tens of instructions.
 //
-// What bounds it: 5 Mbp graph, 128 slots, 305 us a row-step (the sweeps'
-// chain: 771): 0.94 GB from and to HBM is 145 us at the copy peak and 144 M
-// warp-instructions are 125 us of issue; the rest is load latency at 32 warps
-// an SM (8.7 of 14 stall cycles an instruction). Without the gathers it takes
-// 100 us less, without the chain 150. Blocks of 128 threads with barriers
+// What bounds it: load latency at the 32 warps an SM that 64 registers allow.
+// 5 Mbp graph, 128 slots, 305 us a row-step (the sweeps' chain: 771). On the
+// 2 Mbp graph ncu counts 145 us, 0.35 GB from and to HBM (54 us at the copy
+// peak), 62 M warp-instructions (54 us of issue) and 9.2 of 15.3 cycles between
+// a warp's instructions waiting for loads. At 5 Mbp it takes 100 us less
+// without the gathers, 150 without the chain. Blocks of 128 threads with barriers
 // between the passes took 353, five or six gathers in flight 316-357 (spills
 // past 64 registers), prefetches to L2 or shared memory 374-440.
 //
@@ -1091,7 +1093,9 @@ __device__ __forceinline__ void sliced_warp(const BitArgs& a, const HeadFlags& h
       *reinterpret_cast<uint4*>(RLout + so) = o;
     }
     if (hf.end) {
-      // hand the best so far to the other blocks and take theirs
+      // hand the best so far to the other blocks and take theirs. Warps read
+      // lim and best while others write them: values only fall, and an old one
+      // only prunes less
       for (int r = (int)lane; r < R; r += 32) {
         const unsigned long long b = *(volatile unsigned long long*)&sh.best[0][r];
         if (b == ~0ull) continue;

@@ -853,8 +853,10 @@ bool bits_apply(const chsga_ctx& c) {
 // 32-bit scores and vertices too long for one thread's serial chain keep a
 // read's bits in words. So do graphs of at most 400,000 (vertex, slot) pairs:
 // there a row-step is one thread's chain of loads, which is shorter with
-// words (64 slots on 5,500 vertices: 13.9 us against 14.5, 32 slots 11.4
-// against 14.6; on 22,000 vertices 28.7 against 22.0 and 19.0 against 18.4).
+// words (us a row-step, words and sliced: 32 slots on 7,700 vertices 10.6 and
+// 13.0, on 11,100 12.0 and 12.7; 64 slots on 5,500 13.0 and 13.3, on 7,700
+// 14.8 and 13.6; 128 slots on 2,200 10.2 and 10.4, on 3,100 12.1 and 11.2, on
+// 3,900 15.6 and 12.7).
 template <int R, typename ST>
 bool bits_sliced(const chsga_ctx& c) {
   if (R < 32 || !std::is_same_v<ST, uint16_t> || c.g->L.max_len > 512) return false;
@@ -2925,7 +2927,7 @@ chsga_status chsga_open(const chsga_opts* opts, chsga_ctx** out) {
       if (std::string(rk) == "delta") c->row_kernel = RowKernel::Delta;
     }
     // CHSGA_PLAIN_LAUNCH=stream|graphs|persistent: how chsga_align_scores
-    // runs its row-steps (default graphs)
+    // runs its row-steps (default kPlainAuto)
     if (const char* pl = std::getenv("CHSGA_PLAIN_LAUNCH")) {
       if (std::string(pl) == "stream") c->plain_mode = CHSGA_LAUNCH_STREAM;
       if (std::string(pl) == "graphs") c->plain_mode = CHSGA_LAUNCH_GRAPHS;

@@ -332,9 +332,10 @@ chsga_status chsga_align_scores_batched(chsga_ctx* ctx, const char* const* reads
  * arrays then) and align with this call. It returns the same scores as
  * chsga_align_scores for the same reads. Every per-call buffer comes from
  * one fixed array of CHSGA_NOALLOC_SCRATCH_BYTES inside the library: read
- * bytes, read queue, two 16-bit score rows, per-vertex boundary scores,
- * slot state and results. The call makes no cudaMalloc, no cudaFree and no
- * other allocating call.
+ * bytes, read queue, the row's state (bit rows where they apply and fit, else
+ * two 16-bit score rows and per-vertex boundary scores), slot state and
+ * results. The call makes no cudaMalloc, no cudaFree and no other allocating
+ * call.
  *
  * - The CUDA driver reserves the array on each GPU where it loads the
  *   library's device code, and the GPU keeps it until the process exits.
@@ -346,7 +347,8 @@ chsga_status chsga_align_scores_batched(chsga_ctx* ctx, const char* const* reads
  * - The call fails with CHSGA_ERR_OOM, and runs nothing, when the graph and
  *   the reads need more than the array holds. The need is about
  *   4 N + 8 S + (read bytes) + 52 n bytes, where N = chars and S = string
- *   vertices, each part rounded up to 256 bytes.
+ *   vertices, each part rounded up to 256 bytes; it is counted so whichever
+ *   rows run.
  * - It fails with CHSGA_ERR_UNSUPPORTED for a read longer than 65000 bases,
  *   because its rows are 16-bit.
  * - All calls on one device share the array, which keeps the last call's
